@@ -133,14 +133,19 @@ int batch_enqueue(gbn_batch* b, bool graph_mode) {
                                       : RandStart{lcg48_apply(j, ctx->rand48), nullptr, 1, 0};
       n_launch += launch_constants(ctx, b->probs[i], b->out[i], rs, s);
     }
+    const bool pair = g.row_local && kh->pair_cols;
+    for (size_t k = 0; pair && k < g.idx.size(); ++k)
+      n_launch += launch_pair_setup(ctx, b->probs[g.idx[k]], g.tab + k, s);
     for (unsigned nl = 1; nl <= g.maxIntIter; ++nl) {
       for (int i : g.idx) {
-        n_launch += launch_outer_begin(ctx, b->probs[i], int(nl), b->out[i], s);
+        n_launch += pair ? launch_outer_begin_pair(ctx, b->probs[i], int(nl), b->out[i], s)
+                         : launch_outer_begin(ctx, b->probs[i], int(nl), b->out[i], s);
         if (mixed) n_launch += launch_mixed_colmax(b->probs[i], s);
       }
       if (g.row_local || g.row_local_tc) {
         // one launch more recomputes a member's last update when its stopping test ends the loop
-        const unsigned nit = g.maxIter + (g.any_stoptest ? 1u : 0u);
+        // (the column pairs run one iteration ahead of the test, and sum the last one's objective in a launch of its own)
+        const unsigned nit = g.maxIter + (g.any_stoptest ? (pair ? 2u : 1u) : 0u);
         for (unsigned it = 0; it < nit; ++it) {
           if (g.row_local_tc)
             launch_iter_tc(g.tab, g.bm, int(it), g.npad_max, g.cnmax_tc, g.g_tc, s);
@@ -148,6 +153,10 @@ int batch_enqueue(gbn_batch* b, bool graph_mode) {
             kh->iter_cols(g.tab, g.bm, int(it), false, g.g3, s);
         }
         n_launch += nit;
+        if (pair && !g.any_stoptest) {
+          kh->iter_finish(g.tab, g.bm, int(g.maxIter), g.g3, s);
+          n_launch += 1;
+        }
       }
       for (unsigned it = 0; it < ((g.row_local || g.row_local_tc) ? 0u : g.maxIter); ++it) {
         if (mixed)
@@ -161,7 +170,9 @@ int batch_enqueue(gbn_batch* b, bool graph_mode) {
           kh->inv_cols(g.tab, g.bm, int(it), true, g.g3, s);
         n_launch += 3;
       }
-      for (int i : g.idx) n_launch += launch_outer_end(ctx, b->probs[i], b->out[i], s);
+      for (int i : g.idx)
+        n_launch += pair ? launch_outer_end_pair(ctx, b->probs[i], b->out[i], s)
+                         : launch_outer_end(ctx, b->probs[i], b->out[i], s);
     }
     if ((e = cudaEventRecord(g.done, s)) != cudaSuccess) return cuda_status(e, "batch join");
     if ((e = cudaStreamWaitEvent(ctx->stream, g.done, 0)) != cudaSuccess) return cuda_status(e, "batch join");

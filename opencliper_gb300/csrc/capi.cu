@@ -194,11 +194,13 @@ int gbn_ctx_create(int device, gbn_ctx** out) {
   }
   // two-pass twiddle tables for every supported length L = A*B:
   // [k1*B + s] = w_L^(s*k1) (k1 < A, s < B) and [L + k1'*A + s'] = w_L^(s'*k1')
-  // (k1' < B, s' < A), w_L^j = (cos, -sin)(2 pi j / L)
+  // (k1' < B, s' < A), w_L^j = (cos, -sin)(2 pi j / L), then, for the
+  // column-pair iteration, rows s < PB of pair_ts(L) entries w_L^(s*k1) (k1 < PA), each as (c, c, s, s)
   int lens[64];
   const int nl = supported_sizes(lens, 64);
   size_t total = 0;
-  for (int i = 0; i < nl; ++i) total += 2 * size_t(lens[i]);
+  auto pair_entries = [](int L) { return pair_split_ok(L) ? 2 * size_t(pair_b(L)) * pair_ts(L) : 0; };
+  for (int i = 0; i < nl; ++i) total += 2 * size_t(lens[i]) + pair_entries(lens[i]);
   std::vector<float2> h(total);
   size_t off = 0;
   std::vector<size_t> offs(nl);
@@ -210,7 +212,15 @@ int gbn_ctx_create(int device, gbn_ctx** out) {
       for (int s = 0; s < B; ++s) h[off + size_t(k1) * B + s] = w((long long)s * k1, L);
     for (int k1 = 0; k1 < B; ++k1)
       for (int s = 0; s < A; ++s) h[off + L + size_t(k1) * A + s] = w((long long)s * k1, L);
-    off += 2 * size_t(L);
+    if (pair_split_ok(L))
+      for (int s = 0; s < pair_b(L); ++s)
+        for (int k1 = 0; k1 < pair_a(L); ++k1) {
+          const float2 v = w((long long)s * k1, L);
+          const size_t o = off + 2 * size_t(L) + 2 * (size_t(s) * pair_ts(L) + k1);
+          h[o] = make_float2(v.x, v.x);
+          h[o + 1] = make_float2(v.y, v.y);
+        }
+    off += 2 * size_t(L) + pair_entries(L);
   }
   if ((e = cudaMalloc(&ctx->tw_block, total * sizeof(float2))) != cudaSuccess ||
       (e = cudaMemcpy(ctx->tw_block, h.data(), total * sizeof(float2), cudaMemcpyHostToDevice)) != cudaSuccess) {

@@ -131,6 +131,15 @@ struct gbn_problem {
   float2* mc_gm = nullptr;            // M^T of it
   double* mc_part = nullptr;          // power-method norm partials
   gbn::McTables* mc_tab = nullptr;    // gather tables of the meshes (motion.cu)
+  // column-pair row-local iteration (rowpair.cuh)
+  float4* St = nullptr;               // S in tiles
+  float4* Tt = nullptr;               // kept rows' IDFT_W(y) in tiles
+  size_t Tt_rows = 0;                 // kept rows Tt holds
+  float2* xk2 = nullptr;              // third x_k and w_k buffers
+  float2* wacc2 = nullptr;
+  float4* xt = nullptr;               // x_ref in tiles
+  uint4* ptab = nullptr;              // [F][PA]
+  int* rowslot = nullptr;             // [F*H] staged slot of each kept row
   gbn::FusedArgs* d_args = nullptr;   // one-entry instance table of the fused kernels
   gbn::ClassCtl* ctl = nullptr;       // row-pass control block
 };

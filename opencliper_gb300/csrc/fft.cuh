@@ -49,6 +49,16 @@ constexpr int split_a(int L) { return split_b(L) ? L / split_b(L) : 0; }
 // Data.cpp:1360-1372), 7-smooth (clFFT radices 2,3,5,7), 8..512.
 constexpr bool fft_size_ok(int L) { return L >= 8 && L <= 512 && L % 8 == 0 && is_7smooth(L) && split_b(L) != 0; }
 
+// Split L = PA * PB of the column-pair iteration (rowpair.cuh): PB lanes of a
+// warp hold one pair of columns, PA values each.  Eight lanes (four pairs per
+// warp) while PA stays within 16 values, else sixteen (two pairs).
+constexpr int pair_b(int L) { return (L % 16 != 0 || L / 8 <= 16) ? 8 : 16; }
+constexpr int pair_a(int L) { return L / pair_b(L); }
+constexpr bool pair_split_ok(int L) { return pair_a(L) * pair_b(L) == L && pair_a(L) <= 32; }
+constexpr int pair_np(int L) { return 32 / pair_b(L); }   // column pairs per warp
+constexpr int pair_cols(int L) { return 2 * pair_np(L); }  // columns per tile
+constexpr int pair_ts(int L) { return pair_a(L) | 1; }    // twiddle row stride: rows start in different banks
+
 // ---------------------------------------------------------------------------
 // Multiply by the compile-time forward twiddle w_N^J = e^{-2*pi*i*J/N};
 // trivial angles avoid multiplications.

@@ -4,6 +4,7 @@
 #include "nesta_kernels.cuh"
 #include "registry.h"
 #include "rowlocal.cuh"
+#include "rowpair.cuh"
 
 namespace gbn {
 
@@ -63,7 +64,18 @@ struct Launchers {
     }
   }
   static void iter_cols(const FusedArgs* tab, const BatchMap& bm, int it, bool motion, dim3 grid, cudaStream_t s) {
-    if constexpr (iter_cols_ok(L)) {
+    if constexpr (iter_pair_ok(L)) {
+      using P = PairShape<L>;
+      static bool ok0 = false, ok1 = false;
+      const int ncg = int(grid.x) * kWB / P::COLS, frames = int(grid.z);
+      if (motion) {
+        allow_smem(k_iter_pair<L, true>, P::BYTES, ok1);
+        launch_pdl(k_iter_pair<L, true>, dim3(ncg, frames), kPairNT, P::BYTES, s, tab, bm, it, 0);
+      } else {
+        allow_smem(k_iter_pair<L, false>, P::BYTES, ok0);
+        launch_pdl(k_iter_pair<L, false>, dim3(ncg, frames + cdiv(bm.n, ncg)), kPairNT, P::BYTES, s, tab, bm, it, 0);
+      }
+    } else if constexpr (iter_cols_ok(L)) {
       static bool ok0 = false, ok1 = false;
       if (motion) {
         allow_smem(k_iter_cols<L, true>, IterColsSmem<L>::BYTES, ok1);
@@ -72,6 +84,15 @@ struct Launchers {
         allow_smem(k_iter_cols<L, false>, IterColsSmem<L>::BYTES, ok0);
         launch_pdl(k_iter_cols<L, false>, grid, IterColsSmem<L>::NT, IterColsSmem<L>::BYTES, s, tab, bm, it);
       }
+    }
+  }
+  static void iter_finish(const FusedArgs* tab, const BatchMap& bm, int it, dim3 grid, cudaStream_t s) {
+    if constexpr (iter_pair_ok(L)) {
+      using P = PairShape<L>;
+      static bool ok = false;
+      allow_smem(k_iter_pair<L, false>, P::BYTES, ok);
+      const int ncg = int(grid.x) * kWB / P::COLS;
+      launch_pdl(k_iter_pair<L, false>, dim3(ncg, cdiv(bm.n, ncg)), kPairNT, P::BYTES, s, tab, bm, it, int(grid.z));
     }
   }
   static void fft_rows(const float2* in, float2* out, int nrows, int inv, float scale, const float2* tw, int grid,
@@ -85,7 +106,7 @@ struct Launchers {
   static SizeKernels entry() {
     static_assert(fft_size_ok(L), "unsupported transform length");
     return SizeKernels{L, &fwd_cols, &rows, &inv_cols, &fft_rows, &fft_cols,
-                       iter_cols_ok(L) ? &iter_cols : nullptr, RowCfg<L>::RPC, &rows_occupancy};
+                       iter_cols_ok(L) ? &iter_cols : nullptr, &iter_finish, iter_pair_ok(L) ? pair_cols(L) : 0, RowCfg<L>::RPC, &rows_occupancy};
   }
 };
 

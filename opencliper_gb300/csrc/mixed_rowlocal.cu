@@ -115,7 +115,7 @@ __global__ void __maxnreg__(224)
   __shared__ uint32_t tslot;
   __shared__ float s_isig3[128];  // per-pair scale of the adjoint B operand
   __shared__ float s_cmx[kRtNT / 32][kRtCols];
-  __shared__ double sred[kRtNT / 32];
+  __shared__ double sred[3 * (kRtNT / 32)];
   __shared__ float fm[kFmeanCopy];
 
   const int inst = find_inst(bm, blockIdx.z);
@@ -493,7 +493,7 @@ __global__ void __maxnreg__(224)
     a.part_tv[2 * blk + 1] = t2;
   }
   if (rowlocal_last_cta(bm.ctl, inst, gridDim.x * unsigned(F)))
-    rowlocal_finish<kRtNT>(a, st, bm.ctl, inst, it, apk, a.ntv, a.ntv, sred, fm);
+    rowlocal_finish<kRtNT>(a, st, bm.ctl, inst, it, apk, a.part_tv, a.ntv, a.part_r, a.ntv, sred, fm);
 }
 
 // ---------------------------------------------------------------------------

@@ -1011,8 +1011,14 @@ int nesta_run_mc(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, floa
     // (the update gathering M^T g itself, without k_mc_adjoint, measured
     // slower: 20.7 against 16.7 ms per reconstruction at 256x256x20, 12 coils)
     const unsigned n_iter_launch = prm->maxIter + (prm->stoptest == 1 ? 1u : 0u);
+    if (kh->pair_cols) ctx->launches += launch_pair_setup(ctx, P, tab, s);
     for (unsigned nl = 1; nl <= prm->maxIntIter; ++nl) {
-      ctx->launches += launch_outer_begin(ctx, P, int(nl), x_out, s);
+      if (kh->pair_cols) {  // the gathers read x_k in the natural order
+        ctx->launches += launch_outer_begin_pair(ctx, P, int(nl), x_out, s);
+        cudaMemcpyAsync(P->xk0, x_out, size_t(W) * H * F * sizeof(float2), cudaMemcpyDeviceToDevice, s);
+      } else {
+        ctx->launches += launch_outer_begin(ctx, P, int(nl), x_out, s);
+      }
       for (unsigned it = 0; it < n_iter_launch; ++it) {
         launch_pdl(k_mc_tv, gtv, kNT, 0, s, (const float2*)P->xk0, (const float2*)P->xk1, int(it),
                    (const float*)P->mc_xn, (const int*)t->inv, r, (const NestaDevState*)P->st, P->mc_g, t->tvpart, W,

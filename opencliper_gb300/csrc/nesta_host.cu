@@ -402,6 +402,23 @@ __global__ void k_setup(NestaDevState* st) {
   s.tolVar = 0.1f;
 }
 
+__device__ void outer_begin_state(NestaDevState* st, int nl, float* fmean) {
+  NestaDevState& s = *st;
+  s.outer_active = 1;
+  s.nl = nl;
+  s.mu = s.mu * s.gamma;
+  s.tolVar = s.tolVar * s.gammat;
+  s.Ak = 0.0f;
+  float Lmu = s.normU / s.mu;
+  if (s.miniter > 0) fmean[s.miniter - 1] = float(LONG_MAX);
+  Lmu = s.lambda * Lmu + s.La;
+  s.Lmu = Lmu;
+  s.Lmu1 = 1.0f / Lmu;
+  s.qpDone = 0;
+  s.fixup = 0;
+  s.last_iter = s.maxIter - 1;
+}
+
 // Start of an outer (continuation) loop (NestaUp.cpp:604-648):
 // mu and tolVar updates, Lmu, w = 0, x_k = x_ref.
 __global__ void k_outer_begin(NestaDevState* st, int nl, float* fmean, const float2* __restrict__ xref,
@@ -414,25 +431,115 @@ __global__ void k_outer_begin(NestaDevState* st, int nl, float* fmean, const flo
     }
     return;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    NestaDevState& s = *st;
-    s.outer_active = 1;
-    s.nl = nl;
-    s.mu = s.mu * s.gamma;
-    s.tolVar = s.tolVar * s.gammat;
-    s.Ak = 0.0f;
-    float Lmu = s.normU / s.mu;
-    if (s.miniter > 0) fmean[s.miniter - 1] = float(LONG_MAX);
-    Lmu = s.lambda * Lmu + s.La;
-    s.Lmu = Lmu;
-    s.Lmu1 = 1.0f / Lmu;
-    s.qpDone = 0;
-    s.fixup = 0;
-    s.last_iter = s.maxIter - 1;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) outer_begin_state(st, nl, fmean);
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
     xk0[i] = xref[i];
     wacc[i] = make_float2(0.f, 0.f);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Tiles of the column-pair row-local iteration (rowpair.cuh).  A tile holds the
+// columns [cg*2NP, (cg+1)*2NP) as [row][pair], each pair of adjacent columns
+// planar: (re0, re1, im0, im1).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float4 planar_pair(const float2* src) {
+  const float2 u = src[0], v = src[1];  // the caller's images are 8-byte aligned
+  return make_float4(u.x, v.x, u.y, v.y);
+}
+
+// One warp per frame: the kept rows of every second-pass item k1 (rows k1 +
+// PA*k2; PA <= 32, PB <= 16) and their staged slots in (k1, k2) order.
+__global__ void __launch_bounds__(32) k_pair_tables(const int* __restrict__ rowmap, const int* __restrict__ rowoff,
+                                                    const int* __restrict__ row_full, int H, int PA, int PB,
+                                                    uint4* __restrict__ ptab, int* __restrict__ rowslot) {
+  const int f = blockIdx.x, t = threadIdx.x, rowbase = rowoff[f];
+  unsigned mk = 0, ms = 0;
+  int n = 0;
+  if (t < PA) {
+    for (int k2 = 0; k2 < PB; ++k2) {
+      const int j = rowmap[f * H + t + PA * k2];
+      if (j >= 0) {
+        mk |= 1u << k2;
+        ms |= (row_full[rowbase + j] ? 1u : 0u) << k2;
+      }
+    }
+    n = __popc(mk);
+  }
+  int end = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, end, o);
+    if (t >= o) end += v;
+  }
+  if (t < PA) {
+    int q = end - n;
+    ptab[f * PA + t] = make_uint4(mk, ms, unsigned(q), 0u);
+    for (int k2 = 0; k2 < PB; ++k2) {
+      const int j = rowmap[f * H + t + PA * k2];
+      if (j >= 0) rowslot[rowbase + j] = q++;
+    }
+  }
+}
+
+// S and the kept rows' IDFT_W(y) into tiles (two adjacent columns per thread
+// and step).  Skipped when the rows do not suit the row-local iteration: they
+// may then exceed Tt (the run or replay reports it).
+__global__ void __launch_bounds__(256) k_pair_pack(const FusedArgs* __restrict__ tab, float4* __restrict__ St,
+                                                   float4* __restrict__ Tt, const int* __restrict__ rowslot, int NP) {
+  const FusedArgs& a = *tab;
+  if (a.st->partial_rows) return;
+  const int W = a.W, H = a.H, C = a.C, WQ = W / 2;
+  const size_t nS = size_t(C) * H * WQ, nT = size_t(a.rowoff[a.F]) * C * WQ;
+  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < nS + nT; i += size_t(gridDim.x) * blockDim.x) {
+    if (i < nS) {
+      const int q = int(i % WQ);
+      const size_t cr = i / WQ, c = cr / H, row = cr % H;
+      St[((c * (WQ / NP) + q / NP) * H + row) * NP + q % NP] = planar_pair(a.S + 2 * i);
+    } else {
+      const size_t k = i - nS, gc = k / WQ;
+      const int q = int(k % WQ), c = int(gc % C), g = int(gc / C), f = a.rows_f[g];
+      const size_t base = size_t(a.rowoff[f]) * C * WQ, nr = a.rowoff[f + 1] - a.rowoff[f];
+      Tt[base + ((size_t(q / NP) * C + c) * nr + rowslot[g]) * NP + q % NP] = planar_pair(a.T + 2 * k);
+    }
+  }
+}
+
+// x_ref into tiles at the start of an outer loop, and the scalar state as
+// k_outer_begin leaves it
+__global__ void __launch_bounds__(256) k_outer_begin_pair(NestaDevState* st, int nl, float* fmean,
+                                                          const float2* __restrict__ xref, float4* __restrict__ xt,
+                                                          int W, int H, size_t n2, int NP) {
+  if (nl > st->maxIntIter) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      st->outer_active = 0;
+      st->last_iter = -1;
+    }
+    return;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) outer_begin_state(st, nl, fmean);
+  const int WQ = W / 2;
+  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n2; i += size_t(gridDim.x) * blockDim.x) {
+    const int q = int(i % WQ);
+    const size_t fr = i / WQ, f = fr / H, row = fr % H;
+    xt[((f * (WQ / NP) + q / NP) * H + row) * NP + q % NP] = planar_pair(xref + 2 * i);
+  }
+}
+
+// End of an outer loop from tiles: x_ref = x_k (nothing ran: x_ref stays)
+__global__ void __launch_bounds__(256) k_outer_end_pair(const NestaDevState* st, const float4* __restrict__ xk0,
+                                                        const float4* __restrict__ xk1, const float4* __restrict__ xk2,
+                                                        float2* __restrict__ xref, int W, int H, size_t n2, int NP) {
+  if (!st->outer_active || st->last_iter < 0) return;
+  const int k3 = (st->last_iter + 1) % 3;
+  const float4* src = k3 == 0 ? xk0 : k3 == 1 ? xk1 : xk2;
+  const int WQ = W / 2;
+  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n2; i += size_t(gridDim.x) * blockDim.x) {
+    const int q = int(i % WQ);
+    const size_t fr = i / WQ, f = fr / H, row = fr % H;
+    const float4 v = src[((f * (WQ / NP) + q / NP) * H + row) * NP + q % NP];
+    xref[2 * i] = make_float2(v.x, v.z);
+    xref[2 * i + 1] = make_float2(v.y, v.w);
   }
 }
 
@@ -513,6 +620,17 @@ int problem_alloc(gbn_problem* P) {
   A((void**)&P->wacc, X * sizeof(float2));
   A((void**)&P->wacc1, X * sizeof(float2));
   A((void**)&P->st, sizeof(NestaDevState));
+  const SizeKernels* kh = find_size(P->H);
+  if (kh && kh->pair_cols) {
+    P->Tt_rows = size_t(P->F) * std::min(P->H, iter_cols_rcap(P->H));
+    A((void**)&P->St, size_t(P->C) * P->H * P->W * sizeof(float2));
+    A((void**)&P->Tt, P->Tt_rows * P->C * P->W * sizeof(float2));
+    A((void**)&P->xt, X * sizeof(float2));
+    A((void**)&P->xk2, X * sizeof(float2));
+    A((void**)&P->wacc2, X * sizeof(float2));
+    A((void**)&P->ptab, size_t(P->F) * pair_a(P->H) * sizeof(uint4));
+    A((void**)&P->rowslot, FH * sizeof(int));
+  }
   A((void**)&P->d_args, sizeof(FusedArgs));
   A((void**)&P->ctl, sizeof(ClassCtl));
   if (e != cudaSuccess) {
@@ -546,6 +664,18 @@ int problem_fit_rows(gbn_problem* P, int headroom, int* kept) {
           cudaFree(P->T);
           P->T = nt;
           P->T_rows = want;
+          // the tiles follow: never more than the row-local iteration takes
+          const size_t tt = std::min<size_t>(want, size_t(P->F) * std::min(P->H, iter_cols_rcap(P->H)));
+          if (P->Tt && tt != P->Tt_rows) {
+            cudaFree(P->Tt);
+            P->Tt = nullptr;
+            P->Tt_rows = 0;
+            if ((e = cudaMalloc(&P->Tt, std::max<size_t>(tt, 1) * P->C * P->W * sizeof(float2))) != cudaSuccess) {
+              cudaGetLastError();
+              return set_error(GBN_ERR_NOMEM, "row buffer allocation failed");
+            }
+            P->Tt_rows = tt;
+          }
           if (kept) *kept = g;
           return GBN_OK;
         }
@@ -567,7 +697,9 @@ void motion_free(gbn_problem* P);
 void problem_free(gbn_problem* P) {
   void* ptrs[] = {P->flags, P->full_fh, P->rowmap, P->rowoff,  P->rows_h, P->rows_f,  P->row_full, P->T,
                   P->xk0,   P->xk1,     P->wacc,   P->wacc1,  P->st,      P->fmean,  P->part_tv, P->part_r,   P->part_ne,
-                  P->ne_b,  P->d_args,  P->ctl,      P->fk,     P->colmax, P->smax,   P->fa};
+                  P->ne_b,  P->d_args,  P->ctl,      P->fk,     P->colmax, P->smax,   P->fa,
+                  P->St,    P->Tt,      P->xt,     P->ptab,   P->rowslot,
+                  P->xk2,   P->wacc2};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   motion_free(P);
@@ -614,6 +746,16 @@ FusedArgs make_args(gbn_problem* P, float2* xref) {
   a.s_adj = std::sqrt(float(N)) * (1.0f / float(N));        // NestaUp.cpp:749 sqrt(float(N)) times clFFT 1/N
   a.s_row = float(double(P->W) * double(a.s_fwd));
   a.ntv = P->F * (P->W / kWB);
+  a.St = P->St;
+  a.Tt = P->Tt;
+  a.xt = P->xt;
+  float2* const px[3] = {P->xk0, P->xk1, P->xk2};
+  float2* const pw[3] = {P->wacc, P->wacc1, P->wacc2};
+  for (int b = 0; b < 3; ++b) {
+    a.px[b] = reinterpret_cast<float4*>(px[b]);
+    a.pw[b] = reinterpret_cast<float4*>(pw[b]);
+  }
+  a.ptab = P->ptab;
   return a;
 }
 
@@ -651,8 +793,9 @@ int run_prepare(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm) {
   int rc;
   if ((rc = grow(P->fmean, P->fmean_cap, std::max<int>(1, int(prm->miniter)))) != GBN_OK) return rc;
   // one (|u|^2, Re<u,d>) pair per (frame, 8-column tile) and coil half (row-local iteration)
-  if ((rc = grow(P->part_tv, P->part_tv_cap, 4 * F * (W / kWB))) != GBN_OK) return rc;
-  if ((rc = grow(P->part_r, P->part_r_cap, std::max(int(steps_max) * kRowWarps, 2 * F * (W / kWB)))) != GBN_OK)
+  // (two sets for the column pairs, which sum one iteration while the next runs)
+  if ((rc = grow(P->part_tv, P->part_tv_cap, (kh->pair_cols ? 8 : 4) * F * (W / kWB))) != GBN_OK) return rc;
+  if ((rc = grow(P->part_r, P->part_r_cap, std::max(int(steps_max) * kRowWarps, 4 * F * (W / kWB)))) != GBN_OK)
     return rc;
   if ((rc = grow(P->part_ne, P->part_ne_cap, nblk_ne * kNeMaxSlots * 2)) != GBN_OK) return rc;
   if ((rc = grow(P->ne_b, P->ne_b_cap, N * F)) != GBN_OK) return rc;
@@ -712,6 +855,30 @@ int launch_maxima(gbn_ctx* ctx, gbn_problem* P, const float2* x0, const float2* 
 
 int launch_setup(gbn_problem* P, cudaStream_t s) {
   k_setup<<<1, 1, 0, s>>>(P->st);
+  return 1;
+}
+
+int launch_pair_setup(gbn_ctx* ctx, gbn_problem* P, const FusedArgs* tab, cudaStream_t s) {
+  const int H = P->H;
+  k_pair_tables<<<P->F, 32, 0, s>>>(P->rowmap, P->rowoff, P->row_full, H, pair_a(H), pair_b(H), P->ptab, P->rowslot);
+  const size_t n = (size_t(P->C) * H + P->Tt_rows * P->C) * (P->W / 2);
+  k_pair_pack<<<elementwise_grid(ctx, n), 256, 0, s>>>(tab, P->St, P->Tt, P->rowslot, pair_np(H));
+  return 2;
+}
+
+int launch_outer_begin_pair(gbn_ctx* ctx, gbn_problem* P, int nl, const float2* xref, cudaStream_t s) {
+  const size_t n2 = size_t(P->W) * P->H * P->F / 2;
+  k_outer_begin_pair<<<elementwise_grid(ctx, n2), 256, 0, s>>>(P->st, nl, P->fmean, xref, P->xt, P->W, P->H, n2,
+                                                                pair_np(P->H));
+  return 1;
+}
+
+int launch_outer_end_pair(gbn_ctx* ctx, gbn_problem* P, float2* xref, cudaStream_t s) {
+  const size_t n2 = size_t(P->W) * P->H * P->F / 2;
+  k_outer_end_pair<<<elementwise_grid(ctx, n2), 256, 0, s>>>(P->st, reinterpret_cast<const float4*>(P->xk0),
+                                                              reinterpret_cast<const float4*>(P->xk1),
+                                                              reinterpret_cast<const float4*>(P->xk2), xref, P->W,
+                                                              P->H, n2, pair_np(P->H));
   return 1;
 }
 
@@ -816,15 +983,20 @@ int nesta_run(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, float2*
     if ((ef = cudaEventSynchronize(ctx->ev_partial)) != cudaSuccess) return cuda_status(ef, "row structure read-back");
     row_local = *ctx->host_partial == 0;
   }
-  // stopping test on: one more launch per outer loop recomputes the last
-  // update if the rule stops the loop (row-local iteration only)
-  const unsigned n_iter_launch = prm->maxIter + ((row_local && prm->stoptest == 1) ? 1u : 0u);
+  // stopping test on: the launches that recompute the last update if the rule
+  // stops the loop (row-local iteration only; the column pairs run one iteration
+  // ahead of the test)
+  const bool pair = row_local && kh->pair_cols;
+  const unsigned n_iter_launch = prm->maxIter + ((row_local && prm->stoptest == 1) ? (pair ? 2u : 1u) : 0u);
 
+  if (pair) GBN_LAUNCH(ctx, GBN_PROF_SETUP, 2, launch_pair_setup(ctx, P, tab, s));
   for (unsigned nl = 1; nl <= prm->maxIntIter; ++nl) {
-    GBN_LAUNCH(ctx, GBN_PROF_OUTER, 1, launch_outer_begin(ctx, P, int(nl), x_out, s));
+    GBN_LAUNCH(ctx, GBN_PROF_OUTER, 1,
+               pair ? launch_outer_begin_pair(ctx, P, int(nl), x_out, s) : launch_outer_begin(ctx, P, int(nl), x_out, s));
     if (row_local) {
       for (unsigned it = 0; it < n_iter_launch; ++it)
         GBN_LAUNCH(ctx, GBN_PROF_ITER, 1, kh->iter_cols(tab, bm, int(it), false, g3, s));
+      if (pair && prm->stoptest != 1) GBN_LAUNCH(ctx, GBN_PROF_OUTER, 1, kh->iter_finish(tab, bm, int(prm->maxIter), g3, s));
     } else {
       for (unsigned it = 0; it < prm->maxIter; ++it) {
         GBN_LAUNCH(ctx, GBN_PROF_FWD_COLS, 1, kh->fwd_cols(tab, bm, int(it), cpb, g1, s));
@@ -832,7 +1004,8 @@ int nesta_run(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, float2*
         GBN_LAUNCH(ctx, GBN_PROF_INV_COLS, 1, kh->inv_cols(tab, bm, int(it), true, g3, s));
       }
     }
-    GBN_LAUNCH(ctx, GBN_PROF_OUTER, 1, launch_outer_end(ctx, P, x_out, s));
+    GBN_LAUNCH(ctx, GBN_PROF_OUTER, 1,
+               pair ? launch_outer_end_pair(ctx, P, x_out, s) : launch_outer_end(ctx, P, x_out, s));
   }
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_status(e, "nesta launch");

@@ -73,12 +73,13 @@ __device__ __forceinline__ float2 tv_normalize(float2 d, float inv_mu) {
 // and the Nesterov weights (NestaUp.cpp:791-831), executed by one thread.
 // Arithmetic types follow the reference: host floats, std::pow in double.
 // ---------------------------------------------------------------------------
-// `fm` is a copy of the first min(miniter, kFmeanCopy) entries of fmean.
+// `fm` is a copy of the first min(miniter, kFmeanCopy) entries of fmean, `cur`
+// the state itself or a copy of it.
 constexpr int kFmeanCopy = 64;
 __device__ inline void nesta_scalar_step(NestaDevState* gst, float* fmean, const float* fm, int it, double su2,
-                                         double sud, double sr2) {
+                                         double sud, double sr2, const NestaDevState* cur) {
   // work on a register copy: one batch of loads instead of a chain of round trips
-  NestaDevState loc = *gst;
+  NestaDevState loc = *cur;
   NestaDevState* st = &loc;
   const float normUk = float(sqrt(su2));  // Scnrm2(u)
   const float fxdot = float(sud);         // real part of Cdotc(u, d)
@@ -596,7 +597,7 @@ __global__ void __launch_bounds__(kRowNT)
         sud = block_sum<kRowNT>(sud, sred);
         sr2 = block_sum<kRowNT>(sr2, sred);
         if (t == 0) {
-          nesta_scalar_step(st, ai.fmean, fm, it, su2, sud, sr2);
+          nesta_scalar_step(st, ai.fmean, fm, it, su2, sud, sr2, st);
           ctl->done[inst] = 0;
         }
         __syncthreads();

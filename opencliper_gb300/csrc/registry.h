@@ -26,6 +26,9 @@ struct SizeKernels {
   // frames) in clusters of 2; nullptr for lengths that run only the three-pass
   // iteration
   void (*iter_cols)(const FusedArgs* tab, const BatchMap& bm, int it, bool motion, dim3 grid, cudaStream_t s);
+  // the sums and scalar step of iteration it - 1 alone (column-pair form)
+  void (*iter_finish)(const FusedArgs* tab, const BatchMap& bm, int it, dim3 grid, cudaStream_t s);
+  int pair_cols;     // columns per tile of the column-pair form of iter_cols; 0: iter_cols works on natural buffers
   int rows_per_cta;  // rows processed per CTA step by the row kernels
   int (*rows_occupancy)(bool resid);  // resident row-kernel CTAs per SM
 };

@@ -18,8 +18,7 @@
 // and the whole inner iteration runs in one kernel.
 //
 // k_iter_cols<H, MOTION>: grid (W/kWB, 2, frames) in clusters of 2 along y;
-// CTA = (frame, 8 columns, half of the coils), 128 threads (160 at H = 288,
-// 320).  Per coil: forward column DFT of
+// CTA = (frame, 8 columns, half of the coils), 128 threads.  Per coil: forward column DFT of
 // S_c x_f (dit2<A,B>), residual on the kept rows, inverse column DFT
 // (dit2<B,A> of the conjugate) and conj(S_c) accumulation.  The forward
 // pass-2 item (w, k1) holds rows k1 + A*k2, exactly the rows the inverse
@@ -30,9 +29,10 @@
 // The tTV objective terms (Scnrm2, Cdotc of NestaUp.cpp:686-691; each CTA of
 // the pair over half of the tile) and ||r||^2 are written as fixed-slot
 // partial sums; the last CTA of an instance reduces them in fixed order and
-// runs the scalar recurrence (nesta_scalar_step).  Register budgets per length
-// (x and the accumulators in registers or in tensor memory) are set by
-// iter_cols_tmem / iter_cols_threads / iter_cols_min_blocks below.
+// runs the scalar recurrence (nesta_scalar_step).  The lengths whose second
+// factor is 8 or 16 run the column-pair form instead (rowpair.cuh: 256 x 256 x
+// 20 frames x 12 coils 59 us per iteration against 96 us); this kernel remains
+// for 280, 360 and 392.
 //
 // The update of iteration k uses apk = (k+1)/2 and tauk = 2/(k+3), what the
 // scalar recurrence yields unless the stopping test fires for the second time
@@ -104,45 +104,46 @@ __device__ __forceinline__ bool rowlocal_last_cta(ClassCtl* ctl, int inst, unsig
 // order and runs the scalar recurrence; ||E x - y||^2 = sum |rho|^2 / W
 // (Parseval along the rows).  `apk_used` is the weight the CTAs updated with:
 // when the recurrence's differs, the stopping test fired for the second time
-// and the next launch recomputes this iteration's update.  All NT threads call it.
+// and the next launch recomputes this iteration's update.  `unseen` iterations
+// before this one left no sums (the stopping test is off).  All NT threads call it.
+// Everything it reads is requested at once: the state and fmean copies beside
+// the first round of partial sums.  sred holds 3 * NT/32 doubles.
 template <int NT>
 __device__ void rowlocal_finish(const FusedArgs& a, NestaDevState* st, ClassCtl* ctl, int inst, int it, float apk_used,
-                                int ntv, int npr, double* sred, float* fm) {
+                                const double* part_tv, int ntv, const double* part_r, int npr, double* sred, float* fm,
+                                int unseen = 0) {
+  constexpr int SW = int(sizeof(NestaDevState) / 4);
+  static_assert(sizeof(NestaDevState) % 4 == 0 && SW <= NT, "the state is copied a word per thread");
+  __shared__ uint32_t s_st[SW];
   const int t = threadIdx.x;
   __threadfence();
-  if (t < kFmeanCopy && t < st->miniter) fm[t] = __ldcg(a.fmean + t);
+  if (t < SW) s_st[t] = __ldcg(reinterpret_cast<const uint32_t*>(st) + t);
+  if (t < kFmeanCopy && t < __ldcg(&st->miniter)) fm[t] = __ldcg(a.fmean + t);
   constexpr int U = 8;
   double s1 = 0.0, s2 = 0.0, s3 = 0.0;
-  const double2* ptv = reinterpret_cast<const double2*>(a.part_tv);
-  for (int i0 = 0; i0 < ntv; i0 += U * NT) {
+  const double2* ptv = reinterpret_cast<const double2*>(part_tv);
+  for (int i0 = 0; i0 < ntv || i0 < npr; i0 += U * NT) {
     double2 vv[U];
+    double vr[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = i0 + u * NT + t;
       vv[u] = (i < ntv) ? __ldcg(ptv + i) : make_double2(0.0, 0.0);
+      vr[u] = (i < npr) ? __ldcg(part_r + i) : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       s1 += vv[u].x;
       s2 += vv[u].y;
+      s3 += vr[u];
     }
   }
-  for (int i0 = 0; i0 < npr; i0 += U * NT) {
-    double vv[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int i = i0 + u * NT + t;
-      vv[u] = (i < npr) ? __ldcg(a.part_r + i) : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) s3 += vv[u];
-  }
-  s1 = block_sum<NT>(s1, sred);
-  s2 = block_sum<NT>(s2, sred);
-  s3 = block_sum<NT>(s3, sred);
+  double r1, r2, r3;
+  rowlocal_block_sum3<NT>(s1, s2, s3, sred, &r1, &r2, &r3);
   if (t == 0) {
-    nesta_scalar_step(st, a.fmean, fm, it, s1, s2, s3 / double(a.W));
+    nesta_scalar_step(st, a.fmean, fm, it, r1, r2, r3 / double(a.W), reinterpret_cast<const NestaDevState*>(s_st));
     if (st->apk != apk_used) st->fixup = 1;
+    st->iters_total += unseen;
     ctl->done[inst] = 0;
   }
 }
@@ -163,12 +164,9 @@ __device__ __forceinline__ float2 twiddle(const float2* row, int m) {
   }
 }
 
-// Lengths whose x values and coil accumulators live in tensor memory instead
-// of registers: first factors above 16 with one pass-1 and one inverse pass-2
-// item per thread (H = 288, 320, 336, 384).  With the registers this frees and
-// a single S buffer, three CTAs share an SM at H = 320 and 384 instead of two
-// (measured: 1.28x at 384 x 384).  At H = 256 the register form is faster.
-constexpr bool iter_cols_tmem(int L) { return split_a(L) > 16 && kWB * split_b(L) == kColNT; }
+// k_iter_cols keeps x and the accumulators in registers at every length it
+// runs (the column-pair form of rowpair.cuh uses tensor memory).
+constexpr bool iter_cols_tmem(int) { return false; }
 
 // Calls fn(offset, count) for consecutive pieces of F TMEM columns: pieces of
 // 16, then one each of 8, 4 and 2 as F requires (F even); every piece starts
@@ -194,29 +192,14 @@ __device__ __forceinline__ void tmem_st_n(uint32_t taddr, const float* v) {
   if constexpr (N == 16) tc::tmem_st16(taddr, v);
   else tc::tmem_st_small<N>(taddr, v);
 }
-constexpr int iter_cols_sbufs(int L) { return iter_cols_tmem(L) ? 1 : 2; }
-
-// Threads per CTA: 128, or for the tensor-memory lengths one per pass-2 item
-// (kWB * A of them, rounded up to whole warps) where three such CTAs still fit
-// at 128 registers a thread (H = 288, 320: 160 threads).  With 128 threads
-// those items fall twice to some threads and the pass waits for them; more
-// threads at fewer CTAs per SM measured slower (H = 384: 288 us per iteration
-// with 192 threads at two CTAs, against 280 us).  The pass-1 and pass-3 items
-// (kWB * B = 128) stay on warps 0-3, whose tensor-memory lanes hold their state.
-// Short columns with at most 64 pass-2 items (A <= 8: H = 64, 96, 128 ...)
-// run 64 threads with two pass-1 and pass-3 items each, so no thread idles in
-// pass 2, at twice the CTAs per SM.
-constexpr int iter_cols_threads(int L) {
-  return (iter_cols_tmem(L) && (kWB * split_a(L) + 31) / 32 * 32 * 3 * 128 <= 65536) ? (kWB * split_a(L) + 31) / 32 * 32
-         : (!iter_cols_tmem(L) && kWB * split_a(L) <= 64 && kWB * split_b(L) == kColNT) ? 64
-                                                                                        : kColNT;
-}
+// Threads per CTA of k_iter_cols.
+constexpr int iter_cols_threads(int) { return kColNT; }
 
 // Shared-memory bytes of k_iter_cols<L> (the layout of IterColsSmem<L>).
 constexpr int iter_cols_bytes(int L) {
   const int a = split_a(L), b = split_b(L);
   const int ex = (a * col_ks(b) > b * col_ks(a)) ? a * col_ks(b) : b * col_ks(a);
-  return (iter_cols_sbufs(L) * L * kWB + 2 * iter_cols_rcap(L) * kWB + ex + b * (a + 2) + a * (b + 2)) * 8 + L * 4 +
+  return (2 * L * kWB + 2 * iter_cols_rcap(L) * kWB + ex + b * (a + 2) + a * (b + 2)) * 8 + L * 4 +
          3 * (iter_cols_threads(L) / 32) * 8 + kFmeanCopy * 4 + 16;
 }
 
@@ -230,9 +213,8 @@ struct IterColsSmem {
   static constexpr int KSI = col_ks(A);  // inverse exchange: slot (k1', s'*kWB + w), k1' < B
   static constexpr int EXN = (A * KSF > B * KSI) ? A * KSF : B * KSI;
   static constexpr int RCAP = iter_cols_rcap(H);         // kept rows whose IDFT_W(y) is staged
-  static constexpr int SB = iter_cols_sbufs(H);          // S buffers: 2 (next coil copied during this one) or 1
-  static constexpr int S_OFF = 0;                        // float2 [SB][H][kWB]
-  static constexpr int Y_OFF = S_OFF + SB * H * kWB;     // float2 [2][RCAP][kWB]
+  static constexpr int S_OFF = 0;                        // float2 [2][H][kWB]
+  static constexpr int Y_OFF = S_OFF + 2 * H * kWB;      // float2 [2][RCAP][kWB]
   static constexpr int EX_OFF = Y_OFF + 2 * RCAP * kWB;  // float2 [EXN]
   // twiddles: B rows of A (forward first pass, one row per item s) and A rows
   // of B (inverse first pass, one per item k1), each row padded by one 16-byte
@@ -242,35 +224,25 @@ struct IterColsSmem {
   static constexpr int TWI_OFF = B * TWF;                // inverse rows, from TW_OFF
   static constexpr int F2_END = TW_OFF + TWI_OFF + A * TWI;
   static constexpr int BYTES = F2_END * 8 + H * 4 + 3 * (NT / 32) * 8 + kFmeanCopy * 4 + 16;
-  static_assert(NI3 * A * XST <= SB * H * kWB, "accumulator exchange must fit the S buffers");
+  static_assert(NI3 * A * XST <= 2 * H * kWB, "accumulator exchange must fit the S buffers");
   static_assert(BYTES == iter_cols_bytes(H), "layout and byte count agree");
   static_assert(TW_OFF % 2 == 0, "twiddle rows start on 16-byte boundaries");
 };
 
 
-// CTAs per SM the launch bounds ask for.  With x and the accumulators in
-// tensor memory, as many as shared memory allows and keep 128 registers a
-// thread (at most three); otherwise a
-// first factor A <= 16 keeps the per-thread state (x at the pass-1 items, the
-// accumulators, one pass-2 item) within 168 registers at three CTAs per SM,
-// and longer first factors hold more per thread at the two CTAs per SM (one
-// past 448) their shared memory allows, with up to 255 registers a thread.
+// CTAs per SM the launch bounds ask for: a first factor A <= 16 keeps the
+// per-thread state (x at the pass-1 items, the accumulators, one pass-2 item)
+// within 168 registers at three CTAs per SM; longer ones take two (one past
+// 448) with up to 255 registers a thread.
 constexpr int iter_cols_min_blocks(int H) {
-  if (iter_cols_tmem(H)) {
-    const int by_smem = (228 * 1024) / (iter_cols_bytes(H) + 1024);
-    const int by_regs = 65536 / (iter_cols_threads(H) * 128);  // at least 128 registers a thread
-    const int m = by_smem < by_regs ? by_smem : by_regs;
-    return m < 3 ? m : 3;
-  }
-  if (iter_cols_threads(H) == 64) return 6;
   return split_a(H) <= 16 ? 3 : (iter_cols_bytes(H) + 1024 <= 114 * 1024 ? 2 : 1);
 }
 
-// Lengths that run the row-local iteration; the others (whose per-thread
-// state would spill) run the three-pass iteration.
+// Lengths that run the row-local iteration, in this form or as column pairs;
+// the others (200, 216, 504) run the three-pass iteration.
 constexpr bool iter_cols_ok(int H) {
-  return split_a(H) != 0 && (split_a(H) <= 16 || (split_b(H) >= 8 && split_b(H) <= 16 && split_a(H) <= 24) ||
-                             (iter_cols_tmem(H) && split_a(H) <= 32));
+  return split_a(H) != 0 &&
+         (split_a(H) <= 16 || (split_b(H) == 8 && split_a(H) <= 24) || (split_b(H) == 16 && split_a(H) <= 32));
 }
 
 // MOTION: the motion-compensated form (tTV gradient M^T(tTVadj u) and the
@@ -284,13 +256,6 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(iter_cols_threads(H)
   constexpr int N2 = kWB * A;  // forward pass-2 = inverse pass-1 items (w, k1), k1 < A: rows k1 + A*k2
   constexpr int N3 = kWB * B;  // inverse pass-2 items (w, k1'), k1' < B: rows k1' + B*k2
   constexpr int NI1 = cdiv(N1, NT), NI2 = cdiv(N2, NT), NI3 = cdiv(N3, NT);
-  // tensor memory: columns [0, 2A) x at the pass-1 item, [ACC0, ACC0 + 2A) the accumulators
-  constexpr bool TM = iter_cols_tmem(H);
-  constexpr int ACC0 = (2 * A + 15) / 16 * 16;
-  constexpr uint32_t TCOLS = (ACC0 + 2 * A <= 32) ? 32u : (ACC0 + 2 * A <= 64) ? 64u : 128u;
-  static_assert(!TM || (N1 == kColNT && N3 == kColNT && NI1 == 1 && NI3 == 1 && ACC0 + 2 * A <= 128),
-                "one pass-1 and one pass-3 item on each thread of warps 0-3");
-  __shared__ uint32_t tslot;
   extern __shared__ float4 smem4[];
   float2* Sb = reinterpret_cast<float2*>(smem4) + L::S_OFF;
   float2* Yb = reinterpret_cast<float2*>(smem4) + L::Y_OFF;
@@ -326,7 +291,7 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(iter_cols_threads(H)
   const float2* const s_src0 = a.S + size_t(srow) * W + w0 + 2 * spart;
   const float2* const t_src0 = a.T + size_t(rowbase) * C * W + w0;
   auto issue_S = [&](int c, int buf) {
-    float2* dst = Sb + (L::SB == 2 ? buf : 0) * H * kWB;
+    float2* dst = Sb + buf * H * kWB;
     if constexpr (H % RSTEP == 0) {
       const float2* src = s_src0 + size_t(c) * N;
       float2* d0 = dst + srow * kWB + 2 * spart;
@@ -409,17 +374,6 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(iter_cols_threads(H)
   const float2* __restrict__ x = xk + size_t(f) * N;
   const float inv_mu = 1.0f / st->mu;
 
-  uint32_t tl = 0;  // this thread's TMEM lane
-  if constexpr (TM) {
-    if (t < 32) {
-      tc::tmem_alloc(&tslot, TCOLS);
-      tc::tmem_relinquish();
-    }
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    tl = tslot + (uint32_t(32 * (t >> 5)) << 16);
-  }
   // x_k at this thread's forward pass-1 items, reused for every coil
   float2 xv[NI1][A];
 #pragma unroll
@@ -437,21 +391,6 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(iter_cols_threads(H)
   for (int ii = 0; ii < NI3; ++ii)
 #pragma unroll
     for (int k2 = 0; k2 < A; ++k2) acc[ii][k2] = make_float2(0.f, 0.f);
-  if constexpr (TM) {  // x and the zeroed accumulators move to tensor memory for the coil loop
-    if (t < N1) tmem_pieces<2 * A>([&](auto oc, auto nc) {
-      constexpr int o = decltype(oc)::value, n = decltype(nc)::value;
-      float xf[n], zf[n];
-#pragma unroll
-      for (int e = 0; e < n / 2; ++e) {
-        xf[2 * e] = xv[0][o / 2 + e].x;
-        xf[2 * e + 1] = xv[0][o / 2 + e].y;
-        zf[2 * e] = zf[2 * e + 1] = 0.f;
-      }
-      tmem_st_n<n>(tl + o, xf);
-      tmem_st_n<n>(tl + ACC0 + o, zf);
-    });
-    if (t < N1) tc::tmem_wait_st();
-  }
   const float s_row = a.s_row;
   float racc = 0.f;
   // kept rows of each pass-2 item (w, k1): bit k2 for row k1 + A*k2
@@ -472,11 +411,11 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(iter_cols_threads(H)
     cp_async_wait<0>();
     __syncthreads();  // coil c staged; the previous coil's inverse pass 2 has read the exchange
     if (c + 1 < cend) {
-      if constexpr (L::SB == 2) issue_S(c + 1, buf ^ 1);  // one buffer: copied once this coil's pass 2 read S
+      issue_S(c + 1, buf ^ 1);
       issue_Y(c + 1, buf ^ 1);
     }
     cp_async_commit();
-    const float2* Sc = Sb + (L::SB == 2 ? buf : 0) * H * kWB;
+    const float2* Sc = Sb + buf * H * kWB;
     const float2* Yc = Yb + buf * RCAP * kWB;
     // forward pass 1: S_c x_f, DFT_A, twiddles
 #pragma unroll
@@ -485,19 +424,8 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(iter_cols_threads(H)
       if (i < N1) {
         const int w = i % kWB, s = i / kWB;
         float2 v[A];
-        if constexpr (TM) {
-          tmem_pieces<2 * A>([&](auto oc, auto nc) {
-            constexpr int o = decltype(oc)::value, n = decltype(nc)::value;
-            float xf[n];
-            tmem_ld_n<n>(tl + o, xf);
 #pragma unroll
-            for (int e = 0; e < n / 2; ++e)
-              v[o / 2 + e] = cmul(make_float2(xf[2 * e], xf[2 * e + 1]), Sc[(B * (o / 2 + e) + s) * kWB + w]);
-          });
-        } else {
-#pragma unroll
-          for (int n1 = 0; n1 < A; ++n1) v[n1] = cmul(xv[ii][n1], Sc[(B * n1 + s) * kWB + w]);
-        }
+        for (int n1 = 0; n1 < A; ++n1) v[n1] = cmul(xv[ii][n1], Sc[(B * n1 + s) * kWB + w]);
         dft<A>(v);
 #pragma unroll
         for (int k1 = 0; k1 < A; ++k1) ex[k1 * KSF + s * kWB + w] = (k1 == 0) ? v[k1] : cmul(v[k1], twiddle<A>(tws + s * L::TWF, k1));
@@ -557,50 +485,10 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(iter_cols_threads(H)
           const float2 sv = Sc[(k1p + B * k2) * kWB + w];
           return make_float2(fmaf(v[k2].x, sv.x, -v[k2].y * sv.y), fmaf(-v[k2].x, sv.y, -(v[k2].y * sv.x)));
         };
-        if constexpr (TM) {
-          tc::tmem_wait_st();  // the previous coil's accumulator stores
-          tmem_pieces<2 * A>([&](auto oc, auto nc) {
-            constexpr int o = decltype(oc)::value, n = decltype(nc)::value;
-            float af[n];
-            tmem_ld_n<n>(tl + ACC0 + o, af);
 #pragma unroll
-            for (int e = 0; e < n / 2; ++e) {
-              const float2 sum = padd(make_float2(af[2 * e], af[2 * e + 1]), term(o / 2 + e));
-              af[2 * e] = sum.x;
-              af[2 * e + 1] = sum.y;
-            }
-            tmem_st_n<n>(tl + ACC0 + o, af);
-          });
-        } else {
-#pragma unroll
-          for (int k2 = 0; k2 < A; ++k2) acc[ii][k2] = padd(acc[ii][k2], term(k2));
-        }
+        for (int k2 = 0; k2 < A; ++k2) acc[ii][k2] = padd(acc[ii][k2], term(k2));
       }
     }
-    if constexpr (L::SB == 1) {  // one S buffer: the next coil's copy starts once every thread has read this one
-      if (c + 1 < cend) {
-        __syncthreads();
-        issue_S(c + 1, 0);
-        cp_async_commit();
-      }
-    }
-  }
-  if constexpr (TM) {  // x and the accumulators back to registers; the tensor memory is released
-    if (t < N1) tc::tmem_wait_st();
-    if (t < N1) tmem_pieces<2 * A>([&](auto oc, auto nc) {
-      constexpr int o = decltype(oc)::value, n = decltype(nc)::value;
-      float xf[n], af[n];
-      tmem_ld_n<n>(tl + o, xf);
-      tmem_ld_n<n>(tl + ACC0 + o, af);
-#pragma unroll
-      for (int e = 0; e < n / 2; ++e) {
-        xv[0][o / 2 + e] = make_float2(xf[2 * e], xf[2 * e + 1]);
-        acc[0][o / 2 + e] = make_float2(af[2 * e], af[2 * e + 1]);
-      }
-    });
-    tc::fence_before_sync();
-    __syncthreads();
-    if (t < 32) tc::tmem_dealloc(tslot, TCOLS);
   }
 
   // tTV objective partial sums over the tile, each CTA of the pair over half
@@ -624,12 +512,8 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(iter_cols_threads(H)
     }
   }
 
-  // This CTA finishes half of the tile's rows (k2 < A/2 for the first).  The
-  // update's operands at those rows (x_k and its neighbouring frames, w_k,
-  // x_ref: independent of the accumulators) are requested between the two
-  // halves of the cluster barrier below, so that they arrive during the
-  // exchange.
-  constexpr int KH = A / 2, KM = A - KH;
+  // This CTA finishes half of the tile's rows (k2 < A/2 for the first).
+  constexpr int KH = A / 2;
   const int kb = half ? KH : 0, ke = half ? A : KH;
   const size_t offm = size_t((f + F - 1) % F) * N, off0 = size_t(f) * N, offp = size_t((f + 1) % F) * N;
   // Sum the two halves' accumulators through distributed shared memory.
@@ -641,35 +525,9 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(iter_cols_threads(H)
 #pragma unroll
     for (int k2 = 0; k2 < A; ++k2)  // the rows the other CTA finishes
       if ((k2 < kb || k2 >= ke) && t + ii * NT < N3) mine[(ii * A + k2) * L::XST + t] = acc[ii][k2];
-  // the cluster barrier in two halves: the arrive publishes this CTA's rows
-  // (release), the update's operands are requested while the partner gets
-  // there, and the wait makes the partner's rows visible (acquire)
+  // the arrive publishes this CTA's rows (release), the wait makes the
+  // partner's visible (acquire)
   asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-  // (x_k, w_k and x_ref for every form with one pass-3 item per thread and
-  // A <= 24 at 168 registers a thread; the neighbouring frames too for the
-  // plain form at A <= 16; the rest after the exchange)
-  constexpr bool PRE = NI3 == 1 && (A <= 16 || (A <= 24 && NT == kColNT));
-  constexpr bool PRE_T = PRE && !MOTION && A <= 16;
-  float2 pxa[PRE ? KM : 1], pxm[PRE ? KM : 1], pxp[PRE ? KM : 1], pwo[PRE ? KM : 1], pxr[PRE ? KM : 1];
-  if constexpr (PRE) {
-    if (t < N3) {
-      const int w = t % kWB, k1p = t / kWB;
-#pragma unroll
-      for (int k = 0; k < KM; ++k) {
-        if (kb + k < ke) {
-          const size_t p = size_t(k1p + B * (kb + k)) * W + w0 + w;
-          pxa[k] = xk[off0 + p];
-          if constexpr (PRE_T) {
-            pxm[k] = xk[offm + p];
-            pxp[k] = xk[offp + p];
-          }
-          pwo[k] = wk[off0 + p];
-          pxr[k] = a.xref[off0 + p];
-        }
-      }
-    }
-  }
-
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   const float2* other = cluster.map_shared_rank(mine, half ^ 1);
 #pragma unroll
@@ -714,39 +572,9 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(iter_cols_threads(H)
     wn[off0 + p] = wnv;
     xn[off0 + p] = make_float2(fmaf(omt, yk.x, tauk * zk.x), fmaf(omt, yk.y, tauk * zk.y));
   };
-  if constexpr (PRE) {
-    if (t < N3) {
-      float2 af[KM];  // the accumulators of this CTA's rows
-      if (half == 0) {
-#pragma unroll
-        for (int k = 0; k < KH; ++k) af[k] = acc[0][k];
-      } else {
-#pragma unroll
-        for (int k = 0; k < KM; ++k) af[k] = acc[0][KH + k];
-      }
-      const int w = t % kWB, k1p = t / kWB;
-      if constexpr (!PRE_T) {
-#pragma unroll
-        for (int k = 0; k < KM; ++k) {
-          if (kb + k < ke) {
-            const size_t p = size_t(k1p + B * (kb + k)) * W + w0 + w;
-            if constexpr (motion) {
-              pxm[k] = a.grad_ext[off0 + p];  // M^T (tTVadj u) of the motion-compensated form
-            } else {
-              pxm[k] = xk[offm + p];
-              pxp[k] = xk[offp + p];
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < KM; ++k)
-        if (kb + k < ke) update(size_t(k1p + B * (kb + k)) * W + w0 + w, pxa[k], pxm[k], pxp[k], pwo[k], pxr[k], af[k]);
-    }
-  }
   constexpr int BATCH = A <= 16 ? 8 : 4;  // one round of loads for a CTA's 8 rows at A = 16
 #pragma unroll
-  for (int ii = 0; ii < (PRE ? 0 : NI3); ++ii) {
+  for (int ii = 0; ii < NI3; ++ii) {
     const int i = t + ii * NT;
     if (i < N3) {
       const int w = i % kWB, k1p = i / kWB;
@@ -793,8 +621,8 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(iter_cols_threads(H)
     a.part_r[2 * blk + half] = pr;
   }
   if (rowlocal_last_cta(bm.ctl, inst, 2u * gridDim.x * unsigned(F)))
-    rowlocal_finish<NT>(a, st, bm.ctl, inst, it, apk, motion ? a.ntv : 2 * F * int(gridDim.x),
-                            2 * F * int(gridDim.x), sred, fm);
+    rowlocal_finish<NT>(a, st, bm.ctl, inst, it, apk, a.part_tv, motion ? a.ntv : 2 * F * int(gridDim.x), a.part_r,
+                        2 * F * int(gridDim.x), sred, fm);
 }
 
 }  // namespace gbn

@@ -55,6 +55,11 @@ int launch_setup(gbn_problem* P, cudaStream_t s);
 // start (w = 0, x_k = x_ref, mu/tolVar/Lmu) and end (x_ref = x_k) of outer loop nl
 int launch_outer_begin(gbn_ctx* ctx, gbn_problem* P, int nl, const float2* xref, cudaStream_t s);
 int launch_outer_end(gbn_ctx* ctx, gbn_problem* P, float2* xref, cudaStream_t s);
+// the same for the column-pair row-local iteration (rowpair.cuh): its tables
+// and tiles once per solve (T holds IDFT_W(y)), x_ref into tiles and back
+int launch_pair_setup(gbn_ctx* ctx, gbn_problem* P, const FusedArgs* tab, cudaStream_t s);
+int launch_outer_begin_pair(gbn_ctx* ctx, gbn_problem* P, int nl, const float2* xref, cudaStream_t s);
+int launch_outer_end_pair(gbn_ctx* ctx, gbn_problem* P, float2* xref, cudaStream_t s);
 // pinned host slot and event for the per-run row-structure read-back (created on first use)
 int partial_flag_ready(gbn_ctx* ctx);
 // 1-thread kernel storing a 48-bit generator state (outside captured graphs)

@@ -100,6 +100,14 @@ struct FusedArgs {
   CUtensorMap tm_s;
   CUtensorMap tm_se;
   CUtensorMap tm_y;
+  // column-pair row-local iteration (rowpair.cuh): operands in tiles of planar
+  // pairs, laid out per solve; nullptr for lengths without that iteration
+  const float4* St;       // S, [C][column group][row][pair]
+  const float4* Tt;       // kept rows' IDFT_W(y), per frame [column group][C][slot][pair]
+  float4* px[3];          // x_k and w_k in tiles, in turn: the iteration runs one ahead of the stopping test
+  float4* pw[3];          // (motion-compensated form: the first two, x_k in the natural order)
+  float4* xt;             // x_ref, [F][column group][row][pair]
+  const uint4* ptab;      // [F][PA] kept and sampled rows of each second-pass item, first staged slot
   int gmax_box;           // kept rows per box of tm_y (the most kept rows of a frame)
 };
 
