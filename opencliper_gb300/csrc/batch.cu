@@ -134,11 +134,10 @@ int batch_enqueue(gbn_batch* b, bool graph_mode) {
       n_launch += launch_constants(ctx, b->probs[i], b->out[i], rs, s);
     }
     const bool pair = g.row_local && kh->pair_cols;
-    for (size_t k = 0; pair && k < g.idx.size(); ++k)
-      n_launch += launch_pair_setup(ctx, b->probs[g.idx[k]], g.tab + k, s);
     for (unsigned nl = 1; nl <= g.maxIntIter; ++nl) {
-      for (int i : g.idx) {
-        n_launch += pair ? launch_outer_begin_pair(ctx, b->probs[i], int(nl), b->out[i], s)
+      for (size_t k = 0; k < g.idx.size(); ++k) {
+        const int i = g.idx[k];
+        n_launch += pair ? launch_outer_begin_pair(ctx, b->probs[i], int(nl), b->out[i], g.tab + k, s)
                          : launch_outer_begin(ctx, b->probs[i], int(nl), b->out[i], s);
         if (mixed) n_launch += launch_mixed_colmax(b->probs[i], s);
       }

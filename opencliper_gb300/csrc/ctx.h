@@ -83,7 +83,8 @@ struct gbn_problem {
   const float2* y = nullptr;          // caller's KData, not owned
   const float2* S = nullptr;          // caller's sensitivity maps, not owned
   const uint8_t* mask = nullptr;      // caller's pixel mask, not owned
-  // owned workspace
+  // owned workspace (everything up to the row buffers in one block)
+  void* block = nullptr;
   int* flags = nullptr;               // [F*H]
   int* full_fh = nullptr;             // [F*H]
   int* rowmap = nullptr;              // [F*H]

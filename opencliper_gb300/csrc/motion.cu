@@ -968,7 +968,7 @@ int nesta_run_mc(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, floa
   // pinned host memory while the setup is queued
   const bool check_rows = ctx->row_local && kh->iter_cols;
   if (check_rows && (rc = partial_flag_ready(ctx)) != GBN_OK) return rc;
-  ctx->launches += launch_pre(P, *prm, s);
+  ctx->launches += launch_pre(P, *prm, s, P->d_args, &a, P->ctl);
   cudaError_t ef = cudaSuccess;
   if (check_rows) {
     ef = cudaMemcpyAsync(ctx->host_partial, &P->st->partial_rows, sizeof(int), cudaMemcpyDeviceToHost, s);
@@ -976,8 +976,6 @@ int nesta_run_mc(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, floa
     if (ef != cudaSuccess) return cuda_status(ef, "row structure read-back");
   }
   if ((rc = tables_build(ctx, t, P->mc_xn, P->mc_xmesh, r, W, H, F, &P->st->status, s)) != GBN_OK) return rc;
-  ctx->launches += launch_store_args(P->d_args, a, s);
-  ctx->launches += launch_group_init(tab, 1, kw->rows_per_cta, P->ctl, s);
   if (check_rows) {  // T = IDFT_W(y) of the kept rows, the row-local iteration's data term
     kw->rows(tab, bm, 0, false, row_grid(ctx, kw, false, steps, k2), s);
     ctx->launches += 1;
@@ -1011,10 +1009,9 @@ int nesta_run_mc(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, floa
     // (the update gathering M^T g itself, without k_mc_adjoint, measured
     // slower: 20.7 against 16.7 ms per reconstruction at 256x256x20, 12 coils)
     const unsigned n_iter_launch = prm->maxIter + (prm->stoptest == 1 ? 1u : 0u);
-    if (kh->pair_cols) ctx->launches += launch_pair_setup(ctx, P, tab, s);
     for (unsigned nl = 1; nl <= prm->maxIntIter; ++nl) {
       if (kh->pair_cols) {  // the gathers read x_k in the natural order
-        ctx->launches += launch_outer_begin_pair(ctx, P, int(nl), x_out, s);
+        ctx->launches += launch_outer_begin_pair(ctx, P, int(nl), x_out, tab, s);
         cudaMemcpyAsync(P->xk0, x_out, size_t(W) * H * F * sizeof(float2), cudaMemcpyDeviceToDevice, s);
       } else {
         ctx->launches += launch_outer_begin(ctx, P, int(nl), x_out, s);

@@ -47,12 +47,18 @@ uint64_t lcg48_apply(const Lcg48& j, uint64_t x) { return (j.a * x + j.c) & kMas
 // flags: 0 not kept, 1 kept with sampled pixels, 2 kept for its data only;
 // full: every pixel of the mask row sampled.  grid = (H, F)
 // ---------------------------------------------------------------------------
-__global__ void k_rowflags(const float2* __restrict__ y, const uint8_t* __restrict__ mask, int W, int H, int F, int C,
-                           int* __restrict__ flags, int* __restrict__ full) {
-  const int h = blockIdx.x, f = blockIdx.y, t = threadIdx.x;
+// One CTA per row; the rows without samples are read whole (their data decide),
+// a coil per warp and step, so that a CTA keeps 8 x 4 loads of 512 bytes in
+// flight: bound by memory (256 x 256 x 20 x 12, R = 8, 110 MB: 32 -> 19 us
+// against a coil at a time with a CTA barrier after each).
+constexpr int kFlagNT = 256;
+__global__ void __launch_bounds__(kFlagNT) k_rowflags(const float2* __restrict__ y, const uint8_t* __restrict__ mask,
+                                                      int W, int H, int F, int C, int* __restrict__ flags,
+                                                      int* __restrict__ full) {
+  const int h = blockIdx.x, f = blockIdx.y, t = threadIdx.x, lane = t & 31;
   const uint8_t* m = mask + (size_t(f) * H + h) * W;
   int any = 0, all = 1;
-  for (int w = t; w < W; w += blockDim.x) {
+  for (int w = t; w < W; w += kFlagNT) {
     const int nz = m[w] != 0;
     any |= nz;
     all &= nz;
@@ -61,15 +67,21 @@ __global__ void k_rowflags(const float2* __restrict__ y, const uint8_t* __restri
   all = __syncthreads_and(all);
   const int sampled = any;
   if (!any) {
-    for (int c = 0; c < C && !any; ++c) {
-      const float4* yr = reinterpret_cast<const float4*>(y + ((size_t(f) * C + c) * H + h) * W);
-      int nz = 0;
-      for (int i = t; i < W / 2; i += blockDim.x) {
-        const float4 v = yr[i];
-        nz |= (v.x != 0.f) | (v.y != 0.f) | (v.z != 0.f) | (v.w != 0.f);
+    const int WQ = W / 2;
+    const size_t coil = size_t(H) * WQ;
+    const float4* row = reinterpret_cast<const float4*>(y) + (size_t(f) * C * H + h) * WQ;
+    int nz = 0;
+    for (int c = t >> 5; c < C; c += kFlagNT / 32) {
+      const float4* yr = row + c * coil;
+      for (int q = lane; q < WQ; q += 4 * 32) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = (q + 32 * u < WQ) ? yr[q + 32 * u] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) nz |= (v[u].x != 0.f) | (v[u].y != 0.f) | (v[u].z != 0.f) | (v[u].w != 0.f);
       }
-      any = __syncthreads_or(nz);
     }
+    any = __syncthreads_or(nz);
   }
   if (t == 0) {
     flags[f * H + h] = sampled ? 1 : (any ? 2 : 0);
@@ -79,52 +91,107 @@ __global__ void k_rowflags(const float2* __restrict__ y, const uint8_t* __restri
 
 constexpr int kStatusRowsOverflow = 6;  // NestaDevState::status: kept rows beyond the row buffer were dropped
 
-// one CTA of 512 threads (H <= 512): per-frame prefix numbering of kept rows;
-// rows beyond the row buffer's capacity `cap` are dropped (rowmap -1) and
-// reported in *status; *partial counts what keeps a problem off the
-// row-local iteration: kept rows whose mask row is sampled in part, and
-// frames with more kept rows than that iteration stages (iter_cols_rcap)
-__global__ void __launch_bounds__(512) k_rowscan(const int* __restrict__ flags, const int* __restrict__ full, int H,
-                                                 int F, int* __restrict__ rowmap, int* __restrict__ rowoff,
-                                                 int* __restrict__ rows_h, int* __restrict__ rows_f,
-                                                 int* __restrict__ row_full, int cap, int* __restrict__ status,
-                                                 int* __restrict__ partial) {
-  __shared__ int wsum[16];
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  int base = 0, npart = 0, nwide = 0;
-  bool dropped = false;
-  for (int f = 0; f < F; ++f) {
-    const int fl = (t < H) ? flags[f * H + t] : 0;
-    npart += __syncthreads_count(t < H && fl == 1 && !full[f * H + t]);
-    const unsigned bal = __ballot_sync(0xffffffffu, fl);
-    const int pre = __popc(bal & ((1u << lane) - 1u));
-    if (lane == 0) wsum[wid] = __popc(bal);
-    __syncthreads();
-    int woff = 0, tot = 0;
-    for (int i = 0; i < 16; ++i) {
-      if (i < wid) woff += wsum[i];
-      tot += wsum[i];
+// One CTA of 512 threads per frame (H <= 512): prefix numbering of the frame's
+// kept rows, after those of the frames before it (which every CTA counts for
+// itself: at most 64 x 512 flags); rows beyond the row buffer's capacity `cap`
+// are dropped (rowmap -1) and reported in *status; *partial counts what keeps a
+// problem off the row-local iteration: kept rows whose mask row is sampled in
+// part, and frames with more kept rows than that iteration stages
+// (iter_cols_rcap).  ptab (column pairs, rowpair.cuh; PA <= 32, PB <= 16): the
+// kept rows of every second-pass item k1 (rows k1 + PA*k2) and their staged
+// slots in (k1, k2) order.  ctl: the control block of a group of this one
+// instance.  (One CTA for all frames took 28 us at 20 frames, 41 at 30.)
+struct RowScan {
+  const int* flags;
+  const int* full;
+  int H, F, C, cap;
+  int *rowmap, *rowoff, *rows_h, *rows_f, *row_full, *status, *partial;
+  uint4* ptab;
+  int* rowslot;
+  int PA, PB;
+  ClassCtl* ctl;
+  int rpc;
+};
+__device__ void group_init_one(ClassCtl* ctl, int items, int rpc) {
+  ctl->step_base[0] = 0;
+  ctl->nitems[0] = items;
+  ctl->step_base[1] = (items + rpc - 1) / rpc;
+  ctl->row_next = 0;
+  ctl->ticket = 0;
+}
+__global__ void __launch_bounds__(512) k_rowscan(RowScan a) {
+  __shared__ int wsum[16], wbase[16], srow[512];
+  __shared__ unsigned char sfull[512];
+  const int f = blockIdx.x, t = threadIdx.x, lane = t & 31, wid = t >> 5, H = a.H;
+  int before = 0;
+  for (int i = t; i < f * H; i += 512) before += a.flags[i] != 0;
+  const int fl = (t < H) ? a.flags[f * H + t] : 0, fu = (t < H) ? a.full[f * H + t] : 0;
+  before = __reduce_add_sync(0xffffffffu, before);
+  const unsigned bal = __ballot_sync(0xffffffffu, fl);
+  const int pre = __popc(bal & ((1u << lane) - 1u));
+  if (lane == 0) {
+    wsum[wid] = __popc(bal);
+    wbase[wid] = before;
+  }
+  const int npart = __syncthreads_count(t < H && fl == 1 && !fu);
+  int woff = 0, tot = 0, base = 0;
+  for (int i = 0; i < 16; ++i) {
+    if (i < wid) woff += wsum[i];
+    tot += wsum[i];
+    base += wbase[i];
+  }
+  base = min(base, a.cap);
+  const int room = a.cap - base, j = (fl && woff + pre < room) ? woff + pre : -1;
+  if (t < H) {
+    a.rowmap[f * H + t] = j;
+    if (j >= 0) {
+      a.rows_h[base + j] = t;
+      a.rows_f[base + j] = f;
+      a.row_full[base + j] = fu;
     }
-    const int room = max(0, cap - base);
-    if (t < H) {
-      const int j = (fl && woff + pre < room) ? woff + pre : -1;
-      rowmap[f * H + t] = j;
-      if (j >= 0) {
-        rows_h[base + j] = t;
-        rows_f[base + j] = f;
-        row_full[base + j] = full[f * H + t];
+  }
+  srow[t] = j;
+  sfull[t] = fu != 0;
+  if (t == 0) {
+    a.rowoff[f] = base;
+    const int mine = npart + (tot > iter_cols_rcap(H));
+    if (mine) atomicAdd(a.partial, mine);
+    if (tot > room) atomicExch(a.status, kStatusRowsOverflow);
+    if (f == a.F - 1) {
+      const int g = base + min(tot, room);
+      a.rowoff[a.F] = g;
+      if (a.ctl) group_init_one(a.ctl, g * a.C, a.rpc);
+    }
+  }
+  if (a.ctl && f == a.F - 1 && t < kMaxBatch) a.ctl->done[t] = 0;
+  __syncthreads();
+  if (a.ptab && wid == 0) {
+    unsigned mk = 0, ms = 0;
+    int n = 0;
+    if (lane < a.PA) {
+      for (int k2 = 0; k2 < a.PB; ++k2) {
+        const int h = lane + a.PA * k2;
+        if (srow[h] >= 0) {
+          mk |= 1u << k2;
+          ms |= unsigned(sfull[h]) << k2;
+        }
+      }
+      n = __popc(mk);
+    }
+    int end = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += v;
+    }
+    if (lane < a.PA) {
+      int q = end - n;
+      a.ptab[f * a.PA + lane] = make_uint4(mk, ms, unsigned(q), 0u);
+      for (int k2 = 0; k2 < a.PB; ++k2) {
+        const int jj = srow[lane + a.PA * k2];
+        if (jj >= 0) a.rowslot[base + jj] = q++;
       }
     }
-    if (t == 0) rowoff[f] = base;
-    dropped |= tot > room;
-    nwide += tot > iter_cols_rcap(H);
-    base += min(tot, room);
-    __syncthreads();
-  }
-  if (t == 0) {
-    rowoff[F] = base;
-    *partial = npart + nwide;
-    if (dropped) atomicExch(status, kStatusRowsOverflow);
   }
 }
 
@@ -168,9 +235,10 @@ __global__ void k_group_init(const FusedArgs* __restrict__ tab, int n, int rpc, 
 }
 
 // ---------------------------------------------------------------------------
-// State initialisation from the launch parameters (one thread).
+// State initialisation from the launch parameters, and the instance's table
+// entry if given (one thread).
 // ---------------------------------------------------------------------------
-__global__ void k_state_init(NestaDevState* st, gbn_nesta_params p) {
+__global__ void k_state_init(NestaDevState* st, gbn_nesta_params p, FusedArgs* dst, FusedArgs args) {
   NestaDevState s;
   memset(&s, 0, sizeof(s));
   s.lambda_i = p.lambda_i;
@@ -183,6 +251,7 @@ __global__ void k_state_init(NestaDevState* st, gbn_nesta_params p) {
   s.miniter = int(p.miniter);
   s.last_iter = -1;
   *st = s;
+  if (dst) *dst = args;
 }
 
 // ---------------------------------------------------------------------------
@@ -194,13 +263,14 @@ __global__ void k_state_init(NestaDevState* st, gbn_nesta_params p) {
 __global__ void __launch_bounds__(256) k_maxima(const float2* __restrict__ x, const float2* __restrict__ xu, int N,
                                                 int F, NestaDevState* st) {
   __shared__ float s1[8], s2[8];
-  const size_t total = size_t(N) * F;
   float m1 = 0.f, m2 = 0.f;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
-    const int f = int(i / N);
-    const size_t p = i - size_t(f) * N;
-    const float2 a = x[i];
-    const float2 d = csub(xu[i], xu[size_t((f + F - 1) % F) * N + p]);
+  const int f = blockIdx.y;
+  const float2* xf = x + size_t(f) * N;
+  const float2* uf = xu + size_t(f) * N;
+  const float2* um = xu + size_t((f + F - 1) % F) * N;
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) {
+    const float2 a = xf[p];
+    const float2 d = csub(uf[p], um[p]);
     m1 = fmaxf(m1, sqrtf(a.x * a.x + a.y * a.y));
     m2 = fmaxf(m2, sqrtf(d.x * d.x + d.y * d.y));
   }
@@ -233,9 +303,10 @@ __global__ void __launch_bounds__(256) k_maxima(const float2* __restrict__ x, co
 // frame vector evolves independently: one thread per pixel advances it in
 // registers (scaled by 1/4 per step, exact in binary floating point, to stay
 // in range) and per-step sums of ||b_m||^2 and ||D b_m||^2 are reduced per
-// block.  Steps run in chunks; after each chunk k_normest_check replays the
-// reference's stopping rule on the sums available so far and, once it has
-// stopped, later chunks return immediately.
+// block.  Steps run in chunks; the last CTA of each chunk replays the
+// reference's stopping rule on the sums available so far (normest_check) and,
+// once it has stopped, later chunks return immediately; the last chunk ends
+// with the derived constants (derive_constants).
 // part layout: [block][step - m_begin (+1 for the first chunk)][2]; in the
 // first chunk slot 0 holds ||r||^2.
 // ---------------------------------------------------------------------------
@@ -243,13 +314,111 @@ constexpr int kNeChunks = 3;
 constexpr int kNeBounds[kNeChunks + 1] = {1, 17, 49, kNeIters};
 constexpr int kNeMaxSlots = 52;  // largest chunk (51 steps) + ||r||^2 slot
 
+// one CTA of kNeNT threads: reduce the chunk's per-block sums (two threads per
+// sum, blocks in order) and continue the reference's convergence loop
+// (NestaUp.cpp:325-431).  tot holds 2 * kNeSums doubles.
+constexpr int kNeSums = 128;
+static_assert(2 * kNeMaxSlots <= kNeSums && 2 * kNeSums == kNeNT, "two threads per sum");
+__device__ void normest_check(const double* __restrict__ part, int nblk, int m_begin, int m_end, int N, int F,
+                              NestaDevState* st, double* tot) {
+  const int slot0 = (m_begin == 1) ? 1 : 0;
+  const int nsum = (slot0 + m_end - m_begin) * 2;
+  const int i = threadIdx.x % kNeSums, half = threadIdx.x / kNeSums;
+  double s = 0.0;
+  if (i < nsum) {
+    constexpr int U = 8;
+    for (int b0 = half; b0 < nblk; b0 += 2 * U) {
+      double v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        v[u] = (b0 + 2 * u < nblk) ? __ldcg(part + size_t(b0 + 2 * u) * kNeMaxSlots * 2 + i) : 0.0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) s += v[u];
+    }
+  }
+  tot[threadIdx.x] = s;
+  __syncthreads();
+  if (half == 0) tot[i] += tot[i + kNeSums];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const float tol = 1e-3f;
+    float e, e0;
+    int cnt;
+    if (m_begin == 1) {
+      e = sqrtf(float(unsigned(N) * unsigned(F)));  // ||ones||
+      e0 = 0.f;
+      cnt = 0;
+    } else {
+      e = st->ne_e;
+      e0 = st->ne_e0;
+      cnt = st->ne_cnt;
+    }
+    bool stopped = false;
+    for (;;) {
+      if (!(fabsf(e - e0) > tol * e && cnt < kNeIters)) {
+        stopped = true;
+        break;
+      }
+      if (cnt > 0 && cnt >= m_end) break;  // needs steps of a later chunk
+      const float en = (cnt == 0) ? float(sqrt(tot[0]))
+                                  : float(sqrt(tot[2 * (slot0 + cnt - m_begin) + 1] / tot[2 * (slot0 + cnt - m_begin)]));
+      e0 = e;
+      e = en;
+      ++cnt;
+    }
+    st->ne_e = e;
+    st->ne_e0 = e0;
+    st->ne_cnt = cnt;
+    if (stopped) {
+      st->normU = e;
+      st->normest_iters = cnt;
+      st->ne_done = 1;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Derived constants (NestaUp.cpp:570-583), by the first warp of a CTA: gamma and
+// gammat, each a pow in double, on a lane of its own (and none with one outer
+// loop, where both are the bases themselves).
+// ---------------------------------------------------------------------------
+__device__ void derive_constants(NestaDevState* st) {
+  NestaDevState& s = *st;
+  const int lane = threadIdx.x;
+  const float maxX = __uint_as_float(s.maxX_bits), maxUX = __uint_as_float(s.maxUX_bits);
+  const float lambda = s.lambda_i * maxX, muf = s.mu_f * maxX;
+  float mu0 = float(0.9 * double(maxUX));
+  const float muL = lambda / s.La;
+  if (muL > mu0) mu0 = muL;
+  double g = (lane == 0) ? double(muf / mu0) : double(s.tolVar_in) / 0.1;
+  if (s.maxIntIter != 1 && lane < 2) g = pow(g, 1.0 / double(unsigned(s.maxIntIter)));
+  const float gamma = float(g), gammat = __shfl_sync(0xffffffffu, float(g), 1);
+  if (lane == 0) {
+    s.maxX = maxX;
+    s.maxUX = maxUX;
+    s.lambda = lambda;
+    s.muf = muf;
+    s.mu0 = mu0;
+    s.gamma = gamma;
+    s.mu = mu0;
+    s.gammat = gammat;
+    s.tolVar = 0.1f;
+  }
+}
+__global__ void k_setup(NestaDevState* st) { derive_constants(st); }
+
 template <int FMAX>
 __global__ void __launch_bounds__(kNeNT) k_normest_chunk(int N, int F, RandStart rs,
                                                          unsigned long long jumpN_a, unsigned long long jumpN_c,
                                                          int m_begin, int m_end, float* __restrict__ bstore,
-                                                         double* __restrict__ part, const NestaDevState* st) {
+                                                         double* __restrict__ part, NestaDevState* st) {
   __shared__ float sw[kNeNT / 32][kNeMaxSlots][2];
-  if (st->ne_done) return;
+  __shared__ double tot[2 * kNeSums];
+  __shared__ bool s_last;
+  if (st->ne_done) {
+    if (m_end == kNeIters && blockIdx.x == 0 && threadIdx.x < 32) derive_constants(st);
+    return;
+  }
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
   const int p = blockIdx.x * kNeNT + t;
   const bool act = p < N;
@@ -328,78 +497,21 @@ __global__ void __launch_bounds__(kNeNT) k_normest_chunk(int N, int F, RandStart
     for (int w = 0; w < kNeNT / 32; ++w) s += double(sw[w][i >> 1][i & 1]);
     part[size_t(blockIdx.x) * kNeMaxSlots * 2 + i] = s;
   }
-}
-
-// one CTA: reduce the chunk's per-block sums (one warp per sum) and continue
-// the reference's convergence loop (NestaUp.cpp:325-431)
-__global__ void __launch_bounds__(256) k_normest_check(const double* __restrict__ part, int nblk, int m_begin,
-                                                       int m_end, int N, int F, NestaDevState* st) {
-  __shared__ double tot[kNeMaxSlots * 2];
-  if (st->ne_done) return;
-  const int slot0 = (m_begin == 1) ? 1 : 0;
-  const int nsum = (slot0 + m_end - m_begin) * 2;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int i = wid; i < nsum; i += blockDim.x / 32) {
-    double s = 0.0;
-    for (int b = lane; b < nblk; b += 32) s += part[size_t(b) * kNeMaxSlots * 2 + i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) tot[i] = s;
+  // the chunk's last CTA replays the stopping rule
+  __threadfence();
+  __syncthreads();
+  if (t == 0) {
+    s_last = atomicAdd(&st->ne_arrived, 1u) == gridDim.x - 1;
+    if (s_last) st->ne_arrived = 0;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const float tol = 1e-3f;
-    float e, e0;
-    int cnt;
-    if (m_begin == 1) {
-      e = sqrtf(float(unsigned(N) * unsigned(F)));  // ||ones||
-      e0 = 0.f;
-      cnt = 0;
-    } else {
-      e = st->ne_e;
-      e0 = st->ne_e0;
-      cnt = st->ne_cnt;
-    }
-    bool stopped = false;
-    for (;;) {
-      if (!(fabsf(e - e0) > tol * e && cnt < kNeIters)) {
-        stopped = true;
-        break;
-      }
-      if (cnt > 0 && cnt >= m_end) break;  // needs steps of a later chunk
-      const float en = (cnt == 0) ? float(sqrt(tot[0]))
-                                  : float(sqrt(tot[2 * (slot0 + cnt - m_begin) + 1] / tot[2 * (slot0 + cnt - m_begin)]));
-      e0 = e;
-      e = en;
-      ++cnt;
-    }
-    st->ne_e = e;
-    st->ne_e0 = e0;
-    st->ne_cnt = cnt;
-    if (stopped) {
-      st->normU = e;
-      st->normest_iters = cnt;
-      st->ne_done = 1;
-    }
+  if (!s_last) return;
+  __threadfence();
+  normest_check(part, gridDim.x, m_begin, m_end, N, F, st, tot);
+  if (m_end == kNeIters) {
+    __syncthreads();
+    if (t < 32) derive_constants(st);
   }
-}
-
-// ---------------------------------------------------------------------------
-// Derived constants (NestaUp.cpp:570-583), one thread.
-// ---------------------------------------------------------------------------
-__global__ void k_setup(NestaDevState* st) {
-  NestaDevState& s = *st;
-  s.maxX = __uint_as_float(s.maxX_bits);
-  s.maxUX = __uint_as_float(s.maxUX_bits);
-  s.lambda = s.lambda_i * s.maxX;
-  s.muf = s.mu_f * s.maxX;
-  s.mu0 = float(0.9 * double(s.maxUX));
-  const float muL = s.lambda / s.La;
-  if (muL > s.mu0) s.mu0 = muL;
-  s.gamma = float(pow(double(s.muf / s.mu0), 1.0 / double(unsigned(s.maxIntIter))));
-  s.mu = s.mu0;
-  s.gammat = float(pow(double(s.tolVar_in) / 0.1, 1.0 / double(unsigned(s.maxIntIter))));
-  s.tolVar = 0.1f;
 }
 
 __device__ void outer_begin_state(NestaDevState* st, int nl, float* fmean) {
@@ -448,68 +560,17 @@ __device__ __forceinline__ float4 planar_pair(const float2* src) {
   return make_float4(u.x, v.x, u.y, v.y);
 }
 
-// One warp per frame: the kept rows of every second-pass item k1 (rows k1 +
-// PA*k2; PA <= 32, PB <= 16) and their staged slots in (k1, k2) order.
-__global__ void __launch_bounds__(32) k_pair_tables(const int* __restrict__ rowmap, const int* __restrict__ rowoff,
-                                                    const int* __restrict__ row_full, int H, int PA, int PB,
-                                                    uint4* __restrict__ ptab, int* __restrict__ rowslot) {
-  const int f = blockIdx.x, t = threadIdx.x, rowbase = rowoff[f];
-  unsigned mk = 0, ms = 0;
-  int n = 0;
-  if (t < PA) {
-    for (int k2 = 0; k2 < PB; ++k2) {
-      const int j = rowmap[f * H + t + PA * k2];
-      if (j >= 0) {
-        mk |= 1u << k2;
-        ms |= (row_full[rowbase + j] ? 1u : 0u) << k2;
-      }
-    }
-    n = __popc(mk);
-  }
-  int end = n;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, end, o);
-    if (t >= o) end += v;
-  }
-  if (t < PA) {
-    int q = end - n;
-    ptab[f * PA + t] = make_uint4(mk, ms, unsigned(q), 0u);
-    for (int k2 = 0; k2 < PB; ++k2) {
-      const int j = rowmap[f * H + t + PA * k2];
-      if (j >= 0) rowslot[rowbase + j] = q++;
-    }
-  }
-}
-
-// S and the kept rows' IDFT_W(y) into tiles (two adjacent columns per thread
-// and step).  Skipped when the rows do not suit the row-local iteration: they
+// Start of an outer loop: x_ref into tiles and the scalar state as k_outer_begin
+// leaves it; before the first loop (St given) also S and the kept rows'
+// IDFT_W(y), which T holds since x0 = E^H y.  A warp per row of W/2 pairs.  The
+// data tiles are skipped when the rows do not suit the row-local iteration: they
 // may then exceed Tt (the run or replay reports it).
-__global__ void __launch_bounds__(256) k_pair_pack(const FusedArgs* __restrict__ tab, float4* __restrict__ St,
-                                                   float4* __restrict__ Tt, const int* __restrict__ rowslot, int NP) {
-  const FusedArgs& a = *tab;
-  if (a.st->partial_rows) return;
-  const int W = a.W, H = a.H, C = a.C, WQ = W / 2;
-  const size_t nS = size_t(C) * H * WQ, nT = size_t(a.rowoff[a.F]) * C * WQ;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < nS + nT; i += size_t(gridDim.x) * blockDim.x) {
-    if (i < nS) {
-      const int q = int(i % WQ);
-      const size_t cr = i / WQ, c = cr / H, row = cr % H;
-      St[((c * (WQ / NP) + q / NP) * H + row) * NP + q % NP] = planar_pair(a.S + 2 * i);
-    } else {
-      const size_t k = i - nS, gc = k / WQ;
-      const int q = int(k % WQ), c = int(gc % C), g = int(gc / C), f = a.rows_f[g];
-      const size_t base = size_t(a.rowoff[f]) * C * WQ, nr = a.rowoff[f + 1] - a.rowoff[f];
-      Tt[base + ((size_t(q / NP) * C + c) * nr + rowslot[g]) * NP + q % NP] = planar_pair(a.T + 2 * k);
-    }
-  }
-}
-
-// x_ref into tiles at the start of an outer loop, and the scalar state as
-// k_outer_begin leaves it
-__global__ void __launch_bounds__(256) k_outer_begin_pair(NestaDevState* st, int nl, float* fmean,
+__global__ void __launch_bounds__(256) k_outer_begin_pair(const FusedArgs* __restrict__ tab, int nl,
                                                           const float2* __restrict__ xref, float4* __restrict__ xt,
-                                                          int W, int H, size_t n2, int NP) {
+                                                          float4* __restrict__ St, float4* __restrict__ Tt,
+                                                          const int* __restrict__ rowslot, int NP) {
+  const FusedArgs& a = *tab;
+  NestaDevState* st = a.st;
   if (nl > st->maxIntIter) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       st->outer_active = 0;
@@ -517,29 +578,47 @@ __global__ void __launch_bounds__(256) k_outer_begin_pair(NestaDevState* st, int
     }
     return;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) outer_begin_state(st, nl, fmean);
-  const int WQ = W / 2;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n2; i += size_t(gridDim.x) * blockDim.x) {
-    const int q = int(i % WQ);
-    const size_t fr = i / WQ, f = fr / H, row = fr % H;
-    xt[((f * (WQ / NP) + q / NP) * H + row) * NP + q % NP] = planar_pair(xref + 2 * i);
+  if (blockIdx.x == 0 && threadIdx.x == 0) outer_begin_state(st, nl, a.fmean);
+  const int W = a.W, H = a.H, F = a.F, C = a.C, WQ = W / 2, NCG = WQ / NP, lane = threadIdx.x & 31;
+  const int nX = F * H, nS = St && !st->partial_rows ? C * H : 0;
+  const long long rows = nX + nS + (nS ? (long long)a.rowoff[F] * C : 0);
+  for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * 8) {
+    const float2* src;
+    float4* dst;
+    size_t step;  // from one column group to the next
+    if (r < nX + nS) {
+      const int k = int(r < nX ? r : r - nX), img = k / H, row = k % H;  // img: frame, or coil
+      src = (r < nX ? xref : a.S) + size_t(k) * W;
+      step = size_t(H) * NP;
+      dst = (r < nX ? xt : St) + size_t(img) * NCG * step + row * NP;
+    } else {
+      const long long k = r - nX - nS;
+      const int g = int(k / C), c = int(k % C), f = a.rows_f[g];
+      const size_t nr = a.rowoff[f + 1] - a.rowoff[f];
+      src = a.T + size_t(k) * W;
+      step = size_t(C) * nr * NP;
+      dst = Tt + size_t(a.rowoff[f]) * C * WQ + (size_t(c) * nr + rowslot[g]) * NP;
+    }
+    for (int q = lane; q < WQ; q += 32) dst[(q / NP) * step + q % NP] = planar_pair(src + 2 * q);
   }
 }
 
 // End of an outer loop from tiles: x_ref = x_k (nothing ran: x_ref stays)
 __global__ void __launch_bounds__(256) k_outer_end_pair(const NestaDevState* st, const float4* __restrict__ xk0,
                                                         const float4* __restrict__ xk1, const float4* __restrict__ xk2,
-                                                        float2* __restrict__ xref, int W, int H, size_t n2, int NP) {
+                                                        float2* __restrict__ xref, int W, int H, int rows, int NP) {
   if (!st->outer_active || st->last_iter < 0) return;
   const int k3 = (st->last_iter + 1) % 3;
   const float4* src = k3 == 0 ? xk0 : k3 == 1 ? xk1 : xk2;
-  const int WQ = W / 2;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n2; i += size_t(gridDim.x) * blockDim.x) {
-    const int q = int(i % WQ);
-    const size_t fr = i / WQ, f = fr / H, row = fr % H;
-    const float4 v = src[((f * (WQ / NP) + q / NP) * H + row) * NP + q % NP];
-    xref[2 * i] = make_float2(v.x, v.z);
-    xref[2 * i + 1] = make_float2(v.y, v.w);
+  const int WQ = W / 2, lane = threadIdx.x & 31, step = H * NP;
+  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8) {  // a warp per row
+    const float4* from = src + size_t(r / H) * (WQ / NP) * step + (r % H) * NP;
+    float2* to = xref + size_t(r) * W;
+    for (int q = lane; q < WQ; q += 32) {
+      const float4 v = from[size_t(q / NP) * step + q % NP];
+      to[2 * q] = make_float2(v.x, v.z);
+      to[2 * q + 1] = make_float2(v.y, v.w);
+    }
   }
 }
 
@@ -578,7 +657,7 @@ int normest_fmax(int F) {
 }
 
 void launch_normest_chunk(int fmax, int nblk, cudaStream_t s, int N, int F, const RandStart& x0, const Lcg48& jN, int mb,
-                          int me, float* bstore, double* part, const NestaDevState* st) {
+                          int me, float* bstore, double* part, NestaDevState* st) {
 #define GBN_NE_CASE(M)                                                                                  \
   case M:                                                                                               \
     k_normest_chunk<M><<<nblk, kNeNT, 0, s>>>(N, F, x0, jN.a, jN.c, mb, me, bstore, part, st); \
@@ -602,37 +681,49 @@ int problem_alloc(gbn_problem* P) {
   const size_t FH = size_t(P->F) * P->H;
   const size_t X = size_t(P->F) * P->H * P->W;
   const size_t K = X * P->C;
-  cudaError_t e = cudaSuccess;
-  auto A = [&](void** p, size_t bytes) {
-    if (e == cudaSuccess) e = cudaMalloc(p, bytes);
-  };
-  A((void**)&P->flags, FH * sizeof(int));
-  A((void**)&P->full_fh, FH * sizeof(int));
-  A((void**)&P->rowmap, FH * sizeof(int));
-  A((void**)&P->rowoff, (P->F + 1) * sizeof(int));
-  A((void**)&P->rows_h, FH * sizeof(int));
-  A((void**)&P->rows_f, FH * sizeof(int));
-  A((void**)&P->row_full, FH * sizeof(int));
-  A((void**)&P->T, K * sizeof(float2));
-  P->T_rows = FH;
-  A((void**)&P->xk0, X * sizeof(float2));
-  A((void**)&P->xk1, X * sizeof(float2));
-  A((void**)&P->wacc, X * sizeof(float2));
-  A((void**)&P->wacc1, X * sizeof(float2));
-  A((void**)&P->st, sizeof(NestaDevState));
   const SizeKernels* kh = find_size(P->H);
-  if (kh && kh->pair_cols) {
-    P->Tt_rows = size_t(P->F) * std::min(P->H, iter_cols_rcap(P->H));
-    A((void**)&P->St, size_t(P->C) * P->H * P->W * sizeof(float2));
-    A((void**)&P->Tt, P->Tt_rows * P->C * P->W * sizeof(float2));
-    A((void**)&P->xt, X * sizeof(float2));
-    A((void**)&P->xk2, X * sizeof(float2));
-    A((void**)&P->wacc2, X * sizeof(float2));
-    A((void**)&P->ptab, size_t(P->F) * pair_a(P->H) * sizeof(uint4));
-    A((void**)&P->rowslot, FH * sizeof(int));
+  const bool pair = kh && kh->pair_cols;
+  // one allocation for everything but the row buffers, which fit_rows resizes
+  struct Part {
+    void** p;
+    size_t bytes;
+  };
+  const Part parts[] = {{(void**)&P->flags, FH * sizeof(int)},
+                        {(void**)&P->full_fh, FH * sizeof(int)},
+                        {(void**)&P->rowmap, FH * sizeof(int)},
+                        {(void**)&P->rowoff, (P->F + 1) * sizeof(int)},
+                        {(void**)&P->rows_h, FH * sizeof(int)},
+                        {(void**)&P->rows_f, FH * sizeof(int)},
+                        {(void**)&P->row_full, FH * sizeof(int)},
+                        {(void**)&P->xk0, X * sizeof(float2)},
+                        {(void**)&P->xk1, X * sizeof(float2)},
+                        {(void**)&P->wacc, X * sizeof(float2)},
+                        {(void**)&P->wacc1, X * sizeof(float2)},
+                        {(void**)&P->st, sizeof(NestaDevState)},
+                        {(void**)&P->d_args, sizeof(FusedArgs)},
+                        {(void**)&P->ctl, sizeof(ClassCtl)},
+                        // column pairs only
+                        {(void**)&P->St, size_t(P->C) * P->H * P->W * sizeof(float2)},
+                        {(void**)&P->xt, X * sizeof(float2)},
+                        {(void**)&P->xk2, X * sizeof(float2)},
+                        {(void**)&P->wacc2, X * sizeof(float2)},
+                        {(void**)&P->ptab, size_t(P->F) * pair_a(P->H) * sizeof(uint4)},
+                        {(void**)&P->rowslot, FH * sizeof(int)}};
+  const size_t nparts = sizeof(parts) / sizeof(parts[0]) - (pair ? 0 : 6);
+  auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+  size_t total = 0;
+  for (size_t k = 0; k < nparts; ++k) total += up(parts[k].bytes);
+  cudaError_t e = cudaMalloc(&P->block, total);
+  if (e == cudaSuccess) {
+    unsigned char* b = static_cast<unsigned char*>(P->block);
+    for (size_t k = 0; k < nparts; b += up(parts[k].bytes), ++k) *parts[k].p = b;
+    e = cudaMalloc(&P->T, K * sizeof(float2));
+    P->T_rows = FH;
   }
-  A((void**)&P->d_args, sizeof(FusedArgs));
-  A((void**)&P->ctl, sizeof(ClassCtl));
+  if (e == cudaSuccess && pair) {
+    P->Tt_rows = size_t(P->F) * std::min(P->H, iter_cols_rcap(P->H));
+    e = cudaMalloc(&P->Tt, P->Tt_rows * P->C * P->W * sizeof(float2));
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return set_error(GBN_ERR_NOMEM, std::string("problem workspace allocation failed: ") + cudaGetErrorString(e));
@@ -640,7 +731,7 @@ int problem_alloc(gbn_problem* P) {
   return GBN_OK;
 }
 
-void launch_row_analysis(gbn_problem* P, cudaStream_t s);
+void launch_row_analysis(gbn_problem* P, ClassCtl* ctl, cudaStream_t s);
 
 // Shrinks (or grows) the row buffer T to the rows the current y and mask keep
 // plus `headroom` (at most every row); returns the kept rows in *kept.
@@ -650,10 +741,11 @@ int problem_fit_rows(gbn_problem* P, int headroom, int* kept) {
     return set_error(GBN_ERR_INVALID, "fit rows: the problem belongs to a live batch (destroy it first)");
   cudaStream_t s = P->ctx->stream;
   cudaError_t e = cudaMemsetAsync(&P->st->status, 0, sizeof(int), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(&P->st->partial_rows, 0, sizeof(int), s);
   const size_t saved = P->T_rows;
   P->T_rows = size_t(P->F) * P->H;  // count every kept row
   if (e == cudaSuccess) {
-    launch_row_analysis(P, s);
+    launch_row_analysis(P, nullptr, s);
     int g = 0;
     if ((e = cudaMemcpyAsync(&g, P->rowoff + P->F, sizeof(int), cudaMemcpyDeviceToHost, s)) == cudaSuccess &&
         (e = cudaStreamSynchronize(s)) == cudaSuccess) {
@@ -695,21 +787,39 @@ int problem_fit_rows(gbn_problem* P, int headroom, int* kept) {
 void motion_free(gbn_problem* P);
 
 void problem_free(gbn_problem* P) {
-  void* ptrs[] = {P->flags, P->full_fh, P->rowmap, P->rowoff,  P->rows_h, P->rows_f,  P->row_full, P->T,
-                  P->xk0,   P->xk1,     P->wacc,   P->wacc1,  P->st,      P->fmean,  P->part_tv, P->part_r,   P->part_ne,
-                  P->ne_b,  P->d_args,  P->ctl,      P->fk,     P->colmax, P->smax,   P->fa,
-                  P->St,    P->Tt,      P->xt,     P->ptab,   P->rowslot,
-                  P->xk2,   P->wacc2};
+  void* ptrs[] = {P->block,   P->T,    P->Tt, P->fmean,  P->part_tv, P->part_r,
+                  P->part_ne, P->ne_b, P->fk, P->colmax, P->smax,    P->fa};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   motion_free(P);
 }
 
 // Kept-row analysis for the current contents of y and mask (device only).
-void launch_row_analysis(gbn_problem* P, cudaStream_t s) {
-  k_rowflags<<<dim3(P->H, P->F), 128, 0, s>>>(P->y, P->mask, P->W, P->H, P->F, P->C, P->flags, P->full_fh);
-  k_rowscan<<<1, 512, 0, s>>>(P->flags, P->full_fh, P->H, P->F, P->rowmap, P->rowoff, P->rows_h, P->rows_f,
-                              P->row_full, int(P->T_rows), &P->st->status, &P->st->partial_rows);
+void launch_row_analysis(gbn_problem* P, ClassCtl* ctl, cudaStream_t s) {
+  k_rowflags<<<dim3(P->H, P->F), kFlagNT, 0, s>>>(P->y, P->mask, P->W, P->H, P->F, P->C, P->flags, P->full_fh);
+  RowScan r{};
+  r.flags = P->flags;
+  r.full = P->full_fh;
+  r.H = P->H;
+  r.F = P->F;
+  r.C = P->C;
+  r.cap = int(P->T_rows);
+  r.rowmap = P->rowmap;
+  r.rowoff = P->rowoff;
+  r.rows_h = P->rows_h;
+  r.rows_f = P->rows_f;
+  r.row_full = P->row_full;
+  r.status = &P->st->status;
+  r.partial = &P->st->partial_rows;
+  if (P->ptab) {
+    r.ptab = P->ptab;
+    r.rowslot = P->rowslot;
+    r.PA = pair_a(P->H);
+    r.PB = pair_b(P->H);
+  }
+  r.ctl = ctl;
+  r.rpc = find_size(P->W)->rows_per_cta;
+  k_rowscan<<<P->F, 512, 0, s>>>(r);
 }
 
 FusedArgs make_args(gbn_problem* P, float2* xref) {
@@ -822,9 +932,10 @@ int launch_set_rand(unsigned long long* dst, unsigned long long v, cudaStream_t 
   return 1;
 }
 
-int launch_pre(gbn_problem* P, const gbn_nesta_params& prm, cudaStream_t s) {
-  k_state_init<<<1, 1, 0, s>>>(P->st, prm);
-  launch_row_analysis(P, s);
+int launch_pre(gbn_problem* P, const gbn_nesta_params& prm, cudaStream_t s, FusedArgs* tab, const FusedArgs* args,
+               ClassCtl* ctl) {
+  k_state_init<<<1, 1, 0, s>>>(P->st, prm, tab, args ? *args : FusedArgs{});
+  launch_row_analysis(P, ctl, s);
   return 3;
 }
 
@@ -836,49 +947,41 @@ int launch_constants(gbn_ctx* ctx, gbn_problem* P, const float2* xref, const Ran
   const int N = P->W * P->H, F = P->F;
   const int nblk_ne = (N + kNeNT - 1) / kNeNT;
   // maxima, norm estimate, constants (NestaUp.cpp:521-583)
-  k_maxima<<<elementwise_grid(ctx, size_t(N) * F), 256, 0, s>>>(xref, xref, N, F, P->st);
+  launch_maxima(ctx, P, xref, xref, s);
   const Lcg48 jN = lcg_jump_k(uint64_t(N));
-  for (int ch = 0; ch < kNeChunks; ++ch) {
+  for (int ch = 0; ch < kNeChunks; ++ch)
     launch_normest_chunk(normest_fmax(F), nblk_ne, s, N, F, rs, jN, kNeBounds[ch], kNeBounds[ch + 1], P->ne_b,
                          P->part_ne, P->st);
-    k_normest_check<<<1, 256, 0, s>>>(P->part_ne, nblk_ne, kNeBounds[ch], kNeBounds[ch + 1], N, F, P->st);
-  }
-  k_setup<<<1, 1, 0, s>>>(P->st);
-  return 2 + 2 * kNeChunks;
+  return 1 + kNeChunks;
 }
 
 int launch_maxima(gbn_ctx* ctx, gbn_problem* P, const float2* x0, const float2* xu, cudaStream_t s) {
-  const size_t X = size_t(P->W) * P->H * P->F;
-  k_maxima<<<elementwise_grid(ctx, X), 256, 0, s>>>(x0, xu, P->W * P->H, P->F, P->st);
+  const int N = P->W * P->H;
+  const dim3 g(std::min((N + 511) / 512, std::max(1, ctx->nsm * 8 / P->F)), P->F);
+  k_maxima<<<g, 256, 0, s>>>(x0, xu, N, P->F, P->st);
   return 1;
 }
 
 int launch_setup(gbn_problem* P, cudaStream_t s) {
-  k_setup<<<1, 1, 0, s>>>(P->st);
+  k_setup<<<1, 32, 0, s>>>(P->st);
   return 1;
 }
 
-int launch_pair_setup(gbn_ctx* ctx, gbn_problem* P, const FusedArgs* tab, cudaStream_t s) {
-  const int H = P->H;
-  k_pair_tables<<<P->F, 32, 0, s>>>(P->rowmap, P->rowoff, P->row_full, H, pair_a(H), pair_b(H), P->ptab, P->rowslot);
-  const size_t n = (size_t(P->C) * H + P->Tt_rows * P->C) * (P->W / 2);
-  k_pair_pack<<<elementwise_grid(ctx, n), 256, 0, s>>>(tab, P->St, P->Tt, P->rowslot, pair_np(H));
-  return 2;
-}
-
-int launch_outer_begin_pair(gbn_ctx* ctx, gbn_problem* P, int nl, const float2* xref, cudaStream_t s) {
-  const size_t n2 = size_t(P->W) * P->H * P->F / 2;
-  k_outer_begin_pair<<<elementwise_grid(ctx, n2), 256, 0, s>>>(P->st, nl, P->fmean, xref, P->xt, P->W, P->H, n2,
-                                                                pair_np(P->H));
+int launch_outer_begin_pair(gbn_ctx* ctx, gbn_problem* P, int nl, const float2* xref, const FusedArgs* tab,
+                            cudaStream_t s) {
+  const bool first = nl == 1;
+  const long long rows = (long long)P->F * P->H + (first ? (long long)P->C * P->H + (long long)P->Tt_rows * P->C : 0);
+  const int grid = int(std::min<long long>((rows + 7) / 8, (long long)ctx->nsm * 8));
+  k_outer_begin_pair<<<grid, 256, 0, s>>>(tab, nl, xref, P->xt, first ? P->St : nullptr, P->Tt, P->rowslot,
+                                          pair_np(P->H));
   return 1;
 }
 
 int launch_outer_end_pair(gbn_ctx* ctx, gbn_problem* P, float2* xref, cudaStream_t s) {
-  const size_t n2 = size_t(P->W) * P->H * P->F / 2;
-  k_outer_end_pair<<<elementwise_grid(ctx, n2), 256, 0, s>>>(P->st, reinterpret_cast<const float4*>(P->xk0),
-                                                              reinterpret_cast<const float4*>(P->xk1),
-                                                              reinterpret_cast<const float4*>(P->xk2), xref, P->W,
-                                                              P->H, n2, pair_np(P->H));
+  const int rows = P->F * P->H;
+  k_outer_end_pair<<<std::min((rows + 7) / 8, ctx->nsm * 8), 256, 0, s>>>(
+      P->st, reinterpret_cast<const float4*>(P->xk0), reinterpret_cast<const float4*>(P->xk1),
+      reinterpret_cast<const float4*>(P->xk2), xref, P->W, P->H, rows, pair_np(P->H));
   return 1;
 }
 
@@ -963,13 +1066,11 @@ int nesta_run(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, float2*
   cudaError_t ef = cudaSuccess;
   int n_setup = 0;
   GBN_LAUNCH(ctx, GBN_PROF_SETUP, n_setup, {
-    n_setup += launch_pre(P, *prm, s);
+    n_setup += launch_pre(P, *prm, s, P->d_args, &a, P->ctl);
     if (check_rows) {
       ef = cudaMemcpyAsync(ctx->host_partial, &P->st->partial_rows, sizeof(int), cudaMemcpyDeviceToHost, s);
       if (ef == cudaSuccess) ef = cudaEventRecord(ctx->ev_partial, s);
     }
-    n_setup += launch_store_args(P->d_args, a, s);
-    n_setup += launch_group_init(tab, 1, kw->rows_per_cta, P->ctl, s);
     // x0 = E^H y (NestaUp.cpp:465-486); T keeps IDFT_W(y) of the kept rows
     kw->rows(tab, bm, 0, false, g2a, s);
     kh->inv_cols(tab, bm, 0, false, g3, s);
@@ -989,10 +1090,10 @@ int nesta_run(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, float2*
   const bool pair = row_local && kh->pair_cols;
   const unsigned n_iter_launch = prm->maxIter + ((row_local && prm->stoptest == 1) ? (pair ? 2u : 1u) : 0u);
 
-  if (pair) GBN_LAUNCH(ctx, GBN_PROF_SETUP, 2, launch_pair_setup(ctx, P, tab, s));
   for (unsigned nl = 1; nl <= prm->maxIntIter; ++nl) {
     GBN_LAUNCH(ctx, GBN_PROF_OUTER, 1,
-               pair ? launch_outer_begin_pair(ctx, P, int(nl), x_out, s) : launch_outer_begin(ctx, P, int(nl), x_out, s));
+               pair ? launch_outer_begin_pair(ctx, P, int(nl), x_out, tab, s)
+                    : launch_outer_begin(ctx, P, int(nl), x_out, s));
     if (row_local) {
       for (unsigned it = 0; it < n_iter_launch; ++it)
         GBN_LAUNCH(ctx, GBN_PROF_ITER, 1, kh->iter_cols(tab, bm, int(it), false, g3, s));

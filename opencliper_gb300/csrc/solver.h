@@ -44,8 +44,10 @@ void tuning_for(gbn_ctx* ctx, int W, int H, int F, int C, int* k1_coils_per_bloc
 
 int launch_store_args(FusedArgs* dst, const FusedArgs& a, cudaStream_t s);
 int launch_group_init(const FusedArgs* tab, int n, int rows_per_cta, ClassCtl* ctl, cudaStream_t s);
-// parameters into the state block, then the kept-row analysis of y and mask
-int launch_pre(gbn_problem* P, const gbn_nesta_params& prm, cudaStream_t s);
+// parameters into the state block (and *args into the table entry tab), then the
+// kept-row analysis of y and mask (and the control block of a group of P alone)
+int launch_pre(gbn_problem* P, const gbn_nesta_params& prm, cudaStream_t s, FusedArgs* tab = nullptr,
+               const FusedArgs* args = nullptr, ClassCtl* ctl = nullptr);
 // after x0 = E^H y is in xref: maxima, norm estimate and derived constants
 int launch_constants(gbn_ctx* ctx, gbn_problem* P, const float2* xref, const RandStart& rs, cudaStream_t s);
 // max|x0| and max|D xu| into the state block (xu = x0, or M x0 with motion compensation)
@@ -55,10 +57,10 @@ int launch_setup(gbn_problem* P, cudaStream_t s);
 // start (w = 0, x_k = x_ref, mu/tolVar/Lmu) and end (x_ref = x_k) of outer loop nl
 int launch_outer_begin(gbn_ctx* ctx, gbn_problem* P, int nl, const float2* xref, cudaStream_t s);
 int launch_outer_end(gbn_ctx* ctx, gbn_problem* P, float2* xref, cudaStream_t s);
-// the same for the column-pair row-local iteration (rowpair.cuh): its tables
-// and tiles once per solve (T holds IDFT_W(y)), x_ref into tiles and back
-int launch_pair_setup(gbn_ctx* ctx, gbn_problem* P, const FusedArgs* tab, cudaStream_t s);
-int launch_outer_begin_pair(gbn_ctx* ctx, gbn_problem* P, int nl, const float2* xref, cudaStream_t s);
+// the same for the column-pair row-local iteration (rowpair.cuh): x_ref into tiles
+// and back, and before the first loop the tiles of S and of IDFT_W(y) (in T)
+int launch_outer_begin_pair(gbn_ctx* ctx, gbn_problem* P, int nl, const float2* xref, const FusedArgs* tab,
+                            cudaStream_t s);
 int launch_outer_end_pair(gbn_ctx* ctx, gbn_problem* P, float2* xref, cudaStream_t s);
 // pinned host slot and event for the per-run row-structure read-back (created on first use)
 int partial_flag_ready(gbn_ctx* ctx);

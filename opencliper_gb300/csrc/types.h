@@ -36,6 +36,7 @@ struct NestaDevState {
   // power-method progress across chunks
   int ne_done, ne_cnt;
   float ne_e, ne_e0;
+  unsigned ne_arrived;    // CTAs of the running chunk that have stored their sums
 
   // row-local iteration (rowlocal.cuh): the update of iteration last_iter
   // must be recomputed with the stopping rule's weights; kept rows that are
