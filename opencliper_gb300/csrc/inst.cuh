@@ -23,7 +23,7 @@ struct Launchers {
   static void fwd_cols(const FusedArgs* tab, const BatchMap& bm, int it, int cpb, dim3 grid, cudaStream_t s) {
     static bool ok = false;
     allow_smem(k_fwd_cols<L>, FwdColsSmem<L>::BYTES, ok);
-    launch_pdl(k_fwd_cols<L>, grid, kColNT, FwdColsSmem<L>::BYTES, s, tab, bm, it, cpb);
+    launch_chain(it == 0, k_fwd_cols<L>, grid, kColNT, FwdColsSmem<L>::BYTES, s, tab, bm, it, cpb);
   }
   // resident CTAs per SM of the row kernel (queried once)
   static int rows_occupancy(bool resid) {
@@ -50,7 +50,7 @@ struct Launchers {
       launch_pdl(k_rows<L, true>, dim3(grid), kRowNT, RowsSmem<L, true>::BYTES, s, tab, bm, it);
     } else {
       allow_smem(k_rows<L, false>, RowsSmem<L, false>::BYTES, ok0);
-      launch_pdl(k_rows<L, false>, dim3(grid), kRowNT, RowsSmem<L, false>::BYTES, s, tab, bm, it);
+      launch_chain(true, k_rows<L, false>, dim3(grid), kRowNT, RowsSmem<L, false>::BYTES, s, tab, bm, it);
     }
   }
   static void inv_cols(const FusedArgs* tab, const BatchMap& bm, int it, bool update, dim3 grid, cudaStream_t s) {
@@ -73,7 +73,8 @@ struct Launchers {
         launch_pdl(k_iter_pair<L, true>, dim3(ncg, frames), kPairNT, P::BYTES, s, tab, bm, it, 0);
       } else {
         allow_smem(k_iter_pair<L, false>, P::BYTES, ok0);
-        launch_pdl(k_iter_pair<L, false>, dim3(ncg, frames + cdiv(bm.n, ncg)), kPairNT, P::BYTES, s, tab, bm, it, 0);
+        launch_chain(it == 0, k_iter_pair<L, false>, dim3(ncg, frames + cdiv(bm.n, ncg)), kPairNT, P::BYTES, s, tab, bm,
+                     it, 0);
       }
     } else if constexpr (iter_cols_ok(L)) {
       static bool ok0 = false, ok1 = false;
@@ -82,7 +83,7 @@ struct Launchers {
         launch_pdl(k_iter_cols<L, true>, grid, IterColsSmem<L>::NT, IterColsSmem<L>::BYTES, s, tab, bm, it);
       } else {
         allow_smem(k_iter_cols<L, false>, IterColsSmem<L>::BYTES, ok0);
-        launch_pdl(k_iter_cols<L, false>, grid, IterColsSmem<L>::NT, IterColsSmem<L>::BYTES, s, tab, bm, it);
+        launch_chain(it == 0, k_iter_cols<L, false>, grid, IterColsSmem<L>::NT, IterColsSmem<L>::BYTES, s, tab, bm, it);
       }
     }
   }

@@ -697,7 +697,7 @@ void launch_inv_cols_tc(const FusedArgs* tab, const BatchMap& bm, int it, int nm
 void launch_fwd_cols_tc(const FusedArgs* tab, const BatchMap& bm, int it, int npad_max, dim3 grid, cudaStream_t s) {
   static bool ok = false;
   allow_smem(k_fwd_cols_tc, fwd_cols_tc_smem(256), ok);
-  launch_pdl(k_fwd_cols_tc, grid, 128, fwd_cols_tc_smem(npad_max), s, tab, bm, it);
+  launch_chain(it == 0, k_fwd_cols_tc, grid, 128, fwd_cols_tc_smem(npad_max), s, tab, bm, it);
 }
 
 }  // namespace gbn

@@ -570,7 +570,7 @@ void launch_iter_tc(const FusedArgs* tab, const BatchMap& bm, int it, int npad_m
     cudaFuncSetAttribute(k_iter_tc, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     ok = true;
   }
-  launch_pdl(k_iter_tc, grid, kRtNT, rt_smem(npad_max, cnmax), s, tab, bm, it, npad_max, cnmax);
+  launch_chain(it == 0, k_iter_tc, grid, kRtNT, rt_smem(npad_max, cnmax), s, tab, bm, it, npad_max, cnmax);
 }
 
 }  // namespace gbn

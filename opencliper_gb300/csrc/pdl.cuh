@@ -16,9 +16,15 @@ namespace gbn {
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
-// launch with programmatic stream serialisation
+// launch with programmatic stream serialisation (`first`: without it).  The first
+// kernel of a chain follows one that does not release its successors, such as the
+// kernels that write a group's control block, the scalar state or the tiles of a
+// solve.  That one has ended when a successor starts early, but what it wrote is
+// only certain to be seen after the successor's grid_dep_wait(), and these
+// kernels read such data before it: the first one is launched plainly.
 template <typename... KArgs, typename... Args>
-inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, int smem, cudaStream_t s, Args... args) {
+inline void launch_chain(bool first, void (*kernel)(KArgs...), dim3 grid, int threads, int smem, cudaStream_t s,
+                         Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
@@ -28,8 +34,12 @@ inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, int sme
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = first ? 0 : 1;
   cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <typename... KArgs, typename... Args>
+inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, int smem, cudaStream_t s, Args... args) {
+  launch_chain(false, kernel, grid, threads, smem, s, args...);
 }
 
 }  // namespace gbn
