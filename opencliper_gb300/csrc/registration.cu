@@ -118,7 +118,7 @@ struct RegGeom {
   int bb[4] = {0, 0, 0, 0};
   int box0 = 0, box1 = 0;    // bounding box, 0-based inclusive (rows and columns alike)
   int rect0 = 0, rect1 = 0;  // margin rectangle of the interpolators
-  std::vector<float> roi;    // [N][N]
+  int radius2 = 0;           // the region of interest: within the circle around the centre
   std::vector<int> cr;       // [N] first control point of each pixel (0-based)
   std::vector<float> B;      // [3][N][E+1] spline values at each pixel
   std::vector<float> S;      // [3][dp] spline values over a control point's support
@@ -143,23 +143,23 @@ int reg_geometry(int N, int F, const gbn_registration_params* p, RegGeom* g) {
   g->F = F;
   g->E = p->E;
   g->Dp = p->Dp[0];
-  // setMask (GroupwiseRegistration.cpp:486-531)
-  const int radius2 = int(std::pow(p->radius, 2));
+  // setMask (GroupwiseRegistration.cpp:486-531): the device writes the mask
+  // (k_reg_prepare); here its extent and area
+  g->radius2 = int(std::pow(p->radius, 2));
   const float center = float(N + 1) / 2;
-  g->roi.assign(size_t(N) * N, 0.f);
-  int mn = N, mx = -1, mnr = N, mxr = -1;
-  for (int col = 0; col < N; ++col)
-    for (int row = 0; row < N; ++row) {
-      const float Cv = float(std::pow(1 - center + row, 2)), Dv = float(std::pow(1 - center + col, 2));
-      if ((Cv + Dv) <= radius2) {
-        g->roi[size_t(row) * N + col] = 1.f;
-        mn = std::min(mn, col);
-        mx = std::max(mx, col);
-        mnr = std::min(mnr, row);
-        mxr = std::max(mxr, row);
-        g->area++;
-      }
+  std::vector<float> sq(N);
+  for (int q = 0; q < N; ++q) sq[q] = float(std::pow(1 - center + q, 2));
+  int mn = N, mx = -1;
+  for (int row = 0; row < N; ++row) {
+    int n = 0;
+    for (int col = 0; col < N; ++col) n += (sq[row] + sq[col]) <= g->radius2;
+    if (n) {
+      mn = std::min(mn, row);
+      mx = std::max(mx, row);
     }
+    g->area += n;
+  }
+  const int mnr = mn, mxr = mx;  // the mask is its own transpose
   if (g->area == 0) return set_error(GBN_ERR_INVALID, "registration: empty region of interest");
   g->bb[0] = mn + 1;
   g->bb[1] = mnr + 1;
@@ -190,10 +190,16 @@ int reg_geometry(int N, int F, const gbn_registration_params* p, RegGeom* g) {
   g->cr.resize(N);
   for (int q = 0; q < N; ++q) g->cr[q] = kmin[q] - kmin[g->bb[0]];
   g->B.assign(size_t(3) * N * E1, 0.f);
+  std::vector<float> args(size_t(N) * E1);
   for (int q = 0; q < N; ++q)
     for (int s = 0; s < E1; ++s) {
       const float arg = ((float(q + 1) - c) / float(g->Dp)) - float(kmin[q] + s);
-      for (int t = 0; t < 3; ++t) g->B[(size_t(t) * N + q) * E1 + s] = spline_e(t, arg, g->E);
+      args[size_t(q) * E1 + s] = arg;
+      const int r = q - g->Dp;  // most arguments are the ones a control spacing earlier
+      const bool again = r >= 0 && args[size_t(r) * E1 + s] == arg;
+      for (int t = 0; t < 3; ++t)
+        g->B[(size_t(t) * N + q) * E1 + s] =
+            again ? g->B[(size_t(t) * N + r) * E1 + s] : spline_e(t, arg, g->E);
     }
   // control points and supports (ControlPointsLocation, coefg, BBAux1)
   g->sup.resize(g->Cp);
@@ -228,36 +234,61 @@ int reg_geometry(int N, int F, const gbn_registration_params* p, RegGeom* g) {
 }
 
 // ---- device ----
-__global__ void k_reg_absmax(const float2* __restrict__ x, size_t n, unsigned* __restrict__ maxbits) {
+// |x| and its maximum (the modulus in double, as the reference's hypot: FP64
+// bound, so it is formed once)
+__global__ void k_reg_absmax(const float2* __restrict__ x, size_t n, float* __restrict__ I, unsigned* __restrict__ maxbits) {
   float m = 0.f;
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
     const float2 v = x[i];
-    m = fmaxf(m, float(sqrt(double(v.x) * v.x + double(v.y) * v.y)));
+    const float a = float(sqrt(double(v.x) * v.x + double(v.y) * v.y));
+    I[i] = a;
+    m = fmaxf(m, a);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) atomicMax(maxbits, __float_as_uint(m));  // non-negative: bit order = value order
 }
 
-// DataNormalization (initialize.cl:87-102): I = (500 / max) |x|
-__global__ void k_reg_normalize(const float2* __restrict__ x, const unsigned* __restrict__ maxbits, float* __restrict__ I,
-                                size_t n) {
-  const float factor = 500.f / __uint_as_float(*maxbits);
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-    const float2 v = x[i];
-    I[i] = factor * float(sqrt(double(v.x) * v.x + double(v.y) * v.y));
-  }
+// DataNormalization divides by the largest modulus: frames that are all zero
+// (or not finite) have no registration
+__device__ __forceinline__ bool reg_usable(const unsigned* maxbits) {
+  const float m = __uint_as_float(*maxbits);
+  return m > 0.f && m < __uint_as_float(0x7f800000u);
 }
 
-// gradient (optimizer.cl:189-234): central differences, one-sided at the borders
-__global__ void k_reg_imgrad(const float* __restrict__ I, float* __restrict__ d1, float* __restrict__ d2, int N, int F) {
-  const size_t n = size_t(N) * N * F;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-    const int col = int(i % N), row = int((i / N) % N);
-    const float* f = I + (i - size_t(row) * N - col);
-    const size_t p = size_t(row) * N + col;
-    d1[i] = col == 0 ? f[p + 1] - f[p] : col == N - 1 ? f[p] - f[p - 1] : (f[p + 1] - f[p - 1]) / 2;
-    d2[i] = row == 0 ? f[p + N] - f[p] : row == N - 1 ? f[p] - f[p - N] : (f[p + N] - f[p - N]) / 2;
+// Per pixel of a frame: DataNormalization (initialize.cl:87-102), I = (500 / max)
+// |x|, the image gradients (optimizer.cl:189-234: central differences, one-sided
+// at the borders), the identity mesh; with the first frame also the mask and the
+// original mesh.  The neighbours' values are normalised again, not read back.
+__global__ void k_reg_prepare(const float* __restrict__ A, const unsigned* __restrict__ maxbits, float* __restrict__ I,
+                              float* __restrict__ d1, float* __restrict__ d2, float* __restrict__ roi,
+                              int* __restrict__ xmesh, float* __restrict__ xn, int N, int F, int radius2) {
+  if (!reg_usable(maxbits)) return;
+  const float factor = 500.f / __uint_as_float(*maxbits);
+  const size_t NN = size_t(N) * N;
+  const int f = blockIdx.y;
+  const float* a = A + f * NN;
+  auto v = [&](size_t q) { return factor * a[q]; };
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < int(NN); p += gridDim.x * blockDim.x) {
+    const int row = p / N, col = p - row * N;
+    const size_t o = f * NN + p;
+    const float c = v(p);
+    I[o] = c;
+    d1[o] = col == 0 ? v(p + 1) - c : col == N - 1 ? c - v(p - 1) : (v(p + 1) - v(p - 1)) / 2;
+    d2[o] = row == 0 ? v(p + N) - c : row == N - 1 ? c - v(p - N) : (v(p + N) - v(p - N)) / 2;
+    xn[o] = float(col + 1);
+    xn[size_t(F) * NN + o] = float(row + 1);
+    if (f == 0) {
+      const float center = float(N + 1) / 2;
+      const float cv = 1 - center + row, dv = 1 - center + col;
+      roi[p] = (float(double(cv) * cv) + float(double(dv) * dv)) <= radius2 ? 1.f : 0.f;
+      if (xmesh) {
+        // ArgumentsMotionCompensation::xData: [2][N][N] with the first index the
+        // column (x[i + j N] = j + 1 in plane 0, i + 1 in plane 1)
+        xmesh[p] = row + 1;
+        xmesh[NN + p] = col + 1;
+      }
+    }
   }
 }
 
@@ -299,6 +330,25 @@ __device__ __forceinline__ bool reg_bilinear(const float* __restrict__ img, int 
   const float a = float(ph + 1) - nh, b = nh - float(ph), cc = float(pv + 1) - nv, d = nv - float(pv);
   const float aux1 = a * i1 + b * i2, aux2 = a * i3 + b * i4;
   *out = cc * aux1 + d * aux2;
+  return true;
+}
+
+// the same of three images at one place
+__device__ __forceinline__ bool reg_bilinear3(const float* __restrict__ p1, const float* __restrict__ p2,
+                                              const float* __restrict__ p3, int N, float xh, float xv, float* o1,
+                                              float* o2, float* o3) {
+  const float nh = xh - 1, nv = xv - 1;
+  const int ph = int(floorf(nh)), pv = int(floorf(nv));
+  if (ph < 0 || pv < 0 || ph + 1 >= N || pv + 1 >= N) return false;
+  const size_t q = ph + size_t(pv) * N;
+  const float a = float(ph + 1) - nh, b = nh - float(ph), cc = float(pv + 1) - nv, d = nv - float(pv);
+  auto at = [&](const float* p) {
+    const float aux1 = a * p[q] + b * p[q + 1], aux2 = a * p[q + N] + b * p[q + N + 1];
+    return cc * aux1 + d * aux2;
+  };
+  *o1 = at(p1);
+  *o2 = at(p2);
+  *o3 = at(p3);
   return true;
 }
 
@@ -575,24 +625,429 @@ __device__ void reg_finish(RegArgs& a, int it, int nh, int nd, float et, float e
   if (it == st->nmax || (Tdif < st->p2 && Hdif < st->p4)) st->done = 1;
 }
 
-__global__ void k_reg_mesh(int* __restrict__ xmesh, float* __restrict__ xn, int N, int F) {
-  const size_t NN = size_t(N) * N;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < NN; i += size_t(gridDim.x) * blockDim.x) {
-    // ArgumentsMotionCompensation::xData: [2][N][N] with the first index the
-    // column (x[i + j N] = j + 1 in plane 0, i + 1 in plane 1)
-    const int a0 = int(i % N), b0 = int(i / N);
-    if (xmesh) {
-      xmesh[i] = b0 + 1;
-      xmesh[NN + i] = a0 + 1;
+// ---------------------------------------------------------------------------
+// The whole gradient descent in one cooperative launch, for the reference's cubic
+// splines at spacing 4 without smoothness terms (its defaults).  An iteration is
+// two phases with a grid barrier after each:
+//   1  dH (auxiliarCost, cost6DReduction, cost6D): a CTA takes a block of 8 x 12
+//      control points of one (d, frame), stages the 45 x 61 values they cover and
+//      sums them in the reference's order; other CTAs form the metric's partial
+//      sums of the iteration before, 256 pixels each
+//   2  evolution() and stopCondition() of the iteration before; then per tile of
+//      8 x 4 pixels, all frames: T - Wn (dH - mean_f dH) of the control
+//      points that reach it (each CTA for itself, from the same numbers), xn, the
+//      warped frames, their mean and variance, and dy dx masked, which is all that
+//      phase 1 reads.  T itself is updated once more, into the other buffer, in
+//      the element blocks whose sums of Dif^2 the stopping rule reads.
+// Every sum runs in the order of the kernels above (k_reg_grad ... k_reg_metric),
+// so the results are theirs bit for bit.  Bound by the latency of the two phases
+// and barriers: about 24 K cycles an iteration at 256 x 256 x 20, radius 40, of which
+// the barriers 8 K; a registration of 100 iterations 4.47 -> 1.6 ms (400 launches of
+// ~10 us each on grids of 25 to 1,400 small CTAs before).
+// Data that other CTAs write is read with __ldcg: L1 is not coherent within a launch.
+// ---------------------------------------------------------------------------
+constexpr int kSolveDp = 4, kSolveSup = 17, kSolveE1 = 4;
+constexpr int kSolveKB = 8, kSolveLB = 12;                            // control points of a phase-1 unit
+constexpr int kSolveTR = (kSolveKB - 1) * kSolveDp + kSolveSup;       // and the rows and columns they cover
+constexpr int kSolveTC = (kSolveLB - 1) * kSolveDp + kSolveSup;
+constexpr int kTileW = 8, kTileH = 4, kTilePix = kTileW * kTileH;     // pixels of a phase-2 tile
+constexpr int kTilePts = (kTileH / kSolveDp + kSolveE1) * (kTileW / kSolveDp + kSolveE1);  // control points that reach it, at most
+constexpr int kTileFG = kRegNT / kTilePix;                            // frames in flight per pixel
+static_assert(kTilePts <= 32, "a control point of the tile per lane");
+constexpr int kSolveMaxF = 64;
+constexpr int kStatusBarrier = 8;
+constexpr unsigned kBarrierPolls = 1u << 22;
+
+struct RegSolve {
+  RegArgs a;
+  float* Tb[2];     // T of even and odd iterations; Tb[0] is the caller's T
+  float* pd;        // [2][F][N][N] dy dx inside the region of interest, 0 elsewhere
+  float* hv;        // [L][L] V inside the region of interest
+  unsigned* bar;    // grid barrier's arrivals
+  const unsigned* maxbits;
+  float et, eh;
+  int nmax, flagW, L, ntx, ntiles, nkb, nlb, nunits, gu;
+};
+
+// All CTAs of the launch; false (and the status) if some did not arrive in time.
+// (Polling the counter itself: 3.4 K cycles from arrival to release; a flag that
+// the last one raises on another line, 5.7 K.)
+__device__ __forceinline__ bool reg_barrier(const RegSolve& s, unsigned target) {
+  __shared__ bool ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(s.bar, 1u);
+    unsigned seen = 0, polls = 0;
+    for (;;) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(seen) : "l"(s.bar) : "memory");
+      if (seen >= target || ++polls >= kBarrierPolls) break;
+      __nanosleep(32);
     }
-    const int row = b0, col = a0;
-    for (int f = 0; f < F; ++f) {
-      xn[size_t(f) * NN + i] = float(col + 1);
-      xn[(size_t(F) + f) * NN + i] = float(row + 1);
-    }
+    ok = seen >= target;
+    if (!ok) atomicExch(&s.a.st->status, kStatusBarrier);
   }
+  __syncthreads();
+  return ok;
 }
 
+// What iteration `it` came to (reg_finish), by every CTA for itself from the same
+// partial sums in the same order, so that no CTA waits for another one's result;
+// CTA 0 keeps the record.  ss: Wn, the metric before, the thresholds, done.
+struct RegScalars {
+  float Wn, H, p2, p4;
+  int done;
+};
+__device__ __forceinline__ void reg_solve_scalars(const RegSolve& s, int it, float h, float dd, float* sw2, RegScalars* ss) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    h += __shfl_down_sync(0xffffffffu, h, o);
+    dd += __shfl_down_sync(0xffffffffu, dd, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sw2[threadIdx.x >> 5] = h;
+    sw2[kRegNT / 32 + (threadIdx.x >> 5)] = dd;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float H = 0.f, D = 0.f;
+#pragma unroll
+    for (int w = 0; w < kRegNT / 32; ++w) {
+      H = H + sw2[w];
+      D = D + sw2[kRegNT / 32 + w];
+    }
+    RegState* const st = s.a.st;
+    const bool keep = blockIdx.x == 0;
+    if (keep) s.a.H[it] = H;
+    if (it == 0) {
+      ss->p2 = s.et * float(s.a.F * 2);
+      ss->p4 = H * s.eh;
+      ss->done = 0;
+    } else {
+      const float Tdif = sqrtf(D);
+      const float Hdif = ss->H - H;
+      if (s.flagW) ss->Wn = Hdif > 0 ? float(double(ss->Wn) * 1.2) : ss->Wn / 2;
+      ss->done = it == s.nmax || (Tdif < ss->p2 && Hdif < ss->p4);
+      if (keep) {
+        st->Wn = ss->Wn;
+        st->Tdif = Tdif;
+        st->Hdif = Hdif;
+        st->it = it;
+        st->done = ss->done;
+      }
+    }
+    ss->H = H;
+  }
+  __syncthreads();
+}
+
+// FMAX: frames the registers are for (24 or 64)
+template <int FMAX>
+__global__ void __launch_bounds__(kRegNT, 2) k_reg_solve(RegSolve s) {
+  __shared__ union {
+    struct {
+      float tile[kSolveTR][kSolveTC];
+      float cs[kSolveKB * kSolveLB * kSolveSup];
+    } g;
+    struct {
+      float dH[2 * FMAX][32], T[2 * FMAX][32], mean[2][32];  // [d*F + f][control point of the tile]
+      float iw[FMAX][kTilePix], pmean[kTilePix];
+    } w;
+  } sm;
+  __shared__ float sw[2 * (kRegNT / 32)];
+  __shared__ RegScalars ss;
+  if (!reg_usable(s.maxbits)) return;
+  RegArgs& a = s.a;
+  RegState* const st = a.st;
+  const int t = threadIdx.x, F = a.F, N = a.N, Cp = a.Cp, CC = Cp * Cp, nT = 2 * F * CC;
+  const size_t NN = size_t(N) * N;
+  if (t == 0) ss.Wn = st->Wn;
+  const int sup0 = a.sup[0], lane = t & 31, wid = t >> 5;
+  unsigned gen = 0;
+  int fin = 0;  // iterations done
+  // phase 1: a thread keeps its column offset j, and so the products S_i S_j
+  constexpr int kRound = kRegNT / kSolveSup, NI = (kSolveKB * kSolveLB + kRound - 1) / kRound;
+  const int j1 = t % kSolveSup, cp1 = t / kSolveSup;
+  float SS[kSolveSup];
+#pragma unroll
+  for (int i = 0; i < kSolveSup; ++i) SS[i] = a.S[i] * a.S[j1];
+  // phase 2: the CTA's tile (its first one is set up once), pixel px of it, frames
+  // fg, fg + kTileFG, ...; a control point per lane, a (d, frame) per warp and round
+  constexpr int K = 2 * FMAX / (kRegNT / 32);
+  const int px = t % kTilePix, fg = t / kTilePix;
+  int row = 0, col = 0, npc = 1, o0 = 0, pt = 0;
+  bool in = false;
+  float roi = 0.f, bb[kSolveE1][kSolveE1];  // [column offset][row offset]
+  size_t p = 0;
+  auto set_tile = [&](int tile) {
+    const int ty = tile / s.ntx, tx = tile % s.ntx;
+    const int row0 = a.box0 + ty * kTileH, col0 = a.box0 + tx * kTileW;
+    const int rowl = min(row0 + kTileH - 1, a.box1), coll = min(col0 + kTileW - 1, a.box1);
+    const int pr = a.cr[row0], pc = a.cr[col0];  // the first control point that reaches the tile, and how many do
+    npc = a.cr[coll] + kSolveE1 - pc;
+    const int np = (a.cr[rowl] + kSolveE1 - pr) * npc;
+    pt = lane < np ? (pr + lane / npc) * Cp + pc + lane % npc : pr * Cp + pc;
+    row = row0 + px / kTileW;
+    col = col0 + px % kTileW;
+    in = row <= a.box1 && col <= a.box1;
+    const int rr = min(row, a.box1), cc = min(col, a.box1);
+    p = size_t(rr) * N + cc;
+    roi = a.roi[p];
+#pragma unroll
+    for (int aa = 0; aa < kSolveE1; ++aa)
+#pragma unroll
+      for (int b = 0; b < kSolveE1; ++b) bb[aa][b] = a.B[size_t(rr) * kSolveE1 + b] * a.B[size_t(cc) * kSolveE1 + aa];
+    o0 = (a.cr[rr] - pr) * npc + a.cr[cc] - pc;
+  };
+  float tv[K], dv[K];
+  auto load_pts = [&](int it, const float* Told) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int df = wid + k * (kRegNT / 32);
+      if (df < 2 * F) {
+        tv[k] = __ldcg(Told + size_t(df) * CC + pt);
+        if (it > 0) dv[k] = __ldcg(a.dH + size_t(df) * CC + pt);
+      }
+    }
+  };
+  const bool one_tile = s.ntiles <= int(gridDim.x);
+  if (int(blockIdx.x) < s.ntiles) set_tile(blockIdx.x);
+
+  for (int it = 0;; ++it) {
+    // ---- phase 1: dH of iteration it, and what iteration it - 1 came to
+    if (it > 0) {
+      const int nh = (s.L * s.L + kRegNT - 1) / kRegNT;
+      for (int u = it > s.nmax ? s.nunits + int(blockIdx.x) : int(blockIdx.x); u < s.nunits + nh; u += gridDim.x) {
+        if (u >= s.nunits) {  // k_reg_metric's partial sum of 256 pixels, iteration it - 1
+          const int q = (u - s.nunits) * kRegNT + t;
+          const float v = reg_block_sum(q < s.L * s.L ? __ldcg(s.hv + q) : 0.f, sw);
+          if (t == 0) a.part_h[u - s.nunits] = v;
+          __syncthreads();
+          continue;
+        }
+        const int lb = u % s.nlb, kb = (u / s.nlb) % s.nkb, df = u / (s.nlb * s.nkb);  // df = d*F + f
+        const int k0 = kb * kSolveKB, l0 = lb * kSolveLB, nk = min(kSolveKB, Cp - k0), nl = min(kSolveLB, Cp - l0);
+        const int tr = (nk - 1) * kSolveDp + kSolveSup, tc = (nl - 1) * kSolveDp + kSolveSup;
+        const float* src = s.pd + df * NN + size_t(sup0 + k0 * kSolveDp) * N + sup0 + l0 * kSolveDp;
+        {
+          constexpr int R = (kSolveTR + kRegNT / 64 - 1) / (kRegNT / 64);
+          float v[R];
+          const int r0 = t / 64, c = t % 64;
+#pragma unroll
+          for (int n = 0; n < R; ++n) {
+            const int r = r0 + n * (kRegNT / 64);
+            if (r < tr && c < tc) v[n] = __ldcg(src + size_t(r) * N + c);
+          }
+#pragma unroll
+          for (int n = 0; n < R; ++n) {
+            const int r = r0 + n * (kRegNT / 64);
+            if (r < tr && c < tc) sm.g.tile[r][c] = v[n];
+          }
+        }
+        __syncthreads();
+        {
+          // the thread's control points side by side; those past the block's edge
+          // read what the tile holds and are not kept
+          const float* v[NI];
+          float acc[NI];
+#pragma unroll
+          for (int n = 0; n < NI; ++n) {
+            const int cp = min(cp1 + n * kRound, kSolveKB * kSolveLB - 1);
+            v[n] = &sm.g.tile[cp / kSolveLB * kSolveDp][cp % kSolveLB * kSolveDp + j1];
+            acc[n] = 0.f;
+          }
+#pragma unroll
+          for (int i = 0; i < kSolveSup; ++i)
+#pragma unroll
+            for (int n = 0; n < NI; ++n) acc[n] = acc[n] + v[n][i * kSolveTC] * SS[i];
+#pragma unroll
+          for (int n = 0; n < NI; ++n) {
+            const int cp = cp1 + n * kRound;
+            if (cp1 < kRound && cp < kSolveKB * kSolveLB) sm.g.cs[cp * kSolveSup + j1] = acc[n];
+          }
+        }
+        __syncthreads();
+        if (t < kSolveKB * kSolveLB && t / kSolveLB < nk && t % kSolveLB < nl) {
+          float acc = 0.f;
+#pragma unroll
+          for (int j = 0; j < kSolveSup; ++j) acc = acc + sm.g.cs[t * kSolveSup + j];
+          a.dH[size_t(df) * CC + (k0 + t / kSolveLB) * Cp + l0 + t % kSolveLB] = acc;
+        }
+        __syncthreads();
+      }
+      if (!reg_barrier(s, (gen += gridDim.x))) return;
+    }
+    // ---- phase 2
+    const float* const Told = s.Tb[it == 0 ? 0 : (it - 1) & 1];
+    if (int(blockIdx.x) < s.ntiles) {  // under way while the scalars are formed
+      if (!one_tile && it > 0) set_tile(blockIdx.x);
+      load_pts(it, Told);
+    }
+    if (it > 0) {
+      const int nh = (s.L * s.L + kRegNT - 1) / kRegNT;
+      float h = 0.f, dd = 0.f;
+      for (int q = t; q < nh; q += kRegNT) h = h + __ldcg(a.part_h + q);
+      if (it > 1)
+        for (int q = t; q < s.gu; q += kRegNT) dd = dd + __ldcg(a.part_d + q);
+      reg_solve_scalars(s, it - 1, h, dd, sw, &ss);
+      if (ss.done) {
+        fin = it - 1;
+        break;
+      }
+    }
+    const float Wn = ss.Wn;
+    if (it > 0) {
+      float* const Tnew = s.Tb[it & 1];
+      // k_reg_update's blocks, from the CTAs that have no tile
+      for (int b = int(gridDim.x - 1 - blockIdx.x); b < s.gu; b += gridDim.x) {
+        const int q = b * kRegNT + t;
+        float dd = 0.f;
+        if (q < nT) {
+          const int cp = q % CC, d = q / (CC * F);
+          const float* col = a.dH + size_t(d) * F * CC + cp;
+          const float mine = __ldcg(a.dH + q), old = __ldcg(Told + q);
+          float sum = 0.f;
+          for (int f0 = 0; f0 < F; f0 += 16) {
+            float v[16];
+#pragma unroll
+            for (int n = 0; n < 16; ++n) v[n] = f0 + n < F ? __ldcg(col + size_t(f0 + n) * CC) : 0.f;
+#pragma unroll
+            for (int n = 0; n < 16; ++n)
+              if (f0 + n < F) sum = sum + v[n];
+          }
+          const float dif = Wn * (mine - sum / F);
+          Tnew[q] = old - dif;
+          dd = dif * dif;
+        }
+        const float v = reg_block_sum(dd, sw);
+        if (t == 0) a.part_d[b] = v;
+        __syncthreads();
+      }
+    }
+    for (int tile = blockIdx.x; tile < s.ntiles; tile += gridDim.x) {
+      if (tile != int(blockIdx.x)) {
+        set_tile(tile);
+        load_pts(it, Told);
+      }
+      {
+        if (it > 0) {
+#pragma unroll
+          for (int k = 0; k < K; ++k) {
+            const int df = wid + k * (kRegNT / 32);
+            if (df < 2 * F) sm.w.dH[df][lane] = dv[k];
+          }
+          __syncthreads();
+          if (wid < 2) {
+            float sum = 0.f;
+#pragma unroll 8
+            for (int f = 0; f < F; ++f) sum = sum + sm.w.dH[wid * F + f][lane];
+            sm.w.mean[wid][lane] = sum / F;
+          }
+          __syncthreads();
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const int df = wid + k * (kRegNT / 32);
+          if (df < 2 * F) {
+            if (it > 0) {
+              const float dif = Wn * (dv[k] - sm.w.mean[df >= F][lane]);
+              tv[k] = tv[k] - dif;
+            }
+            sm.w.T[df][lane] = tv[k];
+          }
+        }
+        __syncthreads();
+      }
+      float g1[FMAX / kTileFG], g2[FMAX / kTileFG];
+      if (in) {
+        float u[FMAX / kTileFG][2];  // the displacements of the frames, side by side
+#pragma unroll
+        for (int k = 0; k < FMAX / kTileFG; ++k) u[k][0] = u[k][1] = 0.f;
+#pragma unroll
+        for (int aa = 0; aa < kSolveE1; ++aa)
+#pragma unroll
+          for (int b = 0; b < kSolveE1; ++b)
+#pragma unroll
+            for (int k = 0; k < FMAX / kTileFG; ++k) {
+              const int f = min(fg + k * kTileFG, F - 1);
+#pragma unroll
+              for (int d = 0; d < 2; ++d) u[k][d] = u[k][d] + sm.w.T[d * F + f][o0 + b * npc + aa] * bb[aa][b];
+            }
+#pragma unroll
+        for (int k = 0; k < FMAX / kTileFG; ++k) {
+          const int f = fg + k * kTileFG;
+          if (f < F) {
+            const float xh = u[k][0] + float(col + 1), xv = u[k][1] + float(row + 1);
+            float iw = 0.f;
+            const float *d1 = a.d1 + f * NN, *d2 = a.d2 + f * NN, *I = a.I + f * NN;
+            if (!reg_bilinear3(d1, d2, I, N, xh, xv, &g1[k], &g2[k], &iw)) {
+              atomicExch(&st->status, kStatusRange);
+              iw = I[p];
+              g1[k] = g2[k] = 0.f;
+            } else if (it == 0) {
+              iw = I[p];
+            }
+            sm.w.iw[f][px] = iw;
+          }
+        }
+      }
+      __syncthreads();
+      if (t < kTilePix && in) {
+        float sum = 0.f;
+#pragma unroll 8
+        for (int f = 0; f < F; ++f) sum = sum + sm.w.iw[f][px];
+        const float mean = sum / F;
+        float V = 0.f;
+#pragma unroll 8
+        for (int f = 0; f < F; ++f) {
+          const float dl = sm.w.iw[f][px] - mean;
+          V = V + dl * dl;
+        }
+        V = V / F;
+        sm.w.pmean[px] = mean;
+        s.hv[(row - a.box0) * s.L + col - a.box0] = V * roi;
+      }
+      __syncthreads();
+      if (in) {
+        const float m = roi, mean = sm.w.pmean[px];
+#pragma unroll
+        for (int k = 0; k < FMAX / kTileFG; ++k) {
+          const int f = fg + k * kTileFG;
+          if (f < F) {
+            const float dy = (sm.w.iw[f][px] - mean) * a.fac;
+            s.pd[f * NN + p] = dy * g1[k] * m;
+            s.pd[(size_t(F) + f) * NN + p] = dy * g2[k] * m;
+          }
+        }
+      }
+      __syncthreads();
+    }
+    if (!reg_barrier(s, (gen += gridDim.x))) return;
+  }
+
+  // the iterations done, and the mesh at their T
+  const int last = fin;
+  const float* const T = s.Tb[last & 1];
+  if (last & 1)
+    for (int q = blockIdx.x * kRegNT + t; q < nT; q += gridDim.x * kRegNT) s.Tb[0][q] = __ldcg(T + q);
+  const int npx = s.L * s.L * F;
+  for (int q = blockIdx.x * kRegNT + t; q < npx; q += gridDim.x * kRegNT) {
+    const int pix = q % (s.L * s.L), f = q / (s.L * s.L), row = a.box0 + pix / s.L, col = a.box0 + pix % s.L;
+    const size_t p = size_t(row) * N + col;
+    float u[2];
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+      const float* Tf = T + (size_t(d) * F + f) * CC + a.cr[row] * Cp + a.cr[col];
+      float acc = 0.f;
+      for (int aa = 0; aa < kSolveE1; ++aa)
+        for (int b = 0; b < kSolveE1; ++b)
+          acc = acc + __ldcg(Tf + b * Cp + aa) * (a.B[size_t(row) * kSolveE1 + b] * a.B[size_t(col) * kSolveE1 + aa]);
+      u[d] = acc;
+    }
+    a.xn[size_t(f) * NN + p] = u[0] + float(col + 1);
+    a.xn[(size_t(F) + f) * NN + p] = u[1] + float(row + 1);
+  }
+}
 
 // bump allocation of the work arrays in one block (256-byte aligned); a pass
 // with a null base sizes the block
@@ -630,34 +1085,70 @@ int registration_run(gbn_ctx* ctx, const float2* images, int N, int F, const gbn
   if (rc != GBN_OK) return rc;
   cudaStream_t s = ctx->stream;
   const size_t NN = size_t(N) * N, X = NN * F, nT = size_t(2) * F * g.Cp * g.Cp;
+  const int L = g.box1 - g.box0 + 1;
+  const int gu = int((nT + kRegNT - 1) / kRegNT);
+  // the one-launch descent takes the reference's default splines; other orders,
+  // spacings, smoothness terms and more frames run a launch per step
+  RegSolve sv{};
+  sv.ntx = (L + kTileW - 1) / kTileW;
+  sv.ntiles = sv.ntx * ((L + kTileH - 1) / kTileH);
+  sv.nkb = (g.Cp + kSolveKB - 1) / kSolveKB;
+  sv.nlb = (g.Cp + kSolveLB - 1) / kSolveLB;
+  sv.nunits = 2 * F * sv.nkb * sv.nlb;
+  int solve_grid = 0;
+  if (g.E + 1 == kSolveE1 && g.Dp == kSolveDp && g.dp == kSolveSup && F <= kSolveMaxF && g.sum_lambda == 0) {
+    static int per_sm = -1;
+    if (per_sm < 0 &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_reg_solve<kSolveMaxF>, kRegNT, 0) != cudaSuccess) {
+      cudaGetLastError();
+      per_sm = 0;
+    }
+    // every CTA of the launch is resident
+    solve_grid = std::min(ctx->nsm * per_sm, std::max(sv.nunits, sv.ntiles + gu));
+  }
+  const bool solve = solve_grid > 0;
   // all work arrays in one grow-only block of the context (no allocation
-  // after the first call of a size)
+  // after the first call of a size); the host-made tables lie together
   RegArgs a{};
-  float *I, *d1, *d2, *roi, *B, *S, *dH, *Dif, *Iw, *dy, *dx, *H, *part_h, *part_d, *sterm = nullptr;
+  float *I, *A, *d1, *d2, *roi, *B, *S, *dH, *Dif = nullptr, *Iw = nullptr, *dy = nullptr, *dx = nullptr, *H, *part_h,
+                                        *part_d, *sterm = nullptr;
   int *cr, *sup;
   unsigned* maxbits;
   RegState* st;
-  const size_t L2 = size_t(g.box1 - g.box0 + 1) * (g.box1 - g.box0 + 1);
+  const size_t L2 = size_t(L) * L;
+  size_t tab0 = 0, tab1 = 0;
   auto plan = [&](Carve& c) {
     I = c.take<float>(X);
     d1 = c.take<float>(X);
     d2 = c.take<float>(X);
     roi = c.take<float>(NN);
-    B = c.take<float>(g.B.size());
-    S = c.take<float>(g.S.size());
     dH = c.take<float>(nT);
-    Dif = c.take<float>(nT);
-    Iw = c.take<float>(X);
-    dy = c.take<float>(X);
-    dx = c.take<float>(2 * X);
     H = c.take<float>(size_t(prm->nmax) + 1);
     part_h = c.take<float>(L2 / kRegNT + 1);
     part_d = c.take<float>(nT / kRegNT + 1);
-    sterm = g.sum_lambda != 0 ? c.take<float>(size_t(F) * 14 * L2) : nullptr;
+    if (solve) {
+      sv.Tb[1] = c.take<float>(nT);
+      sv.hv = c.take<float>(L2);
+      sv.pd = c.take<float>(2 * X);
+      A = sv.pd;  // the moduli, until the descent's first products
+    } else {
+      Dif = c.take<float>(nT);
+      Iw = c.take<float>(X);
+      dy = c.take<float>(X);
+      dx = c.take<float>(2 * X);
+      A = Iw;
+      sterm = g.sum_lambda != 0 ? c.take<float>(size_t(F) * 14 * L2) : nullptr;
+    }
+    c.off = (c.off + 255) & ~size_t(255);
+    tab0 = c.off;
+    st = c.take<RegState>(1);
+    maxbits = c.take<unsigned>(1);
+    sv.bar = c.take<unsigned>(32);  // a line of its own
+    B = c.take<float>(g.B.size());
+    S = c.take<float>(g.S.size());
     cr = c.take<int>(size_t(N));
     sup = c.take<int>(size_t(g.Cp));
-    maxbits = c.take<unsigned>(1);
-    st = c.take<RegState>(1);
+    tab1 = c.off;
   };
   Carve sizer{nullptr, 0};
   plan(sizer);
@@ -669,40 +1160,28 @@ int registration_run(gbn_ctx* ctx, const float2* images, int N, int F, const gbn
   h0.Wn = g.Wn0;
   h0.nmax = prm->nmax;
   h0.flagW = prm->flagW ? 1 : 0;
-  cudaError_t e = cudaMemcpyAsync(roi, g.roi.data(), NN * sizeof(float), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(B, g.B.data(), g.B.size() * sizeof(float), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(S, g.S.data(), g.S.size() * sizeof(float), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(cr, g.cr.data(), N * sizeof(int), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(sup, g.sup.data(), g.Cp * sizeof(int), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(st, &h0, sizeof(h0), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(maxbits, 0, sizeof(unsigned), s);
-  // the gradient reads dy and dx over whole supports, outside the bounding box
-  // times a zero mask: zero there
-  if (e == cudaSuccess) e = cudaMemsetAsync(dy, 0, X * sizeof(float), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(dx, 0, 2 * X * sizeof(float), s);
+  // state, counters and tables in one copy
+  std::vector<unsigned char> tab(tab1 - tab0, 0);
+  char* const base = static_cast<char*>(block);
+  auto put = [&](const void* dev, const void* host, size_t bytes) {
+    std::memcpy(tab.data() + (static_cast<const char*>(dev) - base - tab0), host, bytes);
+  };
+  put(st, &h0, sizeof(h0));
+  put(B, g.B.data(), g.B.size() * sizeof(float));
+  put(S, g.S.data(), g.S.size() * sizeof(float));
+  put(cr, g.cr.data(), N * sizeof(int));
+  put(sup, g.sup.data(), g.Cp * sizeof(int));
+  cudaError_t e = cudaMemcpyAsync(st, tab.data(), tab.size(), cudaMemcpyHostToDevice, s);
   // T_init may be T_out itself (a continuation in place)
   if (e == cudaSuccess && T_init != T_out)
     e = T_init ? cudaMemcpyAsync(T_out, T_init, nT * sizeof(float), cudaMemcpyDeviceToDevice, s)
                : cudaMemsetAsync(T_out, 0, nT * sizeof(float), s);
   if (e != cudaSuccess) return cuda_status(e, "registration setup");
   const int gx = int(std::min<size_t>((X + kRegNT - 1) / kRegNT, size_t(ctx->nsm) * 8));
-  k_reg_absmax<<<gx, kRegNT, 0, s>>>(images, X, maxbits);
-  {
-    // DataNormalization divides by the largest modulus: frames that are all
-    // zero (or not finite) have no registration
-    unsigned mb = 0;
-    if ((e = cudaMemcpyAsync(&mb, maxbits, sizeof(mb), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(s)) != cudaSuccess)
-      return cuda_status(e, "registration");
-    float mx;
-    std::memcpy(&mx, &mb, sizeof(mx));
-    if (!(mx > 0.f) || !std::isfinite(mx)) return set_error(GBN_ERR_INVALID, "registration: frames all zero, or an infinite modulus");
-  }
-  k_reg_normalize<<<gx, kRegNT, 0, s>>>(images, maxbits, I, X);
-  k_reg_imgrad<<<gx, kRegNT, 0, s>>>(I, d1, d2, N, F);
-  k_reg_mesh<<<int(std::min<size_t>((NN + kRegNT - 1) / kRegNT, size_t(ctx->nsm) * 8)), kRegNT, 0, s>>>(xmesh_out,
-                                                                                                       xn_out, N, F);
-  ctx->launches += 4;
+  k_reg_absmax<<<gx, kRegNT, 0, s>>>(images, X, A, maxbits);
+  const dim3 gp2(unsigned(std::min<size_t>((NN + kRegNT - 1) / kRegNT, 65535)), F);
+  k_reg_prepare<<<gp2, kRegNT, 0, s>>>(A, maxbits, I, d1, d2, roi, xmesh_out, xn_out, N, F, g.radius2);
+  ctx->launches += 2;
   a.N = N;
   a.F = F;
   a.Cp = g.Cp;
@@ -735,52 +1214,91 @@ int registration_run(gbn_ctx* ctx, const float2* images, int N, int F, const gbn
   a.part_h = part_h;
   a.part_d = part_d;
   a.st = st;
-  const int L = g.box1 - g.box0 + 1;
-  const int gp = (L * L + kRegNT - 1) / kRegNT;
-  const int gw = (L * L * F + kRegNT - 1) / kRegNT;
-  const int gpc = kRegNT / g.dp;
-  const int gg = (2 * F * g.Cp * g.Cp + gpc - 1) / gpc;
-  const int gu = int((nT + kRegNT - 1) / kRegNT);
-  // the unregistered frames: metric H[0]; dx at the starting mesh (optimizer.cpp: InitIT, Metric, CostReduction)
-  k_reg_warp<<<gw, kRegNT, 0, s>>>(a);
-  k_reg_metric<<<gp, kRegNT, 0, s>>>(a, 0, gu, prm->et, prm->eh);
-  ctx->launches += 2;
-  a.warp = 1;
-  a.smooth = g.sum_lambda != 0;
-  // chunks of iterations with one chunk of lookahead: while the GPU runs chunk
-  // c the host waits for chunk c-1's stop flag (copied to pinned memory behind
-  // it), so the queue never drains; after the stop, the chunk already queued
-  // returns at each kernel's entry
-  if ((rc = host_flags_ready(ctx)) != GBN_OK) return rc;
-  RegState hs{};
-  int chunk = 0;
-  for (int it = 1; it <= prm->nmax; ++chunk) {
-    for (int k = 0; k < kRegChunk && it <= prm->nmax; ++k, ++it) {
-      // plain launches: chained by programmatic dependent launch these small
-      // grids ran slower (6.3 against 5.1 ms per registration at 256^2 x 20)
-      if (g.dp == 17)
-        k_reg_grad<17><<<gg, kRegNT, 0, s>>>(a);
-      else
-        k_reg_grad<0><<<gg, kRegNT, 0, s>>>(a);
-      k_reg_update<<<gu, kRegNT, 0, s>>>(a);
-      k_reg_warp<<<gw, kRegNT, 0, s>>>(a);
-      k_reg_metric<<<gp, kRegNT, 0, s>>>(a, it, gu, prm->et, prm->eh);
-      ctx->launches += 4;
-    }
-    if ((e = cudaMemcpyAsync(&ctx->host_flags[chunk & 1], &st->done, sizeof(int), cudaMemcpyDeviceToHost, s)) !=
-            cudaSuccess ||
-        (e = cudaEventRecord(ctx->ev_flag[chunk & 1], s)) != cudaSuccess)
+  unsigned mb = 0;
+  auto bad_frames = [&]() {
+    float mx;
+    std::memcpy(&mx, &mb, sizeof(mx));
+    return !(mx > 0.f) || !std::isfinite(mx);
+  };
+  static const char* kBadFrames = "registration: frames all zero, or an infinite modulus";
+  if (solve) {
+    // what phase 1 reads outside the bounding box is zero
+    if ((e = cudaMemsetAsync(sv.pd, 0, 2 * X * sizeof(float), s)) != cudaSuccess) return cuda_status(e, "registration");
+    sv.a = a;
+    sv.Tb[0] = T_out;
+    sv.maxbits = maxbits;
+    sv.et = prm->et;
+    sv.eh = prm->eh;
+    sv.nmax = prm->nmax;
+    sv.flagW = h0.flagW;
+    sv.L = L;
+    sv.gu = gu;
+    void* args[] = {&sv};
+    const void* kernel = F <= 24 ? reinterpret_cast<const void*>(k_reg_solve<24>)
+                                 : reinterpret_cast<const void*>(k_reg_solve<kSolveMaxF>);
+    e = cudaLaunchCooperativeKernel(kernel, dim3(solve_grid), dim3(kRegNT), args, 0, s);
+    if (e != cudaSuccess) return cuda_status(e, "registration");
+    ctx->launches += 1;
+    if ((e = cudaMemcpyAsync(&mb, maxbits, sizeof(mb), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
       return cuda_status(e, "registration");
-    if (chunk > 0) {
-      if ((e = cudaEventSynchronize(ctx->ev_flag[(chunk - 1) & 1])) != cudaSuccess) return cuda_status(e, "registration");
-      if (ctx->host_flags[(chunk - 1) & 1]) break;
+  } else {
+    if ((e = cudaMemcpyAsync(&mb, maxbits, sizeof(mb), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(s)) != cudaSuccess)
+      return cuda_status(e, "registration");
+    if (bad_frames()) return set_error(GBN_ERR_INVALID, kBadFrames);
+    // the gradient reads dy and dx over whole supports, outside the bounding box
+    // times a zero mask: zero there
+    if ((e = cudaMemsetAsync(dy, 0, X * sizeof(float), s)) != cudaSuccess ||
+        (e = cudaMemsetAsync(dx, 0, 2 * X * sizeof(float), s)) != cudaSuccess)
+      return cuda_status(e, "registration setup");
+    const int gp = (L * L + kRegNT - 1) / kRegNT;
+    const int gw = (L * L * F + kRegNT - 1) / kRegNT;
+    const int gpc = kRegNT / g.dp;
+    const int gg = (2 * F * g.Cp * g.Cp + gpc - 1) / gpc;
+    // the unregistered frames: metric H[0]; dx at the starting mesh (optimizer.cpp: InitIT, Metric, CostReduction)
+    k_reg_warp<<<gw, kRegNT, 0, s>>>(a);
+    k_reg_metric<<<gp, kRegNT, 0, s>>>(a, 0, gu, prm->et, prm->eh);
+    ctx->launches += 2;
+    a.warp = 1;
+    a.smooth = g.sum_lambda != 0;
+    // chunks of iterations with one chunk of lookahead: while the GPU runs chunk
+    // c the host waits for chunk c-1's stop flag (copied to pinned memory behind
+    // it), so the queue never drains; after the stop, the chunk already queued
+    // returns at each kernel's entry
+    if ((rc = host_flags_ready(ctx)) != GBN_OK) return rc;
+    int chunk = 0;
+    for (int it = 1; it <= prm->nmax; ++chunk) {
+      for (int k = 0; k < kRegChunk && it <= prm->nmax; ++k, ++it) {
+        // plain launches: chained by programmatic dependent launch these small
+        // grids ran slower (6.3 against 5.1 ms per registration at 256^2 x 20)
+        if (g.dp == kSolveSup)
+          k_reg_grad<kSolveSup><<<gg, kRegNT, 0, s>>>(a);
+        else
+          k_reg_grad<0><<<gg, kRegNT, 0, s>>>(a);
+        k_reg_update<<<gu, kRegNT, 0, s>>>(a);
+        k_reg_warp<<<gw, kRegNT, 0, s>>>(a);
+        k_reg_metric<<<gp, kRegNT, 0, s>>>(a, it, gu, prm->et, prm->eh);
+        ctx->launches += 4;
+      }
+      if ((e = cudaMemcpyAsync(&ctx->host_flags[chunk & 1], &st->done, sizeof(int), cudaMemcpyDeviceToHost, s)) !=
+              cudaSuccess ||
+          (e = cudaEventRecord(ctx->ev_flag[chunk & 1], s)) != cudaSuccess)
+        return cuda_status(e, "registration");
+      if (chunk > 0) {
+        if ((e = cudaEventSynchronize(ctx->ev_flag[(chunk - 1) & 1])) != cudaSuccess) return cuda_status(e, "registration");
+        if (ctx->host_flags[(chunk - 1) & 1]) break;
+      }
     }
   }
+  RegState hs{};
   if ((e = cudaMemcpyAsync(&hs, st, sizeof(hs), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return cuda_status(e, "registration");
   std::vector<float> hH(size_t(prm->nmax) + 1, 0.f);
   if ((e = cudaMemcpyAsync(hH.data(), H, hH.size() * sizeof(float), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
       (e = cudaStreamSynchronize(s)) != cudaSuccess)
     return cuda_status(e, "registration");
+  if (solve && bad_frames()) return set_error(GBN_ERR_INVALID, kBadFrames);
+  if (hs.status == kStatusBarrier)
+    return set_error(GBN_ERR_CUDA, "registration: the CTAs of the descent did not all arrive at a barrier");
   if (h_H) std::memcpy(h_H, hH.data(), hH.size() * sizeof(float));
   if (stats) {
     stats->iterations = hs.it;
