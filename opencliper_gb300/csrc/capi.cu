@@ -141,8 +141,8 @@ int prof_collect(gbn_ctx* ctx) {
   return GBN_OK;
 }
 
-int ctx_scratch(gbn_ctx* ctx, size_t bytes, void** out, int user) {
-  ctx->scratch_user = user;
+int ctx_scratch(gbn_ctx* ctx, size_t bytes, void** out) {
+  ctx->simple_plan = gbn_ctx::SimplePlan{};
   if (bytes > ctx->scratch_bytes) {
     if (ctx->scratch) {
       cudaStreamSynchronize(ctx->stream);

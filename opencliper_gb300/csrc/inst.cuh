@@ -96,17 +96,53 @@ struct Launchers {
       launch_pdl(k_iter_pair<L, false>, dim3(ncg, cdiv(bm.n, ncg)), kPairNT, P::BYTES, s, tab, bm, it, int(grid.z));
     }
   }
-  static void fft_rows(const float2* in, float2* out, int nrows, int inv, float scale, const float2* tw, int grid,
-                       cudaStream_t s) {
-    k_fft_rows_dense<L><<<grid, kRowNT, 0, s>>>(in, out, nrows, inv, scale, tw);
+  static void fft_rows(const float2* in, float2* out, int nrows, int inv, float scale, const float2* tw,
+                       const uint8_t* mask, int C, int H, int grid, cudaStream_t s) {
+    if (mask)
+      k_fft_rows_dense<L, true><<<grid, kRowNT, 0, s>>>(in, out, nrows, inv, scale, tw, mask, C, H);
+    else
+      k_fft_rows_dense<L, false><<<grid, kRowNT, 0, s>>>(in, out, nrows, inv, scale, tw, mask, C, H);
   }
   static void fft_cols(const float2* in, float2* out, int W, int nimg, int inv, float scale, const float2* tw,
                        cudaStream_t s) {
     k_fft_cols_dense<L><<<dim3(W / kWB, nimg), kColNT, 0, s>>>(in, out, W, inv, scale, tw);
   }
+  static void enc_cols(const float2* x, const float2* S, float2* out, int W, int C, int F, const float2* tw,
+                       cudaStream_t s) {
+    k_enc_cols<L><<<dim3(W / kWB, cdiv(C, kEncCoils), F), kColNT, 0, s>>>(x, S, out, W, C, tw);
+  }
+  template <bool RSS>
+  static void adj_cols_of(const float2* T, const float2* S, float2* x, int W, int C, int F, float scale,
+                          const float2* tw, int cs, cudaStream_t s) {
+    static bool ok = false;
+    constexpr int bytes = AdjColsSmem<L>::BYTES;
+    allow_smem(k_adj_cols<L, RSS>, bytes, ok);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(W / kWB, cs, F);
+    cfg.blockDim = dim3(kColNT);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1;
+    at[0].val.clusterDim.y = unsigned(cs);
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    cudaLaunchKernelEx(&cfg, k_adj_cols<L, RSS>, T, S, x, W, C, scale, tw);
+  }
+  static void adj_cols(const float2* T, const float2* S, float2* x, int W, int C, int F, float scale,
+                       const float2* tw, int cs, cudaStream_t s) {
+    if (S)
+      adj_cols_of<false>(T, S, x, W, C, F, scale, tw, cs, s);
+    else
+      adj_cols_of<true>(T, S, x, W, C, F, scale, tw, cs, s);
+  }
   static SizeKernels entry() {
     static_assert(fft_size_ok(L), "unsupported transform length");
-    return SizeKernels{L, &fwd_cols, &rows, &inv_cols, &fft_rows, &fft_cols,
+    return SizeKernels{L, &fwd_cols, &rows, &inv_cols, &fft_rows, &fft_cols, &enc_cols, &adj_cols,
                        iter_cols_ok(L) ? &iter_cols : nullptr, &iter_finish, iter_pair_ok(L) ? pair_cols(L) : 0, RowCfg<L>::RPC, &rows_occupancy};
   }
 };

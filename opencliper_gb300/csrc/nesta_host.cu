@@ -195,19 +195,6 @@ __global__ void __launch_bounds__(512) k_rowscan(RowScan a) {
   }
 }
 
-// every row kept, in natural order (SimpleMRIRecon: fully sampled data)
-__global__ void k_rows_identity(int H, int F, int* __restrict__ rowmap, int* __restrict__ rowoff,
-                                int* __restrict__ rows_h, int* __restrict__ rows_f, int* __restrict__ row_full) {
-  const int n = H * F;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    rowmap[i] = i % H;
-    rows_h[i] = i % H;
-    rows_f[i] = i / H;
-    row_full[i] = 1;
-  }
-  for (int f = blockIdx.x * blockDim.x + threadIdx.x; f <= F; f += gridDim.x * blockDim.x) rowoff[f] = f * H;
-}
-
 // ---------------------------------------------------------------------------
 // Instance tables of a launch group.  k_store_args writes one entry from its
 // by-value parameter (no host buffer has to outlive the call); k_group_init
@@ -1112,112 +1099,6 @@ int nesta_run(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, float2*
   if (e != cudaSuccess) return cuda_status(e, "nesta launch");
   if (stats) return read_stats(P, s, stats);
   return GBN_OK;
-}
-
-// Adjoint-only pass (rows without residual, then columns without update) of
-// one instance with every row kept: SimpleMRIRecon.  `ws` provides the
-// intermediates and tables (simple_recon_bytes); no allocation happens here.
-size_t simple_recon_bytes(int W, int H, int F, int C) {
-  const size_t FH = size_t(F) * H, K = FH * C * W;
-  auto up = [](size_t v) { return (v + 255) / 256 * 256; };
-  return up(K * sizeof(float2)) + up((4 * FH + F + 1) * sizeof(int)) + up(sizeof(NestaDevState)) +
-         up(sizeof(FusedArgs)) + up(sizeof(ClassCtl));
-}
-
-int simple_recon_in(gbn_ctx* ctx, void* ws, const float2* y, const float2* S, float2* x, int W, int H, int F, int C,
-                    bool tables_valid) {
-  const SizeKernels* kh = find_size(H);
-  const SizeKernels* kw = find_size(W);
-  if (!kh || !kw) return set_error(GBN_ERR_UNSUPPORTED, "unsupported FFT length");
-  const size_t FH = size_t(F) * H, K = FH * C * W;
-  auto up = [](size_t v) { return (v + 255) / 256 * 256; };
-  unsigned char* b = static_cast<unsigned char*>(ws);
-  float2* T = reinterpret_cast<float2*>(b);
-  b += up(K * sizeof(float2));
-  int* rowmap = reinterpret_cast<int*>(b);
-  int* rows_h = rowmap + FH;
-  int* rows_f = rows_h + FH;
-  int* row_full = rows_f + FH;
-  int* rowoff = row_full + FH;
-  b += up((4 * FH + F + 1) * sizeof(int));
-  NestaDevState* st = reinterpret_cast<NestaDevState*>(b);
-  b += up(sizeof(NestaDevState));
-  FusedArgs* tab = reinterpret_cast<FusedArgs*>(b);
-  b += up(sizeof(FusedArgs));
-  ClassCtl* ctl = reinterpret_cast<ClassCtl*>(b);
-  cudaStream_t s = ctx->stream;
-  FusedArgs a;
-  memset(&a, 0, sizeof(a));
-  a.W = W;
-  a.H = H;
-  a.F = F;
-  a.C = C;
-  a.N = W * H;
-  a.y = y;
-  a.S = S;
-  a.rowmap = rowmap;
-  a.rowoff = rowoff;
-  a.rows_h = rows_h;
-  a.rows_f = rows_f;
-  a.row_full = row_full;
-  a.T = T;
-  a.xref = x;
-  a.st = st;
-  a.twH = ctx_twiddles(ctx, H);
-  a.twW = ctx_twiddles(ctx, W);
-  a.s_adj = 1.0f / float(W * H);  // clFFT BACKWARD scale
-  a.ntv = F * (W / kWB);
-  const long long steps = ((long long)FH * C + kw->rows_per_cta - 1) / kw->rows_per_cta;
-  const int g2 = row_grid(ctx, kw, false, steps, ctx->k2_ctas_per_sm);
-  const BatchMap bm = single_map(F, ctl);
-  // the tables persist in `ws`, and the row pass leaves its control block
-  // ready for the next launch
-  const int n_tables = tables_valid ? 0 : 3;
-  GBN_LAUNCH(ctx, GBN_PROF_SETUP, n_tables + 2, {
-    if (!tables_valid) {
-      k_rows_identity<<<int(std::min<size_t>((FH + 255) / 256, 1024)), 256, 0, s>>>(H, F, rowmap, rowoff, rows_h,
-                                                                                    rows_f, row_full);
-      k_store_args<<<1, 1, 0, s>>>(tab, a);
-      k_group_init<<<1, 64, 0, s>>>(tab, 1, kw->rows_per_cta, ctl);
-    }
-    kw->rows(tab, bm, 0, false, g2, s);
-    kh->inv_cols(tab, bm, 0, false, dim3(W / kWB, 2, F), s);
-  });
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_status(e, "simple recon launch");
-  return GBN_OK;
-}
-
-// SimpleMRIRecon: x = sum_c conj(S_c) ifft2(y_c) through the adjoint row and
-// column passes with every row kept, working memory from the context scratch.
-int simple_recon(gbn_ctx* ctx, const float2* y, const float2* S, float2* x, int W, int H, int F, int C) {
-  if (!find_size(H) || !find_size(W)) return set_error(GBN_ERR_UNSUPPORTED, "unsupported FFT length");
-  void* scr = nullptr;
-  const bool mine = ctx->scratch_user == kScratchSimple;
-  const int rc = ctx_scratch(ctx, simple_recon_bytes(W, H, F, C), &scr, kScratchSimple);
-  if (rc != GBN_OK) {
-    // a failed allocation freed the old scratch: a later one at the same
-    // address holds no tables
-    ctx->simple_key = gbn_ctx::SimpleKey{};
-    return rc;
-  }
-  gbn_ctx::SimpleKey& k = ctx->simple_key;
-  const bool same = mine && k.y == y && k.S == S && k.x == x && k.ws == scr && k.W == W && k.H == H && k.F == F &&
-                    k.C == C;
-  const int rc2 = simple_recon_in(ctx, scr, y, S, x, W, H, F, C, same);
-  if (rc2 == GBN_OK) {
-    k.y = y;
-    k.S = S;
-    k.x = x;
-    k.ws = scr;
-    k.W = W;
-    k.H = H;
-    k.F = F;
-    k.C = C;
-  } else {
-    k = gbn_ctx::SimpleKey{};
-  }
-  return rc2;
 }
 
 }  // namespace gbn

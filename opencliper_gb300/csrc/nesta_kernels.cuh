@@ -894,17 +894,27 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT)
 }
 
 // ===========================================================================
-// Dense FFT passes (the FFT process on full KData/XData buffers):
-// rows along W, then columns along H.  Forward code only; the backward
+// Dense FFT passes (the FFT process on full KData/XData buffers, and E, E^H,
+// SimpleMRIRecon and SimpleMRIReconSOS on them).  Forward code only; the backward
 // transform is conj(forward(conj(x))).  In place is allowed (out == in).
+// Bound by memory (L2 or DRAM): the element-wise processes around the transforms
+// are folded into their loads and stores, so that E is one pass out of the image
+// and one over k-space, and E^H one over k-space and one into the image.
 // ===========================================================================
-template <int W>
+// rows along W, RPC of them per CTA and step; launched with one step per CTA (8 CTAs
+// per SM that loop: 51 against 44 us at 384 x 384 x 120 images), and the loop stays
+// for its schedule: without it the compiler takes 48 registers instead of 52, and E
+// at 256 x 256 x 240 images takes 225 instead of 187 us.  MASKED: samples where the pixel mask [F][H][W] is
+// 0 become 0 (rows in KData order (f, c, h))
+template <int W, bool MASKED>
 __global__ void __launch_bounds__(kRowNT) k_fft_rows_dense(const float2* in, float2* out, int nrows, int inv,
-                                                           float scale, const float2* twW) {
+                                                           float scale, const float2* twW,
+                                                           const uint8_t* __restrict__ mask, int C, int H) {
   using R = RowCfg<W>;
   constexpr int A = R::A, B = R::B, RPC = R::RPC;
   __shared__ float2 ex1[RPC * R::RS1];
   __shared__ float2 tw[W];
+  grid_dep_release();  // a successor waits for this grid before it reads `out`
   const int t = threadIdx.x;
   for (int i = t; i < W; i += kRowNT) tw[i] = twW[i];
   __syncthreads();
@@ -928,22 +938,39 @@ __global__ void __launch_bounds__(kRowNT) k_fft_rows_dense(const float2* in, flo
     for (int i = t; i < RPC * A; i += kRowNT) {
       const int r = i / A, k1 = i % A, q = base + r;
       if (q >= nrows) continue;
+      const uint8_t* mrow = nullptr;
+      if constexpr (MASKED) mrow = mask + (size_t(q / (C * H)) * H + q % H) * W;
+      uint8_t m[B];
+      if constexpr (MASKED) {
+#pragma unroll
+        for (int k2 = 0; k2 < B; ++k2) m[k2] = __ldg(mrow + k1 + A * k2);
+      }
       float2 v[B];
 #pragma unroll
       for (int s = 0; s < B; ++s) v[s] = ex1[r * R::RS1 + k1 * R::S1 + s];
       dft<B>(v);
       float2* __restrict__ dst = out + size_t(q) * W;
 #pragma unroll
-      for (int k2 = 0; k2 < B; ++k2) dst[k1 + A * k2] = make_float2(v[k2].x * scale, sg * v[k2].y * scale);
+      for (int k2 = 0; k2 < B; ++k2) {
+        float2 o = make_float2(v[k2].x * scale, sg * v[k2].y * scale);
+        if constexpr (MASKED) {
+          if (m[k2] == 0) o = make_float2(0.f, 0.f);
+        }
+        dst[k1 + A * k2] = o;
+      }
     }
     __syncthreads();
   }
 }
 
-// grid = (W/kWB, nimg)
+// columns along H of every image, grid (W/kWB, images).  Five CTAs per SM: with more
+// registers the compiler's fewer CTAs, and with fewer registers the loads in two
+// batches, are slower (384 x 384 x 120 images, 283 MB: 69 us without the bound, 50
+// with five CTAs, 53 with six, 70 with seven); first factors past 24 need more.
+constexpr int cols_dense_blocks(int H) { return split_a(H) <= 24 && split_b(H) <= 24 ? 5 : 1; }
 template <int H>
-__global__ void __launch_bounds__(kColNT) k_fft_cols_dense(const float2* in, float2* out, int W, int inv, float scale,
-                                                           const float2* twH) {
+__global__ void __launch_bounds__(kColNT, cols_dense_blocks(H))
+    k_fft_cols_dense(const float2* in, float2* out, int W, int inv, float scale, const float2* twH) {
   constexpr int A = Split<H>::A, B = Split<H>::B;
   constexpr int KS = col_ks(B);
   constexpr int N1 = kWB * B, N2 = kWB * A;
@@ -951,7 +978,8 @@ __global__ void __launch_bounds__(kColNT) k_fft_cols_dense(const float2* in, flo
   __shared__ float2 tw[H];
   const int t = threadIdx.x;
   const int w0 = blockIdx.x * kWB;
-  const size_t off = size_t(blockIdx.y) * H * W;
+  const size_t off = size_t(blockIdx.y) * H * W + w0;
+  const float2* const src = in + off;
   for (int i = t; i < H; i += kColNT) tw[i] = twH[i];
   __syncthreads();
   const float sg = inv ? -1.f : 1.f;
@@ -959,15 +987,15 @@ __global__ void __launch_bounds__(kColNT) k_fft_cols_dense(const float2* in, flo
     const int w = i % kWB, s = i / kWB;
     float2 v[A];
 #pragma unroll
-    for (int n1 = 0; n1 < A; ++n1) {
-      const float2 e = in[off + size_t(B * n1 + s) * W + w0 + w];
-      v[n1] = make_float2(e.x, sg * e.y);
-    }
+    for (int n1 = 0; n1 < A; ++n1) v[n1] = src[size_t(B * n1 + s) * W + w];
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) v[n1].y *= sg;
     dft<A>(v);
 #pragma unroll
     for (int k1 = 0; k1 < A; ++k1) ex[k1 * KS + s * kWB + w] = (k1 == 0) ? v[k1] : cmul(v[k1], tw[k1 * B + s]);
   }
   __syncthreads();
+  float2* const dst = out + off;
   for (int i = t; i < N2; i += kColNT) {
     const int w = i % kWB, k1 = i / kWB;
     float2 v[B];
@@ -976,7 +1004,209 @@ __global__ void __launch_bounds__(kColNT) k_fft_cols_dense(const float2* in, flo
     dft<B>(v);
 #pragma unroll
     for (int k2 = 0; k2 < B; ++k2)
-      out[off + size_t(k1 + A * k2) * W + w0 + w] = make_float2(v[k2].x * scale, sg * v[k2].y * scale);
+      dst[size_t(k1 + A * k2) * W + w] = make_float2(v[k2].x * scale, sg * v[k2].y * scale);
+  }
+}
+
+// Forward columns of S_c x_f (x [F][H][W], S [C][H][W]) into out [F][C][H][W]: grid
+// (W/kWB, coil groups, frames), the coils of a group from one load of x_f, the next
+// one's S loaded while one is transformed (a coil per CTA: 48.5 against 41.2 us at
+// 256 x 256 x 20 x 12)
+constexpr int kEncCoils = 4;
+template <int H>
+__global__ void __launch_bounds__(kColNT) k_enc_cols(const float2* in, const float2* __restrict__ S, float2* out, int W,
+                                                     int C, const float2* twH) {
+  constexpr int A = Split<H>::A, B = Split<H>::B;
+  constexpr int KS = col_ks(B);
+  constexpr int N1 = kWB * B, N2 = kWB * A, NI1 = cdiv(N1, kColNT);
+  __shared__ float2 ex[A * KS];
+  __shared__ float2 tw[H];
+  const int t = threadIdx.x;
+  const int w0 = blockIdx.x * kWB;
+  const int c0 = blockIdx.y * kEncCoils, c1 = min(C, c0 + kEncCoils);
+  const size_t N = size_t(H) * W;
+  for (int i = t; i < H; i += kColNT) tw[i] = twH[i];
+  float2 xv[NI1][A], sv[NI1][A];
+  auto fetch = [&](float2 (*v)[A], const float2* src) {
+#pragma unroll
+    for (int ii = 0; ii < NI1; ++ii) {
+      const int i = t + ii * kColNT;
+      if (N1 % kColNT == 0 || i < N1) {
+#pragma unroll
+        for (int n1 = 0; n1 < A; ++n1) v[ii][n1] = src[size_t(B * n1 + i / kWB) * W + i % kWB];
+      }
+    }
+  };
+  fetch(xv, in + size_t(blockIdx.z) * N + w0);
+  fetch(sv, S + size_t(c0) * N + w0);
+  __syncthreads();
+  for (int c = c0; c < c1; ++c) {
+#pragma unroll
+    for (int ii = 0; ii < NI1; ++ii) {
+      const int i = t + ii * kColNT;
+      if (N1 % kColNT == 0 || i < N1) {
+        const int w = i % kWB, s = i / kWB;
+        float2 v[A];
+#pragma unroll
+        for (int n1 = 0; n1 < A; ++n1) v[n1] = cmul(xv[ii][n1], sv[ii][n1]);
+        dft<A>(v);
+#pragma unroll
+        for (int k1 = 0; k1 < A; ++k1) ex[k1 * KS + s * kWB + w] = (k1 == 0) ? v[k1] : cmul(v[k1], tw[k1 * B + s]);
+      }
+    }
+    if (c + 1 < c1) fetch(sv, S + size_t(c + 1) * N + w0);
+    __syncthreads();
+    float2* const dst = out + (size_t(blockIdx.z) * C + c) * N + w0;
+    for (int i = t; i < N2; i += kColNT) {
+      const int w = i % kWB, k1 = i / kWB;
+      float2 v[B];
+#pragma unroll
+      for (int s = 0; s < B; ++s) v[s] = ex[k1 * KS + s * kWB + w];
+      dft<B>(v);
+#pragma unroll
+      for (int k2 = 0; k2 < B; ++k2)
+        dst[size_t(k1 + A * k2) * W + w] = v[k2];
+    }
+    __syncthreads();
+  }
+}
+
+// Backward columns along H of the coil images T [F][C][H][W] combined over the
+// coils into x [F][H][W]: scale * sum_c conj(S_c) IDFT_H(T_c), or (RSS) the root of
+// the sum of |scale IDFT_H(T_c)|^2.  grid (W/kWB, CS, frames) in clusters of CS
+// CTAs along y, which share a tile's coils (coil c on CTA c % CS) and add up
+// through distributed shared memory, in CTA order; each finishes part of the
+// tile's rows.  The next coil's values are loaded while this one is transformed.
+template <int H>
+struct AdjColsSmem {
+  static constexpr int A = Split<H>::A, B = Split<H>::B, KS = col_ks(A);
+  static constexpr int NI2 = cdiv(kWB * B, kColNT);
+  static constexpr int EXN = B * KS > NI2 * A * kColNT ? B * KS : NI2 * A * kColNT;  // exchange, then accumulators
+  static constexpr int BYTES = EXN * 8;
+};
+// (at 168 registers and three CTAs per SM, twiddles in shared memory, 60 against 51
+// us at 256 x 256 x 20 x 12)
+template <int H, bool RSS>
+__global__ void __launch_bounds__(kColNT) k_adj_cols(const float2* T, const float2* __restrict__ S,
+                                                     float2* __restrict__ x, int W, int C, float scale,
+                                                     const float2* __restrict__ twH) {
+  using L = AdjColsSmem<H>;
+  constexpr int A = L::A, B = L::B, KS = L::KS;
+  constexpr int N1 = kWB * A, N2 = kWB * B;
+  constexpr int NI1 = cdiv(N1, kColNT), NI2 = L::NI2;
+  extern __shared__ float4 smem4[];
+  float2* const ex = reinterpret_cast<float2*>(smem4);
+  const int t = threadIdx.x, w0 = blockIdx.x * kWB, f = blockIdx.z;
+  const int CS = gridDim.y, rank = blockIdx.y;  // the cluster covers the grid's y
+  const size_t N = size_t(H) * W;
+  float2 twr[NI1][B];
+#pragma unroll
+  for (int ii = 0; ii < NI1; ++ii) {
+    const int i = t + ii * kColNT, s = i < N1 ? i / kWB : 0;
+#pragma unroll
+    for (int k1p = 0; k1p < B; ++k1p) twr[ii][k1p] = __ldg(twH + H + k1p * A + s);
+  }
+  grid_dep_wait();  // T comes from the row pass
+  float2 pf[NI1][B];
+  auto fetch = [&](int c) {
+    const float2* const src = T + (size_t(f) * C + c) * N + w0;
+#pragma unroll
+    for (int ii = 0; ii < NI1; ++ii) {
+      const int i = t + ii * kColNT;
+      if (N1 % kColNT == 0 || i < N1) {
+        const int w = i % kWB, s = i / kWB;
+#pragma unroll
+        for (int n1 = 0; n1 < B; ++n1) pf[ii][n1] = src[size_t(A * n1 + s) * W + w];
+      }
+    }
+  };
+  float2 acc[NI2][A];
+#pragma unroll
+  for (int ii = 0; ii < NI2; ++ii)
+#pragma unroll
+    for (int k2 = 0; k2 < A; ++k2) acc[ii][k2] = make_float2(0.f, 0.f);
+  if (rank < C) fetch(rank);
+  for (int c = rank; c < C; c += CS) {
+#pragma unroll
+    for (int ii = 0; ii < NI1; ++ii) {
+      const int i = t + ii * kColNT;
+      if (N1 % kColNT == 0 || i < N1) {
+        const int w = i % kWB, s = i / kWB;
+        float2 v[B];
+#pragma unroll
+        for (int n1 = 0; n1 < B; ++n1) v[n1] = conjf2(pf[ii][n1]);
+        dft<B>(v);
+#pragma unroll
+        for (int k1p = 0; k1p < B; ++k1p)
+          ex[k1p * KS + s * kWB + w] = (k1p == 0) ? v[k1p] : cmul(v[k1p], twr[ii][k1p]);
+      }
+    }
+    if (c + CS < C) fetch(c + CS);
+    __syncthreads();
+#pragma unroll
+    for (int ii = 0; ii < NI2; ++ii) {
+      const int i = t + ii * kColNT;
+      if (N2 % kColNT == 0 || i < N2) {
+        const int w = i % kWB, k1p = i / kWB;
+        float2 sv[RSS ? 1 : A];
+        if constexpr (!RSS) {
+          const float2* const sc = S + size_t(c) * N + w0 + w;
+#pragma unroll
+          for (int k2 = 0; k2 < A; ++k2) sv[k2] = __ldg(sc + size_t(k1p + B * k2) * W);
+        }
+        float2 v[A];
+#pragma unroll
+        for (int s = 0; s < A; ++s) v[s] = ex[k1p * KS + s * kWB + w];
+        dft<A>(v);
+#pragma unroll
+        for (int k2 = 0; k2 < A; ++k2) {
+          if constexpr (RSS) {
+            const float2 e = cscale(v[k2], scale);
+            acc[ii][k2].x = __fadd_rn(acc[ii][k2].x, __fadd_rn(__fmul_rn(e.x, e.x), __fmul_rn(e.y, e.y)));
+          } else {  // conj(v) * conj(S) == conj(v * S)
+            const float2 p = cmul(v[k2], sv[k2]);
+            acc[ii][k2].x += p.x;
+            acc[ii][k2].y -= p.y;
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  int kb = 0, ke = A;  // the rows k2 this CTA finishes
+  if (CS > 1) {
+    namespace cgr = cooperative_groups;
+    cgr::cluster_group cluster = cgr::this_cluster();
+#pragma unroll
+    for (int ii = 0; ii < NI2; ++ii)
+#pragma unroll
+      for (int k2 = 0; k2 < A; ++k2) ex[(ii * A + k2) * kColNT + t] = acc[ii][k2];
+    cluster.sync();
+    kb = rank * A / CS;
+    ke = (rank + 1) * A / CS;
+#pragma unroll
+    for (int ii = 0; ii < NI2; ++ii)
+#pragma unroll
+      for (int k2 = 0; k2 < A; ++k2)
+        if (k2 >= kb && k2 < ke) {
+          float2 sum = make_float2(0.f, 0.f);
+          for (int g = 0; g < CS; ++g)
+            sum = cadd(sum, cluster.map_shared_rank(ex, g)[(ii * A + k2) * kColNT + t]);
+          acc[ii][k2] = sum;
+        }
+    cluster.sync();  // the others have read this CTA's accumulators
+  }
+#pragma unroll
+  for (int ii = 0; ii < NI2; ++ii) {
+    const int i = t + ii * kColNT;
+    if (N2 % kColNT == 0 || i < N2) {
+      const int w = i % kWB, k1p = i / kWB;
+#pragma unroll
+      for (int k2 = 0; k2 < A; ++k2)
+        if (k2 >= kb && k2 < ke)
+          x[size_t(f) * N + size_t(k1p + B * k2) * W + w0 + w] =
+              RSS ? make_float2(sqrtf(acc[ii][k2].x), 0.f) : cscale(acc[ii][k2], scale);
+    }
   }
 }
 

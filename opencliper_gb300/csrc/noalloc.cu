@@ -7,13 +7,11 @@
 // forbids allocation after start-up.  gbn_simple_recon_static serves them: the
 // caller passes only the input k-space, the sensitivity maps and the output
 // image, and the working memory comes from a fixed array compiled into the
-// library (kStaticScratchBytes, about 8.2 MiB on every device that loads the
+// library (kStaticScratchBytes, 8 MiB on every device that loads the
 // library, held until the process exits).
 //
-// The scratch holds the row-pass intermediates (F*H*C*W complex values), the
-// row tables, the one-entry instance table and the row pass's control block.
-// Every call reuses it: kernels of the call rewrite the tables and reset the
-// control block before anything reads them.  Calls whose work overlaps on the
+// The scratch holds the row-pass intermediates (F*H*C*W complex values), which
+// every call rewrites before it reads them.  Calls whose work overlaps on the
 // GPU (different streams, or several host threads) share the one array and
 // race; serialise them.  The array's device address is resolved on the first
 // call on each device and kept for the life of the process, so the entry point
@@ -30,22 +28,14 @@
 namespace gbn {
 
 size_t simple_recon_bytes(int W, int H, int F, int C);
-int simple_recon_in(gbn_ctx* ctx, void* ws, const float2* y, const float2* S, float2* x, int W, int H, int F, int C,
-                    bool tables_valid);
+int simple_recon_in(gbn_ctx* ctx, void* ws, const float2* y, const float2* S, float2* x, int W, int H, int F, int C);
 
 namespace {
 
 // limits of the static scratch
 constexpr size_t kStaticMaxT = size_t(1) << 20;  // complex elements of the intermediates: F*H*C*W
 constexpr size_t kStaticMaxRows = 8192;          // F*H
-constexpr size_t kStaticTBytes = kStaticMaxT * sizeof(float2);
-constexpr size_t kStaticIntBytes = ((5 * kStaticMaxRows + 1) * sizeof(int) + 255) / 256 * 256;
-// state block, instance table and control block, each rounded to 256 bytes
-constexpr size_t kStaticSmallBytes = 4096;
-static_assert(((sizeof(NestaDevState) + 255) / 256 + (sizeof(FusedArgs) + 255) / 256 + (sizeof(ClassCtl) + 255) / 256) *
-                      256 <= kStaticSmallBytes,
-              "static scratch tail too small");
-constexpr size_t kStaticScratchBytes = kStaticTBytes + kStaticIntBytes + kStaticSmallBytes;
+constexpr size_t kStaticScratchBytes = kStaticMaxT * sizeof(float2);
 
 __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
@@ -80,7 +70,7 @@ int simple_recon_static(gbn_ctx* ctx, const float2* y, const float2* S, float2* 
   if (rc != GBN_OK) return rc;
   if (simple_recon_bytes(W, H, F, C) > kStaticScratchBytes)
     return set_error(GBN_ERR_UNSUPPORTED, "gbn_simple_recon_static: problem exceeds the static scratch");
-  return simple_recon_in(ctx, base, y, S, x, W, H, F, C, false);  // the array is shared between contexts
+  return simple_recon_in(ctx, base, y, S, x, W, H, F, C);
 }
 
 }  // namespace gbn

@@ -97,10 +97,6 @@ __global__ void k_abs(const float2* in, float2* out, size_t n, int squared) {
   }
 }
 
-__global__ void k_scale(float2* data, size_t n, float s) {
-  GRID_STRIDE(i, n) data[i] = cscale(data[i], s);
-}
-
 // ---------------------------------------------------------------------------
 int op_ttv(gbn_ctx* ctx, int dir, const float2* in, float2* out, int W, int H, int F) {
   if (in == out) return set_error(GBN_ERR_INVALID, "TemporalTV needs distinct input and output buffers");
@@ -173,22 +169,19 @@ int op_rss(gbn_ctx* ctx, const float2* k, float2* out, int W, int H, int F, int 
   return cuda_status(cudaGetLastError(), "rss");
 }
 
-int op_fft2(gbn_ctx* ctx, int direction, const float2* in, float2* out, int W, int H, int batch);
-
-// SimpleMRIReconSOS: backward FFT of every coil image into the context scratch
-// (the input stays untouched), then the root sum of squares
-int simple_recon_sos(gbn_ctx* ctx, const float2* y, float2* x, int W, int H, int F, int C) {
-  void* scr = nullptr;
-  int rc = ctx_scratch(ctx, size_t(W) * H * F * C * sizeof(float2), &scr);
-  if (rc != GBN_OK) return rc;
-  float2* t = static_cast<float2*>(scr);
-  if ((rc = op_fft2(ctx, GBN_FFT_BACKWARD, y, t, W, H, F * C)) != GBN_OK) return rc;
-  return op_rss(ctx, t, x, W, H, F, C);
-}
-
 int op_abs(gbn_ctx* ctx, const float2* in, float2* out, size_t n, int squared) {
   k_abs<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(in, out, n, squared);
   return cuda_status(cudaGetLastError(), "abs");
+}
+
+static int rows_pass(gbn_ctx* ctx, const float2* in, float2* out, int W, int H, long long nrows, int inv, float scale,
+                     const uint8_t* mask, int C) {
+  if (nrows > 0x7fffffff) return set_error(GBN_ERR_UNSUPPORTED, "too many rows for one transform");
+  const SizeKernels* kw = find_size(W);
+  const int g = int((nrows + kw->rows_per_cta - 1) / kw->rows_per_cta);
+  kw->fft_rows(in, out, int(nrows), inv, scale, ctx_twiddles(ctx, W), mask, C, H, g, ctx->stream);
+  ctx->launches += 1;
+  return GBN_OK;
 }
 
 // 2-D FFT of `batch` W x H images: rows along W, then columns along H.
@@ -199,40 +192,94 @@ int op_fft2(gbn_ctx* ctx, int direction, const float2* in, float2* out, int W, i
   if (direction != GBN_FFT_FORWARD && direction != GBN_FFT_BACKWARD)
     return set_error(GBN_ERR_INVALID, "FFT direction must be FORWARD or BACKWARD");
   const int inv = direction == GBN_FFT_BACKWARD;
-  const long long nrows = (long long)batch * H;
-  const int g = int(std::max<long long>(1, std::min<long long>((nrows + kw->rows_per_cta - 1) / kw->rows_per_cta,
-                                                                (long long)ctx->nsm * 8)));
-  kw->fft_rows(in, out, int(nrows), inv, 1.0f, ctx_twiddles(ctx, W), g, ctx->stream);
   const float scale = inv ? 1.0f / float(W * H) : 1.0f;
+  // (one pass after the other over everything: in chunks whose intermediate stays
+  // in L2 the launches' ends cost more than that saves: 384 x 384 x 120 images 247
+  // against 230 us there and back)
+  const int rc = rows_pass(ctx, in, out, W, H, (long long)batch * H, inv, 1.0f, nullptr, 1);
+  if (rc != GBN_OK) return rc;
   kh->fft_cols(out, out, W, batch, inv, scale, ctx_twiddles(ctx, H), ctx->stream);
+  ctx->launches += 1;
   return cuda_status(cudaGetLastError(), "fft2");
 }
 
-// operatorA + 1/sqrt(N): k = mask * FFT2(S x) / sqrt(N)
+// operatorA + 1/sqrt(N): k = mask * FFT2(S x) / sqrt(N): the columns of S_c x_f, then
+// the rows with mask and scale
 int op_encode(gbn_ctx* ctx, const float2* x, const float2* S, const uint8_t* mask, float2* k, int W, int H, int F,
               int C) {
-  int rc;
-  if ((rc = op_sensmul(ctx, 0, x, 0, S, k, W, H, F, C)) != GBN_OK) return rc;
-  if ((rc = op_fft2(ctx, GBN_FFT_FORWARD, k, k, W, H, F * C)) != GBN_OK) return rc;
-  if ((rc = op_mask(ctx, k, mask, W, H, F, C)) != GBN_OK) return rc;
-  const size_t n = size_t(W) * H * F * C;
-  k_scale<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(k, n, float(1.0 / std::sqrt(double(unsigned(W * H)))));
+  const SizeKernels* kh = find_size(H);
+  if (!kh || !find_size(W)) return set_error(GBN_ERR_UNSUPPORTED, "unsupported FFT length");
+  if (x == k && C > 1) return set_error(GBN_ERR_INVALID, "XData input cannot alias the KData output");
+  const float scale = float(1.0 / std::sqrt(double(unsigned(W * H))));
+  kh->enc_cols(x, S, k, W, C, F, ctx_twiddles(ctx, H), ctx->stream);
+  ctx->launches += 1;
+  const int rc = rows_pass(ctx, k, k, W, H, (long long)F * C * H, 0, scale, mask, C);
+  if (rc != GBN_OK) return rc;
   return cuda_status(cudaGetLastError(), "encode");
+}
+
+// Backward rows into `scratch`, then backward columns combined over the coils: E^H
+// and SimpleMRIRecon (S given), or SimpleMRIReconSOS.
+size_t simple_recon_bytes(int W, int H, int F, int C) { return size_t(F) * C * W * H * sizeof(float2); }
+static int adjoint_in(gbn_ctx* ctx, float2* scratch, const float2* k, const float2* S, float2* x, int W, int H, int F,
+                      int C, float scale, const float2* twH) {
+  const int rc = rows_pass(ctx, k, scratch, W, H, (long long)F * C * H, 1, 1.0f, nullptr, C);
+  if (rc != GBN_OK) return rc;
+  // CTAs that share a tile's coils: until there are two per SM (six: 192 x 160 x 20 x
+  // 12 coils 44 against 39 us)
+  int cs = 1;
+  while (cs < 8 && 2 * cs <= C && (long long)(W / kWB) * F * cs < 2LL * ctx->nsm) cs *= 2;
+  find_size(H)->adj_cols(scratch, S, x, W, C, F, scale, twH, cs, ctx->stream);
+  ctx->launches += 1;
+  return cuda_status(cudaGetLastError(), "adjoint");
+}
+static int adjoint(gbn_ctx* ctx, const float2* k, const float2* S, float2* x, int W, int H, int F, int C, float scale) {
+  if (!find_size(H) || !find_size(W)) return set_error(GBN_ERR_UNSUPPORTED, "unsupported FFT length");
+  void* scr = nullptr;
+  const int rc = ctx_scratch(ctx, simple_recon_bytes(W, H, F, C), &scr);
+  if (rc != GBN_OK) return rc;
+  return adjoint_in(ctx, static_cast<float2*>(scr), k, S, x, W, H, F, C, scale, ctx_twiddles(ctx, H));
 }
 
 // sqrt(N) pre-scale + operatorAt: x = sum_c conj(S_c) IFFT2(sqrt(N) k_c)
 int op_encode_adjoint(gbn_ctx* ctx, const float2* k, const float2* S, float2* x, int W, int H, int F, int C) {
-  const size_t n = size_t(W) * H * F * C;
+  return adjoint(ctx, k, S, x, W, H, F, C, std::sqrt(float(W * H)) * (1.0f / float(W * H)));
+}
+
+__global__ void k_stage_twiddles(const float2* __restrict__ tw, float2* __restrict__ dst, int n) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = tw[i];
+}
+
+// SimpleMRIRecon: x = sum_c conj(S_c) ifft2(y_c).  Its column twiddles lie beside
+// the intermediates in the scratch, put there by the first call of a shape or
+// after another user of the scratch; further calls launch the two passes alone.
+int simple_recon(gbn_ctx* ctx, const float2* y, const float2* S, float2* x, int W, int H, int F, int C) {
+  if (!find_size(H) || !find_size(W)) return set_error(GBN_ERR_UNSUPPORTED, "unsupported FFT length");
+  gbn_ctx::SimplePlan& p = ctx->simple_plan;
+  const gbn_ctx::SimplePlan had = p;
   void* scr = nullptr;
-  int rc = ctx_scratch(ctx, n * sizeof(float2), &scr);
+  const size_t tb = 2 * size_t(H) * sizeof(float2);
+  const int rc = ctx_scratch(ctx, tb + simple_recon_bytes(W, H, F, C), &scr);  // forgets the plan
   if (rc != GBN_OK) return rc;
-  float2* aux = static_cast<float2*>(scr);
-  cudaError_t e = cudaMemcpyAsync(aux, k, n * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream);
-  if (e != cudaSuccess) return cuda_status(e, "encode_adjoint copy");
-  k_scale<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(aux, n, std::sqrt(float(W * H)));
-  if ((rc = op_fft2(ctx, GBN_FFT_BACKWARD, aux, aux, W, H, F * C)) != GBN_OK) return rc;
-  if ((rc = op_sensmul(ctx, 1, aux, 1, S, aux, W, H, F, C)) != GBN_OK) return rc;
-  return op_coilsum(ctx, aux, x, W, H, F, C);
+  float2* const tw = static_cast<float2*>(scr);
+  if (had.ws != scr || had.W != W || had.H != H || had.F != F || had.C != C) {
+    k_stage_twiddles<<<1, 256, 0, ctx->stream>>>(ctx_twiddles(ctx, H), tw, 2 * H);
+    ctx->launches += 1;
+  }
+  const int rc2 = adjoint_in(ctx, tw + 2 * size_t(H), y, S, x, W, H, F, C, 1.0f / float(W * H), tw);
+  if (rc2 == GBN_OK) p = gbn_ctx::SimplePlan{scr, W, H, F, C};
+  return rc2;
+}
+// the same in working memory of simple_recon_bytes that the caller has
+int simple_recon_in(gbn_ctx* ctx, void* ws, const float2* y, const float2* S, float2* x, int W, int H, int F, int C) {
+  if (!find_size(H) || !find_size(W)) return set_error(GBN_ERR_UNSUPPORTED, "unsupported FFT length");
+  return adjoint_in(ctx, static_cast<float2*>(ws), y, S, x, W, H, F, C, 1.0f / float(W * H), ctx_twiddles(ctx, H));
+}
+
+// SimpleMRIReconSOS: backward FFT of every coil image (the input stays
+// untouched), then the root sum of squares
+int simple_recon_sos(gbn_ctx* ctx, const float2* y, float2* x, int W, int H, int F, int C) {
+  return adjoint(ctx, y, nullptr, x, W, H, F, C, 1.0f / float(W * H));
 }
 
 }  // namespace gbn

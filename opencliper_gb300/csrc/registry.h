@@ -17,11 +17,18 @@ struct SizeKernels {
   void (*rows)(const FusedArgs* tab, const BatchMap& bm, int it, bool resid, int grid, cudaStream_t s);
   // adjoint column pass (k_inv_cols<L, update>), grid (W/8, 2, total frames) in clusters of 2
   void (*inv_cols)(const FusedArgs* tab, const BatchMap& bm, int it, bool update, dim3 grid, cudaStream_t s);
-  // dense FFT passes
-  void (*fft_rows)(const float2* in, float2* out, int nrows, int inv, float scale, const float2* tw, int grid,
-                   cudaStream_t s);
+  // dense FFT passes: rows (k_fft_rows_dense; mask [F][H][W] or nullptr, rows of C
+  // coils), columns of images (k_fft_cols_dense), of S_c x_f (k_enc_cols), and
+  // backward columns combined over the coils (k_adj_cols; S, or nullptr for the root
+  // sum of squares) in clusters of cs CTAs
+  void (*fft_rows)(const float2* in, float2* out, int nrows, int inv, float scale, const float2* tw,
+                   const uint8_t* mask, int C, int H, int grid, cudaStream_t s);
   void (*fft_cols)(const float2* in, float2* out, int W, int nimg, int inv, float scale, const float2* tw,
                    cudaStream_t s);
+  void (*enc_cols)(const float2* x, const float2* S, float2* out, int W, int C, int F, const float2* tw,
+                   cudaStream_t s);
+  void (*adj_cols)(const float2* T, const float2* S, float2* x, int W, int C, int F, float scale, const float2* tw,
+                   int cs, cudaStream_t s);
   // row-local inner iteration (k_iter_cols<L, motion>), grid (W/8, 2, total
   // frames) in clusters of 2; nullptr for lengths that run only the three-pass
   // iteration
