@@ -10,72 +10,134 @@
 
 namespace gbn {
 
+// Element-wise processes: bound by memory.  A thread takes two adjacent complex
+// values (an image has an even number: W is a multiple of 8) in one 16-byte access
+// where every buffer is 16-byte aligned, else in two of 8; frames and coils are grid
+// dimensions (strided over, past the grid's limit), so that no thread divides (with
+// 8-byte accesses and two 64-bit divisions a value, the eight processes of a gradient
+// at 224 x 200 x 16, 10 coils took 117 us; 88 now).
 namespace {
 inline int grid_for(gbn_ctx* ctx, size_t n, int nt = 256) {
   return int(std::max<size_t>(1, std::min<size_t>((n + nt - 1) / nt, size_t(ctx->nsm) * 16)));
 }
+// CTAs along the pixel pairs of an image, for y x z images
+inline dim3 image_grid(gbn_ctx* ctx, int N, int y, int z) {
+  y = std::min(y, 65535);
+  z = std::min(z, 65535);
+  const long long want = std::max<long long>(1, (long long)ctx->nsm * 64 / ((long long)y * z));
+  return dim3(unsigned(std::min<long long>((N / 2 + 255) / 256, want)), unsigned(y), unsigned(z));
+}
+inline bool aligned16(const void* a, const void* b = nullptr, const void* c = nullptr) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
+}
 #define GRID_STRIDE(i, n) \
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < (n); i += size_t(gridDim.x) * blockDim.x)
+#define GRID_PAIRS(i, N) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (N) / 2; i += gridDim.x * blockDim.x)
+
+template <bool V>
+__device__ __forceinline__ float4 ld_pair(const float2* p, size_t i) {
+  if constexpr (V) return reinterpret_cast<const float4*>(p)[i];
+  const float2 a = p[2 * i], b = p[2 * i + 1];
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+template <bool V>
+__device__ __forceinline__ void st_pair(float2* p, size_t i, float4 v) {
+  if constexpr (V) {
+    reinterpret_cast<float4*>(p)[i] = v;
+  } else {
+    p[2 * i] = make_float2(v.x, v.y);
+    p[2 * i + 1] = make_float2(v.z, v.w);
+  }
+}
 }  // namespace
 
-// temporalTV.cl:49-107.  One thread per (frame, pixel).
-__global__ void k_ttv(const float2* __restrict__ in, float2* __restrict__ out, int N, int F, int forward) {
-  const size_t n = size_t(N) * F;
-  GRID_STRIDE(i, n) {
-    const int f = int(i / N);
-    const size_t p = i - size_t(f) * N;
-    if (forward) {
-      out[i] = csub(in[i], in[size_t((f + F - 1) % F) * N + p]);
-    } else {
-      out[i] = csub(in[size_t((f + 1) % F) * N + p], in[i]);
+// temporalTV.cl:49-107, grid y: frames
+template <bool V>
+__global__ void __launch_bounds__(256) k_ttv(const float2* __restrict__ in, float2* __restrict__ out, int N, int F,
+                                             int forward) {
+  for (int f = blockIdx.y; f < F; f += gridDim.y) {
+    const float2* const a = in + size_t(forward ? f : (f + 1) % F) * N;
+    const float2* const b = in + size_t(forward ? (f + F - 1) % F : f) * N;
+    float2* const o = out + size_t(f) * N;
+#pragma unroll 2
+    GRID_PAIRS(i, N) {
+      const float4 u = ld_pair<V>(a, i), w = ld_pair<V>(b, i);
+      st_pair<V>(o, i, make_float4(u.x - w.x, u.y - w.y, u.z - w.z, u.w - w.w));
     }
   }
 }
 
-// vectorNormalization.cl:42-56: out = in / fmax(mu, length(in))
-__global__ void k_normalize(const float2* in, float2* out, size_t n, float mu) {
-  GRID_STRIDE(i, n) {
-    const float2 v = in[i];
-    const float m = fmaxf(mu, sqrtf(fmaf(v.x, v.x, v.y * v.y)));
-    out[i] = make_float2(v.x / m, v.y / m);
+// vectorNormalization.cl:42-56: out = in / fmax(mu, length(in)); pairs, an odd last value apart
+__device__ __forceinline__ float2 normalized(float2 v, float mu) {
+  const float m = fmaxf(mu, sqrtf(fmaf(v.x, v.x, v.y * v.y)));
+  return make_float2(v.x / m, v.y / m);
+}
+template <bool V>
+__global__ void __launch_bounds__(256) k_normalize(const float2* in, float2* out, size_t n, float mu) {
+  GRID_STRIDE(i, n / 2) {
+    const float4 v = ld_pair<V>(in, i);
+    const float2 a = normalized(make_float2(v.x, v.y), mu), b = normalized(make_float2(v.z, v.w), mu);
+    st_pair<V>(out, i, make_float4(a.x, a.y, b.x, b.y));
+  }
+  if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) out[n - 1] = normalized(in[n - 1], mu);
+}
+
+// complexElementProd.cl:42-76: out[f][c][p] = in[f][(c)][p] * (conj?)S[c][p]; grid y: coils, z: frames
+template <bool V>
+__global__ void __launch_bounds__(256) k_sensmul(const float2* in, int in_has_coils, const float2* __restrict__ S,
+                                                 float2* out, int N, int F, int C, int conj) {
+  const float sg = conj ? -1.f : 1.f;
+  for (int f = blockIdx.z; f < F; f += gridDim.z)
+    for (int c = blockIdx.y; c < C; c += gridDim.y) {
+      const size_t o = (size_t(f) * C + c) * N;
+      const float2* const a0 = in + (in_has_coils ? o : size_t(f) * N);
+      const float2* const s0 = S + size_t(c) * N;
+      float2* const o0 = out + o;
+      GRID_PAIRS(i, N) {
+        const float4 a = ld_pair<V>(a0, i);
+        float4 s = ld_pair<V>(s0, i);
+        s.y *= sg;
+        s.w *= sg;
+        st_pair<V>(o0, i, make_float4(a.x * s.x - a.y * s.y, a.x * s.y + a.y * s.x, a.z * s.z - a.w * s.w,
+                                      a.z * s.w + a.w * s.z));
+      }
+    }
+}
+
+// xImageSum.cl:42-61: out[f][p] = sum over coils in order; grid y: frames
+template <bool V>
+__global__ void __launch_bounds__(256) k_coilsum(const float2* __restrict__ in, float2* __restrict__ out, int N, int F,
+                                                 int C) {
+  for (int f = blockIdx.y; f < F; f += gridDim.y) {
+    const float2* const src = in + size_t(f) * C * N;
+    GRID_PAIRS(i, N) {
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int c = 0; c < C; ++c) {
+        const float4 v = ld_pair<V>(src + size_t(c) * N, i);
+        acc = make_float4(acc.x + v.x, acc.y + v.y, acc.z + v.z, acc.w + v.w);
+      }
+      st_pair<V>(out + size_t(f) * N, i, acc);
+    }
   }
 }
 
-// complexElementProd.cl:42-76: out[f][c][p] = in[f][(c)][p] * (conj?)S[c][p]
-__global__ void k_sensmul(const float2* in, int in_has_coils, const float2* __restrict__ S, float2* out, int N, int F,
-                          int C, int conj) {
-  const size_t n = size_t(N) * F * C;
-  GRID_STRIDE(i, n) {
-    const size_t p = i % N;
-    const size_t fc = i / N;
-    const int c = int(fc % C), f = int(fc / C);
-    const float2 a = in_has_coils ? in[i] : in[size_t(f) * N + p];
-    float2 s = S[size_t(c) * N + p];
-    if (conj) s.y = -s.y;
-    out[i] = make_float2(a.x * s.x - a.y * s.y, a.x * s.y + a.y * s.x);
-  }
-}
-
-// xImageSum.cl:42-61: out[f][p] = sum over coils in order
-__global__ void k_coilsum(const float2* __restrict__ in, float2* __restrict__ out, int N, int F, int C) {
-  const size_t n = size_t(N) * F;
-  GRID_STRIDE(i, n) {
-    const int f = int(i / N);
-    const size_t p = i - size_t(f) * N;
-    float2 acc = make_float2(0.f, 0.f);
-    for (int c = 0; c < C; ++c) acc = cadd(acc, in[(size_t(f) * C + c) * N + p]);
-    out[i] = acc;
-  }
-}
-
-// applyMask.cl:5-40
-__global__ void k_mask(float2* data, const uint8_t* __restrict__ mask, int N, int F, int C) {
-  const size_t n = size_t(N) * F * C;
-  GRID_STRIDE(i, n) {
-    const size_t p = i % N;
-    const int f = int(i / (size_t(N) * C));
-    if (mask[size_t(f) * N + p] == 0) data[i] = make_float2(0.f, 0.f);
-  }
+// applyMask.cl:5-40; grid y: coils, z: frames.  Only the masked samples are written.
+template <bool V>
+__global__ void __launch_bounds__(256) k_mask(float2* data, const uint8_t* __restrict__ mask, int N, int F, int C) {
+  for (int f = blockIdx.z; f < F; f += gridDim.z)
+    for (int c = blockIdx.y; c < C; c += gridDim.y) {
+      float2* const d = data + (size_t(f) * C + c) * N;
+      const uint8_t* const m = mask + size_t(f) * N;
+      GRID_PAIRS(i, N) {
+        const bool z0 = m[2 * i] == 0, z1 = m[2 * i + 1] == 0;
+        if (z0 && z1) {
+          st_pair<V>(d, i, make_float4(0.f, 0.f, 0.f, 0.f));
+        } else if (z0 || z1) {
+          d[2 * i + (z0 ? 0 : 1)] = make_float2(0.f, 0.f);
+        }
+      }
+    }
 }
 
 // SamplingMasksData.cpp:389-441: row value 1 -> 255, 0 -> 0, else error flag
@@ -100,13 +162,21 @@ __global__ void k_abs(const float2* in, float2* out, size_t n, int squared) {
 // ---------------------------------------------------------------------------
 int op_ttv(gbn_ctx* ctx, int dir, const float2* in, float2* out, int W, int H, int F) {
   if (in == out) return set_error(GBN_ERR_INVALID, "TemporalTV needs distinct input and output buffers");
-  const size_t n = size_t(W) * H * F;
-  k_ttv<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(in, out, W * H, F, dir == GBN_TTV_FORWARD);
+  const int N = W * H, fwd = dir == GBN_TTV_FORWARD;
+  const dim3 g = image_grid(ctx, N, F, 1);
+  if (aligned16(in, out))
+    k_ttv<true><<<g, 256, 0, ctx->stream>>>(in, out, N, F, fwd);
+  else
+    k_ttv<false><<<g, 256, 0, ctx->stream>>>(in, out, N, F, fwd);
   return cuda_status(cudaGetLastError(), "ttv");
 }
 
 int op_normalize(gbn_ctx* ctx, const float2* in, float2* out, size_t n, float mu) {
-  k_normalize<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(in, out, n, mu);
+  const int g = grid_for(ctx, (n + 1) / 2);
+  if (aligned16(in, out))
+    k_normalize<true><<<g, 256, 0, ctx->stream>>>(in, out, n, mu);
+  else
+    k_normalize<false><<<g, 256, 0, ctx->stream>>>(in, out, n, mu);
   return cuda_status(cudaGetLastError(), "normalize");
 }
 
@@ -114,20 +184,32 @@ int op_sensmul(gbn_ctx* ctx, int conj, const float2* in, int in_has_coils, const
                int F, int C) {
   if (!in_has_coils && in == out && C > 1)
     return set_error(GBN_ERR_INVALID, "XData input cannot alias the KData output");
-  const size_t n = size_t(W) * H * F * C;
-  k_sensmul<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(in, in_has_coils, S, out, W * H, F, C, conj);
+  const int N = W * H;
+  const dim3 g = image_grid(ctx, N, C, F);
+  if (aligned16(in, S, out))
+    k_sensmul<true><<<g, 256, 0, ctx->stream>>>(in, in_has_coils, S, out, N, F, C, conj);
+  else
+    k_sensmul<false><<<g, 256, 0, ctx->stream>>>(in, in_has_coils, S, out, N, F, C, conj);
   return cuda_status(cudaGetLastError(), "sensmul");
 }
 
 int op_coilsum(gbn_ctx* ctx, const float2* in, float2* out, int W, int H, int F, int C) {
-  const size_t n = size_t(W) * H * F;
-  k_coilsum<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(in, out, W * H, F, C);
+  const int N = W * H;
+  const dim3 g = image_grid(ctx, N, F, 1);
+  if (aligned16(in, out))
+    k_coilsum<true><<<g, 256, 0, ctx->stream>>>(in, out, N, F, C);
+  else
+    k_coilsum<false><<<g, 256, 0, ctx->stream>>>(in, out, N, F, C);
   return cuda_status(cudaGetLastError(), "coilsum");
 }
 
 int op_mask(gbn_ctx* ctx, float2* data, const uint8_t* mask, int W, int H, int F, int C) {
-  const size_t n = size_t(W) * H * F * C;
-  k_mask<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(data, mask, W * H, F, C);
+  const int N = W * H;
+  const dim3 g = image_grid(ctx, N, C, F);
+  if (aligned16(data))
+    k_mask<true><<<g, 256, 0, ctx->stream>>>(data, mask, N, F, C);
+  else
+    k_mask<false><<<g, 256, 0, ctx->stream>>>(data, mask, N, F, C);
   return cuda_status(cudaGetLastError(), "mask");
 }
 
@@ -148,23 +230,31 @@ int op_rowmask(gbn_ctx* ctx, const uint32_t* rm, uint8_t* pm, int W, int H, int 
 }
 
 // rss.cl:43-74 (RSoS): out[f][p] = (sqrt(sum_c |k[f][c][p]|^2), 0), the sum in
-// coil order in FP32
-__global__ void k_rss(const float2* __restrict__ k, float2* __restrict__ out, int N, int F, int C) {
-  const size_t n = size_t(N) * F;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-    const size_t f = i / N, p = i - f * N;
-    const float2* src = k + f * size_t(C) * N + p;
-    float acc = 0.f;
-    for (int c = 0; c < C; ++c) {
-      const float2 v = src[size_t(c) * N];
-      acc = __fadd_rn(acc, __fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y)));
+// coil order in FP32; grid y: frames
+template <bool V>
+__global__ void __launch_bounds__(256) k_rss(const float2* __restrict__ k, float2* __restrict__ out, int N, int F, int C) {
+  for (int f = blockIdx.y; f < F; f += gridDim.y) {
+    const float2* const src = k + size_t(f) * C * N;
+    GRID_PAIRS(i, N) {
+      float a = 0.f, b = 0.f;
+#pragma unroll 4
+      for (int c = 0; c < C; ++c) {
+        const float4 v = ld_pair<V>(src + size_t(c) * N, i);
+        a = __fadd_rn(a, __fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y)));
+        b = __fadd_rn(b, __fadd_rn(__fmul_rn(v.z, v.z), __fmul_rn(v.w, v.w)));
+      }
+      st_pair<V>(out + size_t(f) * N, i, make_float4(sqrtf(a), 0.f, sqrtf(b), 0.f));
     }
-    out[i] = make_float2(sqrtf(acc), 0.f);
   }
 }
 
 int op_rss(gbn_ctx* ctx, const float2* k, float2* out, int W, int H, int F, int C) {
-  k_rss<<<grid_for(ctx, size_t(W) * H * F), 256, 0, ctx->stream>>>(k, out, W * H, F, C);
+  const int N = W * H;
+  const dim3 g = image_grid(ctx, N, F, 1);
+  if (aligned16(k, out))
+    k_rss<true><<<g, 256, 0, ctx->stream>>>(k, out, N, F, C);
+  else
+    k_rss<false><<<g, 256, 0, ctx->stream>>>(k, out, N, F, C);
   ctx->launches += 1;
   return cuda_status(cudaGetLastError(), "rss");
 }
