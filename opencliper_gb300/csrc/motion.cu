@@ -30,8 +30,8 @@
 // takes M^T g; k_mc_tv and k_mc_adjoint then run on a side stream beside the
 // forward column pass, events ordering them after the previous iterate and
 // before the row and adjoint column passes.  The power method ||U|| cannot use the plain form's per-pixel
-// recurrence (M mixes pixels), so it runs myNormest's loop step for step on
-// the device (k_ne_*), the host reading the stop flag once per eight steps.
+// recurrence (M mixes pixels), so it runs myNormest's loop step for step, in one
+// cooperative launch (k_normest).
 //
 // Bounds: the reference reads the image at the interpolation corners without
 // checks; here a corner or target outside the image skips that pixel and sets
@@ -501,65 +501,56 @@ __global__ void __launch_bounds__(kNT) k_mc_tv(const float2* __restrict__ x0, co
 __global__ void k_fill(float2* __restrict__ v, size_t n, float2 value) {
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) v[i] = value;
 }
-// sum of |v|^2 and of |Re| + |Im|: FP32 within a thread's few elements and
-// a warp, FP64 across warps and blocks; per-block partials in fixed slots
-// (blocks stride over the vector in a fixed order, so the sums are
-// deterministic)
-__device__ __forceinline__ void warp_sums_to_block(float s2, float s1, double* sred2, double* sred1, double* part) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    s2 += __shfl_down_sync(0xffffffffu, s2, o);
-    s1 += __shfl_down_sync(0xffffffffu, s1, o);
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) {
-    sred2[wid] = double(s2);
-    sred1[wid] = double(s1);
-  }
-  __syncthreads();
-  if (threadIdx.x < 2) {
-    const double* r = threadIdx.x == 0 ? sred2 : sred1;
-    double t = 0.0;
-#pragma unroll
-    for (int w = 0; w < kNT / 32; ++w) t += r[w];
-    part[2 * blockIdx.x + threadIdx.x] = t;
-  }
-}
 int grid1(gbn_ctx* ctx, size_t n) { return int(std::min<size_t>((n + kNT - 1) / kNT, size_t(ctx->nsm) * 8)); }
 
-// ---- the power method on the device ------------------------------------------------
-// myNormest's loop (NestaUp.cpp:291-439) with U = tTV M and U^T = M^T tTVadj,
-// driven by a device-side state so that steps are enqueued in chunks without
-// host round trips.  Each step: U x (warp, tTV, partial sums of |Sx|^2 and
-// |Re|+|Im|), a scalar kernel (restart test, e), the drand48 restart (only when
-// U x is exactly zero), U^T Sx (tTVadj and the ordered M^T gather, partial
-// sums), a scalar kernel (||x||, the stopping test).  x is stored unscaled; its
-// scale 1/||x|| is applied as each value is read, which rounds exactly as a
-// separate scaling pass would.
-struct McNe {
-  float e, e0, s;          // current and previous ||U x||, scale of the stored x
-  int cnt, done, restart;  // steps taken, stop flag, restart in the current step
-  int nrestart;            // restarts so far (each consumed F*H*W drand48 draws)
-  int pad;
-  unsigned long long rand;  // drand48 state
-};
-constexpr int kPartDoubles = 2 * 1024 + 2 + 8;  // block partials, two totals, the McNe state
-static_assert(sizeof(McNe) <= 8 * sizeof(double), "McNe fits its slot");
+// ---- the power method ||U|| ---------------------------------------------------------
+// myNormest's loop (NestaUp.cpp:291-439) with U = tTV M and U^T = M^T tTVadj, whole in
+// one cooperative launch.  A step is two phases with a grid barrier after each:
+//   1  a thread warps its pixel for kNeFrames + 2 frames (each value once, where a
+//      thread per value would warp two frames for it), and writes g = tTVadj(U x)
+//      rather than U x itself; partial sums of |U x|^2
+//   2  x = M^T g, the ordered gather; partial sums of |x|^2
+// After a barrier every CTA adds the same partials in the same order for itself, so
+// that nobody waits for another one's scalars.  U x exactly zero (Scasum == 0,
+// NestaUp.cpp:369-385) takes a third phase, which puts the drand48 vector in U x's
+// place.  x is stored unscaled; its scale 1/||x|| is applied as each value is read,
+// which rounds exactly as a separate scaling pass would.  Bound by the latency of the
+// gathers and barriers.
+constexpr int kNeFrames = 2;     // frames per thread of phase 1
+constexpr int kNeMaxGrid = 1024;
+constexpr unsigned kNePolls = 1u << 22;
 constexpr float kNeTol = 1e-3f;
 constexpr int kNeMax = 100;
+struct McNe {
+  unsigned bar;             // arrivals at the grid barrier
+  int bad;                  // some CTA did not arrive in time
+  int nrestart;             // restarts (each consumed F*H*W drand48 draws)
+  int pad;
+};
+struct NeArgs {
+  float2 *x, *g;
+  double* part;             // [3 phases][kNeMaxGrid][2]: sum of squares, any value not zero
+  McNe* ne;
+  NestaDevState* st;
+  const float* xn;
+  const int *inv, *off, *csrc;
+  const float2* cw;
+  McRect r;
+  int W, H, F;
+  float e;
+  unsigned long long rand, ja, jc;  // drand48 state, and its jump by F*H*W draws
+};
+constexpr size_t kPartBytes = 3 * 2 * kNeMaxGrid * sizeof(double) + sizeof(McNe);
 
-__device__ __forceinline__ McNe* ne_state(double* part) { return reinterpret_cast<McNe*>(part + 2 * 1024 + 2); }
-
-// (M (s x))[k][p] for the stored, unscaled x
-__device__ __forceinline__ float2 warp_scaled(const float2* __restrict__ x, float sc, const float* __restrict__ xn, McRect r,
-                                             int e, int p, int k, int W, int H, int F, int* __restrict__ status) {
-  const float2* xf = x + size_t(k) * H * W;
-  if (e >= 0) {
-    const McPoint q = mc_point(xn, entry_offset(r, e, W), k, W, H, F);
+// (M (s x))[k][p] for the stored, unscaled x.  What other CTAs of the launch write is
+// read through plain pointers, after a barrier's acquire.
+__device__ __forceinline__ float2 warp_scaled(const float2* xf, float sc, const McPoint& q, bool in_rect, int p, int W,
+                                             int* status) {
+  if (in_rect) {
     if (q.ok) {
-      const float2 i1 = cscale(xf[q.ph + size_t(q.pv) * W], sc), i2 = cscale(xf[q.ph + 1 + size_t(q.pv) * W], sc);
-      const float2 i3 = cscale(xf[q.ph + size_t(q.pv + 1) * W], sc);
-      const float2 i4 = cscale(xf[q.ph + 1 + size_t(q.pv + 1) * W], sc);
+      const float2* const c0 = xf + q.ph + size_t(q.pv) * W;
+      const float2* const c1 = c0 + W;
+      const float2 i1 = cscale(c0[0], sc), i2 = cscale(c0[1], sc), i3 = cscale(c1[0], sc), i4 = cscale(c1[1], sc);
       const float a = float(q.ph + 1) - q.nh, b = q.nh - float(q.ph);
       const float c = float(q.pv + 1) - q.nv, d = q.nv - float(q.pv);
       const float2 aux1 = make_float2(lin2(a, i1.x, b, i2.x), lin2(a, i1.y, b, i2.y));
@@ -571,159 +562,199 @@ __device__ __forceinline__ float2 warp_scaled(const float2* __restrict__ x, floa
   return cscale(xf[p], sc);
 }
 
-__global__ void k_ne_init(double* part, float e, unsigned long long rand) {
-  McNe* ne = ne_state(part);
-  ne->e = e;
-  ne->e0 = 0.f;
-  ne->s = 1.0f / e;
-  ne->cnt = 0;
-  ne->done = !(fabsf(e - 0.f) > kNeTol * e && 0 < kNeMax);
-  ne->restart = 0;
-  ne->nrestart = 0;
-  ne->rand = rand;
-}
-
-// Sx = tTV(M (s x)), partial sums
-__global__ void __launch_bounds__(kNT) k_ne_u(const float2* __restrict__ x, float2* __restrict__ Sx,
-                                               const float* __restrict__ xn, const int* __restrict__ inv, McRect r,
-                                               int W, int H, int F, double* __restrict__ part, int* __restrict__ status) {
-  __shared__ double sred2[kNT / 32], sred1[kNT / 32];
-  const McNe* ne = ne_state(part);
-  if (ne->done) return;
-  const float sc = ne->s;
-  const size_t HW = size_t(H) * W, n = HW * F;
-  float s2 = 0.f, s1 = 0.f;
-  for (size_t i = blockIdx.x * size_t(kNT) + threadIdx.x; i < n; i += size_t(gridDim.x) * kNT) {
-    const int p = int(i % HW), k = int(i / HW);
-    const int e = inv[p];
-    const float2 w0 = warp_scaled(x, sc, xn, r, e, p, k, W, H, F, status);
-    const float2 wm = warp_scaled(x, sc, xn, r, e, p, (k + F - 1) % F, W, H, F, status);
-    const float2 a = csub(w0, wm);
-    Sx[i] = a;
-    s2 = fmaf(a.x, a.x, fmaf(a.y, a.y, s2));
-    s1 += fabsf(a.x) + fabsf(a.y);
-  }
-  warp_sums_to_block(s2, s1, sred2, sred1, part);
-}
-
-// sums of the block partials: each thread a strided subset in order, then
-// the threads in order
-__device__ __forceinline__ void ne_totals(const double* __restrict__ part, int nblk, double* sred, double* t2, double* t1) {
-  double s2 = 0.0, s1 = 0.0;
-  for (int b = threadIdx.x; b < nblk; b += kNT) {
-    s2 += part[2 * b];
-    s1 += part[2 * b + 1];
-  }
-  *t2 = block_sum<kNT>(s2, sred);
-  *t1 = block_sum<kNT>(s1, sred);
-}
-
-// e0 = e; restart test (Scasum(U x) == 0, NestaUp.cpp:369-385); e = ||U x||
-__global__ void __launch_bounds__(kNT) k_ne_s1(double* part, int nblk) {
-  __shared__ double sred[kNT / 32];
-  McNe* ne = ne_state(part);
-  if (ne->done) return;
-  double t2, t1;
-  ne_totals(part, nblk, sred, &t2, &t1);
+// All CTAs of the launch; false if some did not arrive in time.
+__device__ __forceinline__ bool ne_barrier(McNe* ne, unsigned target) {
+  __shared__ bool ok;
+  __syncthreads();
   if (threadIdx.x == 0) {
-    ne->e0 = ne->e;
-    ne->restart = (t1 == 0.0) ? 1 : 0;
-    if (!ne->restart) ne->e = float(sqrt(t2));
+    __threadfence();
+    atomicAdd(&ne->bar, 1u);
+    unsigned seen = 0, polls = 0;
+    for (;;) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(seen) : "l"(&ne->bar) : "memory");
+      if (seen >= target || ++polls >= kNePolls) break;
+      __nanosleep(32);
+    }
+    ok = seen >= target;
+    if (!ok) atomicExch(&ne->bad, 1);
   }
+  __syncthreads();
+  return ok;
 }
 
-// restart: Sx = (drand48(), 0) in element order, partial sums
-__global__ void __launch_bounds__(kNT) k_ne_restart(float2* __restrict__ Sx, size_t n, double* __restrict__ part) {
-  __shared__ double sred2[kNT / 32], sred1[kNT / 32];
-  const McNe* ne = ne_state(part);
-  if (ne->done || !ne->restart) return;
-  const unsigned long long x0 = ne->rand;
-  float s2 = 0.f, s1 = 0.f;
-  for (size_t i = blockIdx.x * size_t(kNT) + threadIdx.x; i < n; i += size_t(gridDim.x) * kNT) {
-    unsigned long long ra = 1, rc = 0, ba = 0x5DEECE66DULL, bc = 0xBULL, k = i + 1;
-    const unsigned long long mask = (1ULL << 48) - 1;
-    while (k) {
-      if (k & 1) {
-        rc = (ba * rc + bc) & mask;
-        ra = (ba * ra) & mask;
+// The CTA's partial: FP32 within a thread's few values and a warp, FP64 over the warps.
+__device__ __forceinline__ void ne_put(double* part, float s2, bool any) {
+  __shared__ double sred[kNT / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s2 += __shfl_down_sync(0xffffffffu, s2, o);
+  if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = double(s2);
+  const int some = __syncthreads_or(any);
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < kNT / 32; ++w) t += sred[w];
+    part[2 * blockIdx.x] = t;
+    part[2 * blockIdx.x + 1] = some ? 1.0 : 0.0;
+  }
+}
+// The launch's sum of squares (FP64, one warp: its rate is a small fraction of FP32's
+// here) and whether any value was not zero, to all threads.
+__device__ __forceinline__ double ne_total(const double* part, bool* any) {
+  __shared__ double total;
+  __shared__ int some;
+  if (threadIdx.x < 32) {
+    double t = 0.0, v[4];
+    bool a = false;
+    for (int b0 = 0; b0 < int(gridDim.x); b0 += 128) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int b = b0 + 32 * u + int(threadIdx.x);
+        v[u] = 0.0;
+        if (b < int(gridDim.x)) {
+          const double2 d = *reinterpret_cast<const double2*>(part + 2 * b);
+          v[u] = d.x;
+          a |= d.y != 0.0;
+        }
       }
-      bc = (ba * bc + bc) & mask;
-      ba = (ba * ba) & mask;
-      k >>= 1;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) t += v[u];
     }
-    const float2 a = make_float2(__double2float_rn(double((ra * x0 + rc) & mask) * 0x1p-48), 0.f);
-    Sx[i] = a;
-    s2 = fmaf(a.x, a.x, fmaf(a.y, a.y, s2));
-    s1 += fabsf(a.x) + fabsf(a.y);
-  }
-  warp_sums_to_block(s2, s1, sred2, sred1, part);
-}
-
-// after a restart: e = ||Sx||, the generator moved past the n draws
-__global__ void __launch_bounds__(kNT) k_ne_s1b(double* part, int nblk, unsigned long long ja, unsigned long long jc) {
-  __shared__ double sred[kNT / 32];
-  McNe* ne = ne_state(part);
-  if (ne->done || !ne->restart) return;
-  double t2, t1;
-  ne_totals(part, nblk, sred, &t2, &t1);
-  if (threadIdx.x == 0) {
-    ne->e = float(sqrt(t2));
-    ne->rand = (ja * ne->rand + jc) & ((1ULL << 48) - 1);
-    ne->nrestart += 1;
-  }
-}
-
-// x = M^T tTVadj(Sx) (operatorUt without negation), partial sums
-__global__ void __launch_bounds__(kNT) k_ne_ut(const float2* __restrict__ Sx, float2* __restrict__ x,
-                                                const int* __restrict__ off, const int* __restrict__ csrc,
-                                                const float2* __restrict__ cw, McRect r, int W, int H, int F,
-                                                double* __restrict__ part) {
-  __shared__ double sred2[kNT / 32], sred1[kNT / 32];
-  const McNe* ne = ne_state(part);
-  if (ne->done) return;
-  const size_t HW = size_t(H) * W, n = HW * F;
-  float s2 = 0.f, s1 = 0.f;
-  for (size_t q = blockIdx.x * size_t(kNT) + threadIdx.x; q < n; q += size_t(gridDim.x) * kNT) {
-    const int p = int(q % HW), row = p / W, col = p % W;
-    const size_t k = q / HW;
-    const float2* u0 = Sx + k * HW;                   // tTVadj: u_{f+1} - u_f
-    const float2* u1 = Sx + size_t((k + 1) % F) * HW;
-    const bool in_rect = row >= r.r1b && row < r.r1b + r.l1 && col >= r.r2b && col < r.r2b + r.l2;
-    float2 acc = in_rect ? make_float2(0.f, 0.f) : csub(u1[p], u0[p]);
-    for (int c = off[q], ce = off[q + 1]; c < ce; ++c) {
-      const float2 w = __ldg(cw + c);
-      const int src = __ldg(csrc + c);
-      const float2 v = csub(u1[src], u0[src]);
-      acc.x = __fadd_rn(acc.x, __fmul_rn(__fmul_rn(v.x, w.x), w.y));
-      acc.y = __fadd_rn(acc.y, __fmul_rn(__fmul_rn(v.y, w.x), w.y));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    a = __any_sync(0xffffffffu, a);
+    if (threadIdx.x == 0) {
+      total = t;
+      some = a;
     }
-    x[q] = acc;
-    s2 = fmaf(acc.x, acc.x, fmaf(acc.y, acc.y, s2));
-    s1 += fabsf(acc.x) + fabsf(acc.y);
   }
-  warp_sums_to_block(s2, s1, sred2, sred1, part);
+  __syncthreads();
+  *any = some != 0;
+  return total;
 }
 
-// ||x||, the scale of the next step, the stopping test
-__global__ void __launch_bounds__(kNT) k_ne_s2(double* part, int nblk) {
-  __shared__ double sred[kNT / 32];
-  McNe* ne = ne_state(part);
-  if (ne->done) return;
-  double t2, t1;
-  ne_totals(part, nblk, sred, &t2, &t1);
-  if (threadIdx.x == 0) {
-    const float nx = float(sqrt(t2));
-    ne->s = 1.0f / nx;
-    ne->cnt += 1;
-    ne->done = !(fabsf(ne->e - ne->e0) > kNeTol * ne->e && ne->cnt < kNeMax);
+// draw i + 1 of the drand48 generator in state x0
+__device__ __forceinline__ float ne_draw(unsigned long long x0, unsigned long long i) {
+  unsigned long long ra = 1, rc = 0, ba = 0x5DEECE66DULL, bc = 0xBULL, k = i + 1;
+  const unsigned long long mask = (1ULL << 48) - 1;
+  while (k) {
+    if (k & 1) {
+      rc = (ba * rc + bc) & mask;
+      ra = (ba * ra) & mask;
+    }
+    bc = (ba * bc + bc) & mask;
+    ba = (ba * ba) & mask;
+    k >>= 1;
   }
+  return __double2float_rn(double((ra * x0 + rc) & mask) * 0x1p-48);
 }
 
-__global__ void k_ne_finish(const double* part, NestaDevState* st) {
-  const McNe* ne = ne_state(const_cast<double*>(part));
-  st->normU = ne->e;
-  st->normest_iters = ne->cnt;
-  st->ne_done = 1;
+__global__ void __launch_bounds__(kNT, 4) k_normest(NeArgs n) {
+  const int W = n.W, H = n.H, F = n.F, HW = H * W;
+  const int npb = (HW + kNT - 1) / kNT, nfg = (F + kNeFrames - 1) / kNeFrames;
+  const McRect r = n.r;
+  unsigned long long rand = n.rand;
+  float e = n.e, e0 = 0.f, sc = 1.0f / n.e;
+  int cnt = 0, nrestart = 0;
+  unsigned gen = 0;
+  bool any;
+  while (fabsf(e - e0) > kNeTol * e && cnt < kNeMax) {
+    float s2 = 0.f;
+    bool nz = false;
+    for (int b = blockIdx.x; b < npb * nfg; b += gridDim.x) {
+      const int p = (b % npb) * kNT + threadIdx.x, f0 = (b / npb) * kNeFrames, nf = min(kNeFrames, F - f0);
+      if (p >= HW) continue;
+      const int ent = __ldg(n.inv + p);
+      const int xo = ent >= 0 ? entry_offset(r, ent, W) : 0;
+      constexpr int NW = kNeFrames + 2;
+      int fr[NW];
+      McPoint q[NW];
+      float2 w[NW];
+#pragma unroll
+      for (int u = 0; u < NW; ++u) fr[u] = (f0 - 1 + u + F) % F;
+#pragma unroll
+      for (int u = 0; u < NW; ++u)
+        if (ent >= 0 && u < nf + 2) q[u] = mc_point(n.xn, xo, fr[u], W, H, F);
+#pragma unroll
+      for (int u = 0; u < NW; ++u)
+        if (u < nf + 2) w[u] = warp_scaled(n.x + size_t(fr[u]) * HW, sc, q[u], ent >= 0, p, W, &n.st->status);
+#pragma unroll
+      for (int u = 0; u < kNeFrames; ++u) {
+        if (u < nf) {
+          const float2 a = csub(w[u + 1], w[u]);
+          s2 = fmaf(a.x, a.x, fmaf(a.y, a.y, s2));
+          nz |= fabsf(a.x) + fabsf(a.y) != 0.f;
+          n.g[size_t(f0 + u) * HW + p] = csub(csub(w[u + 2], w[u + 1]), a);
+        }
+      }
+    }
+    double* part = n.part;
+    ne_put(part, s2, nz);
+    if (!ne_barrier(n.ne, (gen += gridDim.x))) return;
+    double t2 = ne_total(part, &any);
+    e0 = e;
+    if (!any) {  // uniform over the grid
+      s2 = 0.f;
+      for (int b = blockIdx.x; b < npb * F; b += gridDim.x) {
+        const int p = (b % npb) * kNT + threadIdx.x, f = b / npb;
+        if (p >= HW) continue;
+        const float a = ne_draw(rand, (unsigned long long)f * HW + p);
+        s2 = fmaf(a, a, s2);
+        n.g[size_t(f) * HW + p] =
+            make_float2(__fsub_rn(ne_draw(rand, (unsigned long long)((f + 1) % F) * HW + p), a), 0.f);
+      }
+      part += 2 * kNeMaxGrid;
+      ne_put(part, s2, false);
+      if (!ne_barrier(n.ne, (gen += gridDim.x))) return;
+      t2 = ne_total(part, &any);
+      rand = (n.ja * rand + n.jc) & ((1ULL << 48) - 1);
+      nrestart += 1;
+    }
+    e = float(sqrt(t2));
+    s2 = 0.f;
+    for (int b = blockIdx.x; b < npb * F; b += gridDim.x) {
+      const int p = (b % npb) * kNT + threadIdx.x, f = b / npb;
+      if (p >= HW) continue;
+      const size_t t = size_t(f) * HW + p;
+      const float2* const gf = n.g + size_t(f) * HW;
+      const int row = p / W, col = p % W;
+      const bool in_rect = row >= r.r1b && row < r.r1b + r.l1 && col >= r.r2b && col < r.r2b + r.l2;
+      int c = __ldg(n.off + t);
+      const int ce = __ldg(n.off + t + 1);
+      float2 acc = in_rect ? make_float2(0.f, 0.f) : gf[p];
+      while (c < ce) {
+        const int m = min(4, ce - c);
+        float2 w[4], v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (u < m) {
+            w[u] = __ldg(n.cw + c + u);
+            v[u] = gf[__ldg(n.csrc + c + u)];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (u < m) {
+            acc.x = __fadd_rn(acc.x, __fmul_rn(__fmul_rn(v[u].x, w[u].x), w[u].y));
+            acc.y = __fadd_rn(acc.y, __fmul_rn(__fmul_rn(v[u].y, w[u].x), w[u].y));
+          }
+        }
+        c += m;
+      }
+      n.x[t] = acc;
+      s2 = fmaf(acc.x, acc.x, fmaf(acc.y, acc.y, s2));
+    }
+    part = n.part + 4 * kNeMaxGrid;
+    ne_put(part, s2, false);
+    if (!ne_barrier(n.ne, (gen += gridDim.x))) return;
+    sc = 1.0f / float(sqrt(ne_total(part, &any)));
+    cnt += 1;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    n.ne->nrestart = nrestart;
+    n.st->normU = e;
+    n.st->normest_iters = cnt;
+    n.st->ne_done = 1;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -816,7 +847,7 @@ int motion_set(gbn_problem* P, const float* xn, const int* xmesh, const int* bb)
     cudaError_t e = cudaMalloc(&P->mc_xw, X * sizeof(float2));
     if (e == cudaSuccess) e = cudaMalloc(&P->mc_g, X * sizeof(float2));
     if (e == cudaSuccess) e = cudaMalloc(&P->mc_gm, X * sizeof(float2));
-    if (e == cudaSuccess) e = cudaMalloc(&P->mc_part, kPartDoubles * sizeof(double));
+    if (e == cudaSuccess) e = cudaMalloc(&P->mc_part, kPartBytes);
     if (e != cudaSuccess) {
       cudaGetLastError();
       motion_free(P);
@@ -843,57 +874,53 @@ void mc_apply(gbn_ctx* ctx, gbn_problem* P, const float2* in, float2* out, cudaS
   ctx->launches += 1;
 }
 
-// myNormest (NestaUp.cpp:291-439) with U = tTV M, U^T = M^T tTVadj: steps on
-// the device (k_ne_*), enqueued kNeChunk at a time; the host reads each
-// chunk's stop flag while the next chunk runs
+// myNormest (NestaUp.cpp:291-439) with U = tTV M, U^T = M^T tTVadj
 int mc_normest(gbn_ctx* ctx, gbn_problem* P, cudaStream_t s) {
-  constexpr int kNeChunk = 8;
-  const int W = P->W, H = P->H, F = P->F;
-  const size_t X = size_t(W) * H * F;
+  const size_t X = size_t(P->W) * P->H * P->F;
   const McTables* t = P->mc_tab;
-  const McRect r = mc_rect(W, H, P->mc_bb);
-  float2 *x = P->mc_gm, *Sx = P->mc_g;
-  const int nblk = std::min(1024, grid1(ctx, X));
-  const float e_init = float(std::sqrt(double(X)));  // ||ones||
   const Lcg48 jX = lcg48_jump(uint64_t(X));
-  k_fill<<<grid1(ctx, X), kNT, 0, s>>>(x, X, make_float2(1.f, 0.f));
-  k_ne_init<<<1, 1, 0, s>>>(P->mc_part, e_init, (unsigned long long)ctx->rand48);
+  static const int per_sm = [] {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_normest, kNT, 0) != cudaSuccess) {
+      cudaGetLastError();
+      n = 1;
+    }
+    return n;
+  }();
+  NeArgs n{};
+  n.x = P->mc_gm;
+  n.g = P->mc_g;
+  n.part = P->mc_part;
+  n.ne = reinterpret_cast<McNe*>(P->mc_part + 3 * 2 * kNeMaxGrid);
+  n.st = P->st;
+  n.xn = P->mc_xn;
+  n.inv = t->inv;
+  n.off = t->off;
+  n.csrc = t->csrc;
+  n.cw = t->cw;
+  n.r = mc_rect(P->W, P->H, P->mc_bb);
+  n.W = P->W;
+  n.H = P->H;
+  n.F = P->F;
+  n.e = float(std::sqrt(double(X)));  // ||ones||
+  n.rand = (unsigned long long)ctx->rand48;
+  n.ja = (unsigned long long)jX.a;
+  n.jc = (unsigned long long)jX.c;
+  // every CTA of the launch is resident
+  const size_t blocks = size_t((P->W * P->H + kNT - 1) / kNT) * P->F;
+  const int grid = int(std::min<size_t>(std::min(kNeMaxGrid, ctx->nsm * per_sm), blocks));
+  cudaError_t e = cudaMemsetAsync(n.ne, 0, sizeof(McNe), s);
+  if (e != cudaSuccess) return cuda_status(e, "power method");
+  k_fill<<<grid1(ctx, X), kNT, 0, s>>>(n.x, X, make_float2(1.f, 0.f));
+  void* args[] = {&n};
+  e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_normest), dim3(grid), dim3(kNT), args, 0, s);
   ctx->launches += 2;
-  // chunks of steps with one chunk of lookahead: the host waits for chunk
-  // c-1's stop flag (pinned, copied behind it) while chunk c runs
-  int rc = host_flags_ready(ctx);
-  if (rc != GBN_OK) return rc;
-  const McNe* dne = reinterpret_cast<const McNe*>(P->mc_part + 2 * 1024 + 2);
-  cudaError_t e = cudaSuccess;
-  int chunk = 0;
-  for (int steps = 0; steps < kNeMax; ++chunk) {
-    for (int k = 0; k < kNeChunk && steps < kNeMax; ++k, ++steps) {
-      k_ne_u<<<nblk, kNT, 0, s>>>(x, Sx, P->mc_xn, t->inv, r, W, H, F, P->mc_part, &P->st->status);
-      k_ne_s1<<<1, kNT, 0, s>>>(P->mc_part, nblk);
-      k_ne_restart<<<nblk, kNT, 0, s>>>(Sx, X, P->mc_part);
-      k_ne_s1b<<<1, kNT, 0, s>>>(P->mc_part, nblk, (unsigned long long)jX.a, (unsigned long long)jX.c);
-      k_ne_ut<<<nblk, kNT, 0, s>>>(Sx, x, t->off, t->csrc, t->cw, r, W, H, F, P->mc_part);
-      k_ne_s2<<<1, kNT, 0, s>>>(P->mc_part, nblk);
-      ctx->launches += 6;
-    }
-    if ((e = cudaMemcpyAsync(&ctx->host_flags[chunk & 1], &dne->done, sizeof(int), cudaMemcpyDeviceToHost, s)) !=
-            cudaSuccess ||
-        (e = cudaEventRecord(ctx->ev_flag[chunk & 1], s)) != cudaSuccess)
-      return cuda_status(e, "power method");
-    if (chunk > 0) {
-      if ((e = cudaEventSynchronize(ctx->ev_flag[(chunk - 1) & 1])) != cudaSuccess) return cuda_status(e, "power method");
-      if (ctx->host_flags[(chunk - 1) & 1]) break;
-    }
-  }
-  struct {
-    int nrestart;
-  } h{0};
-  if ((e = cudaMemcpyAsync(&h.nrestart, &dne->nrestart, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-      (e = cudaStreamSynchronize(s)) != cudaSuccess)
-    return cuda_status(e, "power method");
+  McNe h{};
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, n.ne, sizeof(h), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return cuda_status(e, "power method");
+  if (h.bad) return set_error(GBN_ERR_CUDA, "power method: the CTAs did not all arrive at a barrier");
   for (int i = 0; i < h.nrestart; ++i) ctx->rand48 = lcg48_apply(jX, ctx->rand48);
-  k_ne_finish<<<1, 1, 0, s>>>(P->mc_part, P->st);
-  ctx->launches += 1;
   return GBN_OK;
 }
 
