@@ -53,19 +53,19 @@ uint64_t lcg48_apply(const Lcg48& j, uint64_t x);
 
 // tables of one problem's meshes (rebuilt at every run)
 struct McTables {
-  int* inv = nullptr;         // [H*W] rectangle entry landing on each pixel, -1 none
+  int* inv = nullptr;         // [H*W] rectangle entry landing on each pixel (then its R1*W + R2), -1 none
   int* cnt = nullptr;         // [F*H*W] contributions per target (then fill cursors)
   int* off = nullptr;         // [F*H*W + 1] exclusive prefix sums of cnt
   int* bsum = nullptr;        // [scan blocks] block totals of the prefix sum
   int* key = nullptr;         // [4 * l1 * l2 * F] contributions grouped by target, sorted by entry * 4 + corner,
                               // then rewritten to (the entry's pixel R1*W + R2) * 4 + corner
-  int* srcmap = nullptr;      // [H*W] pixel each entry (by its R1*W + R2) reads in the adjoint
+  int* srcmap = nullptr;      // [H*W + 1] pixel each entry (by its R1*W + R2) reads in the adjoint; whether any differs
+  int* at = nullptr;          // [F][H*W] upper-left pixel of each entry's square in frame f, -1 outside the image
   float2* wts = nullptr;      // [F][H*W] (Whh, Wvv): each entry's fractional position in frame f
-  int* csrc = nullptr;        // [4 * l1 * l2 * F] per contribution: the pixel the adjoint reads
-  float2* cw = nullptr;       // [4 * l1 * l2 * F] per contribution: its two weights (fa, fb)
   double* tvpart = nullptr;   // [F * pixel blocks][2] partial sums of the fused tTV kernel
   size_t x = 0, entries = 0;  // F*H*W and l1*l2 the buffers were sized for
   int nbp = 0, nscan = 0;
+  size_t hw = 0;              // H*W
 };
 
 namespace {
@@ -111,52 +111,62 @@ __device__ __forceinline__ int entry_offset(McRect r, int e, int W) {
 
 __device__ __forceinline__ McPoint mc_point(const float* __restrict__ xn, int xo, int k, int W, int H, int F) {
   const size_t HW = size_t(H) * W;
+  const float* const xk = xn + k * HW;
   McPoint q;
-  q.nh = xn[xo + k * HW] - 1.f;
-  q.nv = xn[xo + k * HW + HW * F] - 1.f;
+  q.nh = __ldg(xk + xo) - 1.f;
+  q.nv = __ldg(xk + HW * F + xo) - 1.f;
   q.ph = int(floorf(q.nh));
   q.pv = int(floorf(q.nv));
   q.ok = q.ph >= 0 && q.ph + 1 < W && q.pv >= 0 && q.pv + 1 < H;
   return q;
 }
 
-// p*u + q*v with both products and the sum rounded separately
-__device__ __forceinline__ float lin2(float p, float u, float q, float v) {
-  return __fadd_rn(__fmul_rn(p, u), __fmul_rn(q, v));
-}
+// frame f of a periodic series, -F <= f < 2 F
+__device__ __forceinline__ int wrap_frame(int f, int F) { return f < 0 ? f + F : f >= F ? f - F : f; }
 
-// the interpolator's value (optimizer.cl:832-877) at q from frame xf, in the
+// M's points, one per entry (at its pixel R1*W + R2) and frame: the square's upper-left
+// pixel (-1: a corner is outside the image, the value stays) and the fractional
+// position (Whh, Wvv).  1 - Whh is the interpolator's float(ph + 1) - nh bit for bit:
+// past the first pixel both are exact, in it they are the same subtraction.
+struct McPoints {
+  const int *inv, *at;
+  const float2* wts;
+};
+
+// the interpolator's value (optimizer.cl:832-877) of frame xf at q, in the
 // kernel's order with separately rounded products and sums: with motion
 // compensation the power method starts from this interpolation's rounding
-// residue on a constant image, so ||U|| depends on these exact bits
-__device__ __forceinline__ float2 bilinear(const float2* __restrict__ xf, const McPoint& q, int W) {
-  const float2 i1 = xf[q.ph + size_t(q.pv) * W], i2 = xf[q.ph + 1 + size_t(q.pv) * W];
-  const float2 i3 = xf[q.ph + size_t(q.pv + 1) * W], i4 = xf[q.ph + 1 + size_t(q.pv + 1) * W];
-  const float a = float(q.ph + 1) - q.nh, b = q.nh - float(q.ph);
-  const float c = float(q.pv + 1) - q.nv, d = q.nv - float(q.pv);
-  const float2 aux1 = make_float2(lin2(a, i1.x, b, i2.x), lin2(a, i1.y, b, i2.y));
-  const float2 aux2 = make_float2(lin2(a, i3.x, b, i4.x), lin2(a, i3.y, b, i4.y));
-  return make_float2(lin2(c, aux1.x, d, aux2.x), lin2(c, aux1.y, d, aux2.y));
+// residue on a constant image, so ||U|| depends on these exact bits.  SCALED: of s x,
+// each product rounded.  x is read through a plain pointer: other CTAs of the launch
+// may have written it before a barrier.
+struct McAt {
+  int at;
+  float2 w;
+};
+__device__ __forceinline__ McAt mc_at(const McPoints& m, int xo, size_t plane) {
+  return {__ldg(m.at + plane + xo), __ldg(m.wts + plane + xo)};
 }
-
-// (M x)[k][p]
-__device__ __forceinline__ float2 warp_at(const float2* __restrict__ x, const float* __restrict__ xn, McRect r, int e,
-                                          int p, int k, int W, int H, int F, int* __restrict__ status) {
-  const float2* xf = x + size_t(k) * H * W;
-  if (e < 0) return xf[p];
-  const McPoint q = mc_point(xn, entry_offset(r, e, W), k, W, H, F);
-  if (!q.ok) {
-    atomicExch(status, kStatusMotionRange);
-    return xf[p];
-  }
-  return bilinear(xf, q, W);
+// p*u + q*v with both products and the sum rounded separately (the packed products and
+// sums fuse)
+__device__ __forceinline__ float2 lin2(float p, float2 u, float q, float2 v) {
+  return make_float2(__fadd_rn(__fmul_rn(p, u.x), __fmul_rn(q, v.x)), __fadd_rn(__fmul_rn(p, u.y), __fmul_rn(q, v.y)));
+}
+template <bool SCALED>
+__device__ __forceinline__ float2 mc_value(const float2* xf, const McAt& q, int p, int W, float s) {
+  auto get = [&](const float2* v) { return SCALED ? make_float2(__fmul_rn(v->x, s), __fmul_rn(v->y, s)) : *v; };
+  if (q.at < 0) return get(xf + p);
+  const float2 *const c0 = xf + q.at, *const c1 = c0 + W;
+  const float2 i1 = get(c0), i2 = get(c0 + 1), i3 = get(c1), i4 = get(c1 + 1);
+  const float a = __fsub_rn(1.f, q.w.x), c = __fsub_rn(1.f, q.w.y);
+  return lin2(c, lin2(a, i1, q.w.x, i2), q.w.y, lin2(a, i3, q.w.x, i4));
 }
 
 // ---- table construction ------------------------------------------------------
 // inv[ver*W + hor] = the largest entry e whose original-mesh point is (hor, ver);
-// srcmap[R1*W + R2] = that pixel (-1 outside the image)
+// srcmap[R1*W + R2] = that pixel (-1 outside the image); moved: some entry's pixel is
+// not its own
 __global__ void k_mc_inv(const int* __restrict__ xm, McRect r, int W, int H, int* __restrict__ inv,
-                         int* __restrict__ srcmap, int* __restrict__ status) {
+                         int* __restrict__ srcmap, int* __restrict__ moved, int* __restrict__ status) {
   const int E = r.l1 * r.l2;
   const size_t HW = size_t(H) * W;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < E; e += gridDim.x * blockDim.x) {
@@ -168,30 +178,33 @@ __global__ void k_mc_inv(const int* __restrict__ xm, McRect r, int W, int H, int
       continue;
     }
     srcmap[R1 * W + R2] = ver * W + hor;
+    if (hor != R2 || ver != R1) *moved = 1;
     atomicMax(inv + size_t(ver) * W + hor, e);
   }
 }
 
-// the (entry, frame) pairs that scatter: target pixel (its original-mesh point) in the image, corners too
-__device__ __forceinline__ bool scatter_point(const float* __restrict__ xn, const int* __restrict__ xm, McRect r, int e,
-                                              int k, int W, int H, int F, McPoint* q, int* src) {
-  const size_t HW = size_t(H) * W;
-  const int R1 = r.r1b + e % r.l1, R2 = r.r2b + e / r.l1;
-  const int hor = xm[R1 + size_t(R2) * H] - 1, ver = xm[R1 + size_t(R2) * H + HW] - 1;
-  *q = mc_point(xn, R2 + R1 * W, k, W, H, F);
-  *src = ver * W + hor;
-  return q->ok && hor >= 0 && hor < W && ver >= 0 && ver < H;
+// The (entry, frame) pairs that scatter: target pixel (its original-mesh point) in the
+// image, corners too.  Grid y: frames; the threads run along an image row, the meshes'
+// and tables' fast axis (entries count down the columns; 256 x 256 x 20: count and fill
+// 118 us with the threads along those, 28 now).
+struct McEntry {
+  int e, xo;  // entry number, pixel R1*W + R2
+};
+__device__ __forceinline__ McEntry row_entry(McRect r, int t, int W) {
+  const int i = t / r.l2, j = t - i * r.l2;
+  return {i + r.l1 * j, (r.r1b + i) * W + r.r2b + j};
 }
 
-__global__ void k_mc_count(const float* __restrict__ xn, const int* __restrict__ xm, McRect r, int W, int H, int F,
-                           int* __restrict__ cnt, int* __restrict__ status) {
-  const int E = r.l1 * r.l2;
-  const size_t HW = size_t(H) * W, n = size_t(E) * F;
-  for (size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x; t < n; t += size_t(gridDim.x) * blockDim.x) {
-    const int e = int(t % E), k = int(t / E);
-    McPoint q;
-    int src;
-    if (!scatter_point(xn, xm, r, e, k, W, H, F, &q, &src)) {
+__global__ void __launch_bounds__(kNT) k_mc_count(const float* __restrict__ xn, const int* __restrict__ srcmap, McRect r,
+                                                  int W, int H, int F, int* __restrict__ cnt, int* __restrict__ status) {
+  const int t = blockIdx.x * kNT + threadIdx.x;
+  if (t >= r.l1 * r.l2) return;
+  const McEntry m = row_entry(r, t, W);
+  const bool in = srcmap[m.xo] >= 0;
+  const size_t HW = size_t(H) * W;
+  for (int k = blockIdx.y; k < F; k += gridDim.y) {
+    const McPoint q = mc_point(xn, m.xo, k, W, H, F);
+    if (!(q.ok && in)) {
       atomicExch(status, kStatusMotionRange);
       continue;
     }
@@ -276,121 +289,151 @@ __global__ void k_scan_add(int* __restrict__ out, size_t n, const int* __restric
 
 // the contributions of every scattering (entry, frame) to its four corners,
 // and the entry's fractional position (Whh, Wvv) the weights derive from
-__global__ void k_mc_fill(const float* __restrict__ xn, const int* __restrict__ xm, McRect r, int W, int H, int F,
-                          const int* __restrict__ off, int* __restrict__ cur, int* __restrict__ key,
-                          float2* __restrict__ wts) {
-  const int E = r.l1 * r.l2;
-  const size_t HW = size_t(H) * W, n = size_t(E) * F;
-  for (size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x; t < n; t += size_t(gridDim.x) * blockDim.x) {
-    const int e = int(t % E), k = int(t / E);
-    McPoint q;
-    int src;
-    if (!scatter_point(xn, xm, r, e, k, W, H, F, &q, &src)) continue;
-    wts[k * HW + entry_offset(r, e, W)] = make_float2(q.nh - float(q.ph), q.nv - float(q.pv));
+__global__ void __launch_bounds__(kNT) k_mc_fill(const float* __restrict__ xn, const int* __restrict__ srcmap, McRect r,
+                                                 int W, int H, int F, const int* __restrict__ off, int* __restrict__ cur,
+                                                 int* __restrict__ key, int* __restrict__ at_out,
+                                                 float2* __restrict__ wts) {
+  const int t = blockIdx.x * kNT + threadIdx.x;
+  if (t >= r.l1 * r.l2) return;
+  const McEntry m = row_entry(r, t, W);
+  const bool in = srcmap[m.xo] >= 0;
+  const size_t HW = size_t(H) * W;
+  for (int k = blockIdx.y; k < F; k += gridDim.y) {
+    const McPoint q = mc_point(xn, m.xo, k, W, H, F);
+    at_out[k * HW + m.xo] = q.ok ? q.ph + q.pv * W : -1;
+    wts[k * HW + m.xo] = make_float2(q.nh - float(q.ph), q.nv - float(q.pv));
+    if (!q.ok || !in) continue;
     const size_t q00 = k * HW + size_t(q.pv) * W + q.ph;
     const size_t tq[4] = {q00, q00 + 1, q00 + W, q00 + W + 1};
+    int at[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) key[off[tq[c]] + atomicAdd(cur + tq[c], 1)] = e * 4 + c;
+    for (int c = 0; c < 4; ++c) at[c] = off[tq[c]] + atomicAdd(cur + tq[c], 1);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) key[at[c]] = m.e * 4 + c;
   }
 }
 
-// each target's contributions into key order (lists are short: insertion sort)
-__global__ void k_mc_sort(const int* __restrict__ off, int* __restrict__ key, size_t n) {
-  for (size_t q = blockIdx.x * size_t(blockDim.x) + threadIdx.x; q < n; q += size_t(gridDim.x) * blockDim.x) {
-    const int b = off[q], e = off[q + 1];
-    for (int i = b + 1; i < e; ++i) {
-      const int v = key[i];
-      int j = i - 1;
-      while (j >= b && key[j] > v) {
-        key[j + 1] = key[j];
-        --j;
+// Each target's contributions in key order (the reference's work-item order), the
+// keys then renumbered to the entry's pixel * 4 + corner, and inv likewise, so that no
+// later kernel divides.  Lists are short, four where the mesh is smooth: up to kMcShort
+// sort in registers, longer ones in place (one kernel for the sort, one for the
+// numbers and one for tables of sources and weights: 97 us; 19 here).
+constexpr int kMcShort = 8;
+__global__ void __launch_bounds__(kNT) k_mc_lists(const int* __restrict__ off, int* __restrict__ key,
+                                                  int* __restrict__ inv, McRect r, int W, int HW, int F) {
+  const int p = blockIdx.x * kNT + threadIdx.x;
+  if (p >= HW) return;
+  if (blockIdx.y == 0) {
+    const int e = inv[p];
+    if (e >= 0) inv[p] = entry_offset(r, e, W);
+  }
+  for (int k = blockIdx.y; k < F; k += gridDim.y) {
+    const size_t q = size_t(k) * HW + p;
+    const int b = off[q], n = off[q + 1] - b;
+    auto number = [&](int kc) { return entry_offset(r, kc >> 2, W) * 4 + (kc & 3); };
+    if (n <= kMcShort) {
+      int v[kMcShort];
+#pragma unroll
+      for (int u = 0; u < kMcShort; ++u) v[u] = u < n ? key[b + u] : 0x7fffffff;
+#pragma unroll
+      for (int s = 0; s < kMcShort; ++s)  // odd-even transposition
+#pragma unroll
+        for (int u = s & 1; u + 1 < kMcShort; u += 2) {
+          const int lo = min(v[u], v[u + 1]);
+          v[u + 1] = max(v[u], v[u + 1]);
+          v[u] = lo;
+        }
+#pragma unroll
+      for (int u = 0; u < kMcShort; ++u)
+        if (u < n) key[b + u] = number(v[u]);
+    } else {
+      for (int i = b + 1; i < b + n; ++i) {
+        const int v = key[i];
+        int j = i - 1;
+        while (j >= b && key[j] > v) {
+          key[j + 1] = key[j];
+          --j;
+        }
+        key[j + 1] = v;
       }
-      key[j + 1] = v;
+      for (int c = b; c < b + n; ++c) key[c] = number(key[c]);
     }
   }
 }
 
-// sorted keys entry * 4 + corner -> (the entry's pixel R1*W + R2) * 4 + corner,
-// so that neighbouring targets read neighbouring table entries
-__global__ void k_mc_rekey(int* __restrict__ key, const int* __restrict__ total, McRect r, int W) {
-  const size_t n = size_t(*total);  // contributions filled (off[F*H*W])
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-    const int k = key[i];
-    key[i] = entry_offset(r, k >> 2, W) * 4 + (k & 3);
+// (M^T g) at pixel p of the frame whose plane starts at `plane`: the target's
+// contributions in the reference's order, where corner c of an entry's square gets
+// (g * fa) * fb with fa = Whh or 1 - Whh (c & 1), fb = Wvv or 1 - Wvv (c & 2), as
+// optimizer.cl:880-937 rounds them.  The loads of up to four are issued before any is
+// accumulated.  The weights come from the entries' table, which four targets share, and
+// the pixel from the key, not from tables per contribution (12 bytes each, 63 MB at 256 x
+// 256 x 20).  g is read through a plain pointer: other CTAs of the launch may have
+// written it before a barrier.
+struct McLists {
+  const int *off, *key, *srcmap, *moved;
+  const float2* wts;
+};
+__device__ __forceinline__ float2 mc_adjoint_at(const McLists& l, const float2* g, size_t plane, int p, bool in_rect,
+                                                bool moved) {
+  const float2 *const gk = g + plane, *const wk = l.wts + plane;
+  int c = __ldg(l.off + plane + p);
+  const int ce = __ldg(l.off + plane + p + 1);
+  float2 acc = in_rect ? make_float2(0.f, 0.f) : gk[p];
+  for (; c < ce; c += 4) {
+    int k[4];
+    float2 w[4], v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) k[u] = c + u < ce ? __ldg(l.key + c + u) : -1;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (k[u] >= 0) {
+        const int xo = k[u] >> 2;
+        w[u] = __ldg(wk + xo);
+        v[u] = gk[moved ? __ldg(l.srcmap + xo) : xo];
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (k[u] >= 0) {
+        const float fa = (k[u] & 1) ? w[u].x : __fsub_rn(1.f, w[u].x);
+        const float fb = (k[u] & 2) ? w[u].y : __fsub_rn(1.f, w[u].y);
+        acc.x = __fadd_rn(acc.x, __fmul_rn(__fmul_rn(v[u].x, fa), fb));
+        acc.y = __fadd_rn(acc.y, __fmul_rn(__fmul_rn(v[u].y, fa), fb));
+      }
   }
-}
-
-// per contribution, what the adjoint gathers need: the pixel it reads and its
-// two weights fa = Whh or 1 - Whh (corner bit 0), fb = Wvv or 1 - Wvv (bit 1),
-// rounded as optimizer.cl:880-937 forms them
-__global__ void k_mc_pack(const int* __restrict__ off, const int* __restrict__ key, const int* __restrict__ srcmap,
-                          const float2* __restrict__ wts, int* __restrict__ csrc, float2* __restrict__ cw, size_t X,
-                          size_t HW) {
-  for (size_t q = blockIdx.x * size_t(blockDim.x) + threadIdx.x; q < X; q += size_t(gridDim.x) * blockDim.x) {
-    const float2* wk = wts + (q / HW) * HW;
-    for (int c = off[q], ce = off[q + 1]; c < ce; ++c) {
-      const int kc = key[c], e = kc >> 2;
-      const float2 w = wk[e];
-      csrc[c] = srcmap[e];
-      cw[c] = make_float2((kc & 1) ? w.x : __fsub_rn(1.f, w.x), (kc & 2) ? w.y : __fsub_rn(1.f, w.y));
-    }
-  }
+  return acc;
 }
 
 // ---- the operators -------------------------------------------------------------
-// out = M x (MotionCompensation: copy, then the interpolator), one thread per pixel
-__global__ void k_mc_warp(const float2* __restrict__ x, float2* __restrict__ out, const float* __restrict__ xn,
-                          const int* __restrict__ inv, McRect r, int W, int H, int F, int* __restrict__ status) {
-  const size_t HW = size_t(H) * W, n = HW * F;
-  for (size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x; t < n; t += size_t(gridDim.x) * blockDim.x) {
-    const int p = int(t % HW), k = int(t / HW);
-    out[t] = warp_at(x, xn, r, inv[p], p, k, W, H, F, status);
+// out = M x (MotionCompensation: copy, then the interpolator), one thread per pixel; grid y: frames
+__global__ void __launch_bounds__(kNT) k_mc_warp(const float2* __restrict__ x, float2* __restrict__ out, McPoints m,
+                                                 int W, int HW, int F) {
+  const int p = blockIdx.x * kNT + threadIdx.x;
+  if (p >= HW) return;
+  const int xo = m.inv[p];
+  for (int k = blockIdx.y; k < F; k += gridDim.y) {
+    const size_t o = size_t(k) * HW;
+    const McAt q = xo >= 0 ? mc_at(m, xo, o) : McAt{-1, make_float2(0.f, 0.f)};
+    out[o + p] = mc_value<false>(x + o, q, p, W, 1.f);
   }
 }
 
-// out = M^T g (AdjointMotionCompensation: copy, zero the rectangle, scatter),
-// one thread per target, contributions in the reference's order; corner c of
-// an entry's square gets (g * fa) * fb with fa = Whh or 1 - Whh (c & 1), fb =
-// Wvv or 1 - Wvv (c & 2), as optimizer.cl:880-937 rounds them.  Loads of up to
-// four contributions are issued before any of them is accumulated.
-__global__ void __launch_bounds__(kNT) k_mc_adjoint(const float2* __restrict__ g, float2* __restrict__ out,
-                                                     const int* __restrict__ off, const int* __restrict__ csrc,
-                                                     const float2* __restrict__ cw, McRect r, int W, int H, int F,
-                                                     int pdl) {
+// out = M^T g (AdjointMotionCompensation: copy, zero the rectangle, scatter), one
+// thread per target (two targets' lists in one thread: 100 us more per solve); grid y: frames
+__global__ void __launch_bounds__(kNT) k_mc_adjoint(const float2* g, float2* __restrict__ out, McLists l, McRect r,
+                                                     int W, int HW, int F, int pdl) {
+  const int p = blockIdx.x * kNT + threadIdx.x;
   if (pdl) {
     grid_dep_wait();  // g comes from the fused tTV kernel two launches back
     grid_dep_release();
   }
-  const size_t HW = size_t(H) * W, n = HW * F;
-  const size_t q = blockIdx.x * size_t(kNT) + threadIdx.x;
-  if (q >= n) return;
-  const int p = int(q % HW), row = p / W, col = p % W;
+  if (p >= HW) return;
+  const int row = p / W, col = p - row * W;
   const bool in_rect = row >= r.r1b && row < r.r1b + r.l1 && col >= r.r2b && col < r.r2b + r.l2;
-  int c = __ldg(off + q);
-  const int ce = __ldg(off + q + 1);
-  float2 acc = in_rect ? make_float2(0.f, 0.f) : g[q];
-  const size_t k = q / HW;
-  const float2* gk = g + k * HW;
-  while (c < ce) {
-    const int m = min(4, ce - c);
-    float2 w[4], v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (u < m) {
-        w[u] = __ldg(cw + c + u);
-        v[u] = gk[__ldg(csrc + c + u)];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (u < m) {
-        acc.x = __fadd_rn(acc.x, __fmul_rn(__fmul_rn(v[u].x, w[u].x), w[u].y));
-        acc.y = __fadd_rn(acc.y, __fmul_rn(__fmul_rn(v[u].y, w[u].x), w[u].y));
-      }
-    }
-    c += m;
+  const bool moved = __ldg(l.moved) != 0;
+  for (int k = blockIdx.y; k < F; k += gridDim.y) {
+    const size_t o = size_t(k) * HW;
+    out[o + p] = mc_adjoint_at(l, g, o, p, in_rect, moved);
   }
-  out[q] = acc;
 }
 
 // g = tTVadj(normalise(D M x)) (temporalTV.cl:78-107 sign: u_{f+1} - u_f) and
@@ -401,15 +444,13 @@ __global__ void __launch_bounds__(kNT) k_mc_adjoint(const float2* __restrict__ g
 // outer loop's last iteration it does nothing, except in the launch that
 // recomputes the last update (row-local iteration, fixup), which reads x_last.
 __global__ void __launch_bounds__(kNT) k_mc_tv(const float2* __restrict__ x0, const float2* __restrict__ x1, int it,
-                                                const float* __restrict__ xn, const int* __restrict__ inv, McRect r,
-                                                const NestaDevState* __restrict__ st, float2* __restrict__ g,
-                                                double* __restrict__ part, int W, int H, int F,
-                                                int* __restrict__ status) {
+                                                McPoints m, const NestaDevState* __restrict__ st,
+                                                float2* __restrict__ g, double* __restrict__ part, int W, int H, int F) {
   __shared__ double sred[2 * kTvFrames][kNT / 32];
   const int HW = H * W;
   const int p = blockIdx.x * kNT + threadIdx.x;
   const bool live = p < HW;
-  const int e = live ? __ldg(inv + p) : -1;
+  const int xo = live ? __ldg(m.inv + p) : -1;
   const int f0 = blockIdx.y * kTvFrames, f1 = min(F, f0 + kTvFrames);
   grid_dep_wait();  // x_k comes from the previous iteration's update
   grid_dep_release();
@@ -426,36 +467,19 @@ __global__ void __launch_bounds__(kNT) k_mc_tv(const float2* __restrict__ x0, co
   for (int u = 0; u < kTvFrames; ++u) su2[u] = sud[u] = 0.f;
   if (live) {
     // M x_k at this pixel for frames f0-1 .. f1 (periodic): positions, then
-    // corners, then values, so that the loads of all frames are in flight together
+    // values, so that the loads of all frames are in flight together
     constexpr int NW = kTvFrames + 2;
     const int nw = f1 - f0 + 2;
-    int fr[NW];
-#pragma unroll
-    for (int u = 0; u < NW; ++u) fr[u] = (f0 - 1 + u + F) % F;
+    McAt q[NW];
     float2 w[NW];
-    if (e < 0) {
 #pragma unroll
-      for (int u = 0; u < NW; ++u)
-        if (u < nw) w[u] = x[size_t(fr[u]) * HW + p];
-    } else {
-      const int xo = entry_offset(r, e, W);
-      McPoint q[NW];
-#pragma unroll
-      for (int u = 0; u < NW; ++u)
-        if (u < nw) q[u] = mc_point(xn, xo, fr[u], W, H, F);
-#pragma unroll
-      for (int u = 0; u < NW; ++u) {
-        if (u < nw) {
-          const float2* xf = x + size_t(fr[u]) * HW;
-          if (q[u].ok) {
-            w[u] = bilinear(xf, q[u], W);
-          } else {
-            atomicExch(status, kStatusMotionRange);
-            w[u] = xf[p];
-          }
-        }
-      }
+    for (int u = 0; u < NW; ++u) {
+      q[u].at = -1;
+      if (xo >= 0 && u < nw) q[u] = mc_at(m, xo, size_t(wrap_frame(f0 - 1 + u, F)) * HW);
     }
+#pragma unroll
+    for (int u = 0; u < NW; ++u)
+      if (u < nw) w[u] = mc_value<false>(x + size_t(wrap_frame(f0 - 1 + u, F)) * HW, q[u], p, W, 1.f);
 #pragma unroll
     for (int u = 0; u < kTvFrames; ++u) {
       const int f = f0 + u;
@@ -515,9 +539,13 @@ int grid1(gbn_ctx* ctx, size_t n) { return int(std::min<size_t>((n + kNT - 1) / 
 // NestaUp.cpp:369-385) takes a third phase, which puts the drand48 vector in U x's
 // place.  x is stored unscaled; its scale 1/||x|| is applied as each value is read,
 // which rounds exactly as a separate scaling pass would.  Bound by the latency of the
-// gathers and barriers.
+// gathers out of L2 and of the barriers: at 256 x 256 x 20, 30 steps, 25 K and 33 K
+// cycles in the phases and 18 K at each barrier with its sums and the SMs' unevenness,
+// 1.4 ms (1.9 before with six launches a step; four frames a thread in phase 1 +70 us,
+// 512 threads +200, 1024 and the next item's loads ahead of this one's: nothing).
 constexpr int kNeFrames = 2;     // frames per thread of phase 1
-constexpr int kNeMaxGrid = 1024;
+constexpr int kNeNT = 768;        // threads of a CTA, one CTA per SM
+constexpr int kNeMaxGrid = 256;
 constexpr unsigned kNePolls = 1u << 22;
 constexpr float kNeTol = 1e-3f;
 constexpr int kNeMax = 100;
@@ -532,35 +560,14 @@ struct NeArgs {
   double* part;             // [3 phases][kNeMaxGrid][2]: sum of squares, any value not zero
   McNe* ne;
   NestaDevState* st;
-  const float* xn;
-  const int *inv, *off, *csrc;
-  const float2* cw;
+  McPoints m;
+  McLists l;
   McRect r;
   int W, H, F;
   float e;
   unsigned long long rand, ja, jc;  // drand48 state, and its jump by F*H*W draws
 };
 constexpr size_t kPartBytes = 3 * 2 * kNeMaxGrid * sizeof(double) + sizeof(McNe);
-
-// (M (s x))[k][p] for the stored, unscaled x.  What other CTAs of the launch write is
-// read through plain pointers, after a barrier's acquire.
-__device__ __forceinline__ float2 warp_scaled(const float2* xf, float sc, const McPoint& q, bool in_rect, int p, int W,
-                                             int* status) {
-  if (in_rect) {
-    if (q.ok) {
-      const float2* const c0 = xf + q.ph + size_t(q.pv) * W;
-      const float2* const c1 = c0 + W;
-      const float2 i1 = cscale(c0[0], sc), i2 = cscale(c0[1], sc), i3 = cscale(c1[0], sc), i4 = cscale(c1[1], sc);
-      const float a = float(q.ph + 1) - q.nh, b = q.nh - float(q.ph);
-      const float c = float(q.pv + 1) - q.nv, d = q.nv - float(q.pv);
-      const float2 aux1 = make_float2(lin2(a, i1.x, b, i2.x), lin2(a, i1.y, b, i2.y));
-      const float2 aux2 = make_float2(lin2(a, i3.x, b, i4.x), lin2(a, i3.y, b, i4.y));
-      return make_float2(lin2(c, aux1.x, d, aux2.x), lin2(c, aux1.y, d, aux2.y));
-    }
-    atomicExch(status, kStatusMotionRange);
-  }
-  return cscale(xf[p], sc);
-}
 
 // All CTAs of the launch; false if some did not arrive in time.
 __device__ __forceinline__ bool ne_barrier(McNe* ne, unsigned target) {
@@ -584,52 +591,51 @@ __device__ __forceinline__ bool ne_barrier(McNe* ne, unsigned target) {
 
 // The CTA's partial: FP32 within a thread's few values and a warp, FP64 over the warps.
 __device__ __forceinline__ void ne_put(double* part, float s2, bool any) {
-  __shared__ double sred[kNT / 32];
+  __shared__ float sred[kNeNT / 32];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s2 += __shfl_down_sync(0xffffffffu, s2, o);
-  if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = double(s2);
+  if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = s2;
   const int some = __syncthreads_or(any);
   if (threadIdx.x == 0) {
     double t = 0.0;
 #pragma unroll
-    for (int w = 0; w < kNT / 32; ++w) t += sred[w];
+    for (int w = 0; w < kNeNT / 32; ++w) t += double(sred[w]);
     part[2 * blockIdx.x] = t;
     part[2 * blockIdx.x + 1] = some ? 1.0 : 0.0;
   }
 }
-// The launch's sum of squares (FP64, one warp: its rate is a small fraction of FP32's
-// here) and whether any value was not zero, to all threads.
-__device__ __forceinline__ double ne_total(const double* part, bool* any) {
-  __shared__ double total;
+// The root of the launch's sum of squares, and whether any value was not zero.  FP64 by
+// one warp, its rate being a small fraction of FP32's here (the root by every thread:
+// 4.5 K cycles a step and phase).
+__device__ __forceinline__ float ne_total(const double* part, bool* any) {
+  __shared__ float root;
   __shared__ int some;
+  constexpr int NL = (kNeMaxGrid + 31) / 32;
   if (threadIdx.x < 32) {
-    double t = 0.0, v[4];
+    double2 v[NL];
+#pragma unroll
+    for (int u = 0; u < NL; ++u) {
+      const int b = 32 * u + int(threadIdx.x);
+      v[u] = b < int(gridDim.x) ? *reinterpret_cast<const double2*>(part + 2 * b) : make_double2(0.0, 0.0);
+    }
+    double t = 0.0;
     bool a = false;
-    for (int b0 = 0; b0 < int(gridDim.x); b0 += 128) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int b = b0 + 32 * u + int(threadIdx.x);
-        v[u] = 0.0;
-        if (b < int(gridDim.x)) {
-          const double2 d = *reinterpret_cast<const double2*>(part + 2 * b);
-          v[u] = d.x;
-          a |= d.y != 0.0;
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) t += v[u];
+    for (int u = 0; u < NL; ++u) {
+      t += v[u].x;
+      a |= v[u].y != 0.0;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
     a = __any_sync(0xffffffffu, a);
     if (threadIdx.x == 0) {
-      total = t;
+      root = float(sqrt(t));
       some = a;
     }
   }
   __syncthreads();
   *any = some != 0;
-  return total;
+  return root;
 }
 
 // draw i + 1 of the drand48 generator in state x0
@@ -648,10 +654,31 @@ __device__ __forceinline__ float ne_draw(unsigned long long x0, unsigned long lo
   return __double2float_rn(double((ra * x0 + rc) & mask) * 0x1p-48);
 }
 
-__global__ void __launch_bounds__(kNT, 4) k_normest(NeArgs n) {
+// a thread's walk over its CTA's share of (pixel p, frame or group of frames f) items
+struct NeItems {
+  int p, f, left;
+  __device__ __forceinline__ void share(long long items, int HW) {
+    const long long each = ((items + gridDim.x - 1) / gridDim.x + 31) / 32 * 32;
+    const long long i0 = each * blockIdx.x + threadIdx.x, i1 = min(items, each * (blockIdx.x + 1));
+    left = int(max(0LL, (i1 - i0 + kNeNT - 1) / kNeNT));
+    f = int(i0 / HW);
+    p = int(i0 - (long long)f * HW);
+  }
+  __device__ __forceinline__ void next(int HW) {
+    --left;
+    for (p += kNeNT; p >= HW; p -= HW) ++f;
+  }
+};
+
+__global__ void __launch_bounds__(kNeNT, 1) k_normest(NeArgs n) {
   const int W = n.W, H = n.H, F = n.F, HW = H * W;
-  const int npb = (HW + kNT - 1) / kNT, nfg = (F + kNeFrames - 1) / kNeFrames;
   const McRect r = n.r;
+  const bool moved = __ldg(n.l.moved) != 0;
+  // a CTA's share of phase 1's (pixel, kNeFrames frames) and phase 2's (pixel, frame)
+  // items: whole warps, so that every SM has the same work
+  NeItems it1, it2;
+  it1.share((long long)HW * ((F + kNeFrames - 1) / kNeFrames), HW);
+  it2.share((long long)HW * F, HW);
   unsigned long long rand = n.rand;
   float e = n.e, e0 = 0.f, sc = 1.0f / n.e;
   int cnt = 0, nrestart = 0;
@@ -660,93 +687,63 @@ __global__ void __launch_bounds__(kNT, 4) k_normest(NeArgs n) {
   while (fabsf(e - e0) > kNeTol * e && cnt < kNeMax) {
     float s2 = 0.f;
     bool nz = false;
-    for (int b = blockIdx.x; b < npb * nfg; b += gridDim.x) {
-      const int p = (b % npb) * kNT + threadIdx.x, f0 = (b / npb) * kNeFrames, nf = min(kNeFrames, F - f0);
-      if (p >= HW) continue;
-      const int ent = __ldg(n.inv + p);
-      const int xo = ent >= 0 ? entry_offset(r, ent, W) : 0;
+    for (NeItems i = it1; i.left > 0; i.next(HW)) {
       constexpr int NW = kNeFrames + 2;
-      int fr[NW];
-      McPoint q[NW];
+      const int f0 = i.f * kNeFrames, nf = min(kNeFrames, F - f0), xo = __ldg(n.m.inv + i.p);
+      McAt q[NW];
       float2 w[NW];
 #pragma unroll
-      for (int u = 0; u < NW; ++u) fr[u] = (f0 - 1 + u + F) % F;
+      for (int u = 0; u < NW; ++u) {
+        q[u].at = -1;
+        if (xo >= 0 && u < nf + 2) q[u] = mc_at(n.m, xo, size_t(wrap_frame(f0 - 1 + u, F)) * HW);
+      }
 #pragma unroll
       for (int u = 0; u < NW; ++u)
-        if (ent >= 0 && u < nf + 2) q[u] = mc_point(n.xn, xo, fr[u], W, H, F);
-#pragma unroll
-      for (int u = 0; u < NW; ++u)
-        if (u < nf + 2) w[u] = warp_scaled(n.x + size_t(fr[u]) * HW, sc, q[u], ent >= 0, p, W, &n.st->status);
+        if (u < nf + 2) w[u] = mc_value<true>(n.x + size_t(wrap_frame(f0 - 1 + u, F)) * HW, q[u], i.p, W, sc);
 #pragma unroll
       for (int u = 0; u < kNeFrames; ++u) {
         if (u < nf) {
-          const float2 a = csub(w[u + 1], w[u]);
-          s2 = fmaf(a.x, a.x, fmaf(a.y, a.y, s2));
-          nz |= fabsf(a.x) + fabsf(a.y) != 0.f;
-          n.g[size_t(f0 + u) * HW + p] = csub(csub(w[u + 2], w[u + 1]), a);
+          const float2 d = csub(w[u + 1], w[u]);
+          s2 = fmaf(d.x, d.x, fmaf(d.y, d.y, s2));
+          nz |= fabsf(d.x) + fabsf(d.y) != 0.f;
+          n.g[size_t(f0 + u) * HW + i.p] = csub(csub(w[u + 2], w[u + 1]), d);
         }
       }
     }
     double* part = n.part;
     ne_put(part, s2, nz);
     if (!ne_barrier(n.ne, (gen += gridDim.x))) return;
-    double t2 = ne_total(part, &any);
     e0 = e;
+    float root = ne_total(part, &any);
     if (!any) {  // uniform over the grid
       s2 = 0.f;
-      for (int b = blockIdx.x; b < npb * F; b += gridDim.x) {
-        const int p = (b % npb) * kNT + threadIdx.x, f = b / npb;
-        if (p >= HW) continue;
-        const float a = ne_draw(rand, (unsigned long long)f * HW + p);
+      for (NeItems i = it2; i.left > 0; i.next(HW)) {
+        const size_t o = size_t(i.f) * HW;
+        const float a = ne_draw(rand, o + i.p);
         s2 = fmaf(a, a, s2);
-        n.g[size_t(f) * HW + p] =
-            make_float2(__fsub_rn(ne_draw(rand, (unsigned long long)((f + 1) % F) * HW + p), a), 0.f);
+        n.g[o + i.p] =
+            make_float2(__fsub_rn(ne_draw(rand, (unsigned long long)wrap_frame(i.f + 1, F) * HW + i.p), a), 0.f);
       }
       part += 2 * kNeMaxGrid;
       ne_put(part, s2, false);
       if (!ne_barrier(n.ne, (gen += gridDim.x))) return;
-      t2 = ne_total(part, &any);
+      root = ne_total(part, &any);
       rand = (n.ja * rand + n.jc) & ((1ULL << 48) - 1);
       nrestart += 1;
     }
-    e = float(sqrt(t2));
+    e = root;
     s2 = 0.f;
-    for (int b = blockIdx.x; b < npb * F; b += gridDim.x) {
-      const int p = (b % npb) * kNT + threadIdx.x, f = b / npb;
-      if (p >= HW) continue;
-      const size_t t = size_t(f) * HW + p;
-      const float2* const gf = n.g + size_t(f) * HW;
-      const int row = p / W, col = p % W;
+    for (NeItems i = it2; i.left > 0; i.next(HW)) {
+      const int p = i.p, row = p / W, col = p - row * W;
       const bool in_rect = row >= r.r1b && row < r.r1b + r.l1 && col >= r.r2b && col < r.r2b + r.l2;
-      int c = __ldg(n.off + t);
-      const int ce = __ldg(n.off + t + 1);
-      float2 acc = in_rect ? make_float2(0.f, 0.f) : gf[p];
-      while (c < ce) {
-        const int m = min(4, ce - c);
-        float2 w[4], v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (u < m) {
-            w[u] = __ldg(n.cw + c + u);
-            v[u] = gf[__ldg(n.csrc + c + u)];
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (u < m) {
-            acc.x = __fadd_rn(acc.x, __fmul_rn(__fmul_rn(v[u].x, w[u].x), w[u].y));
-            acc.y = __fadd_rn(acc.y, __fmul_rn(__fmul_rn(v[u].y, w[u].x), w[u].y));
-          }
-        }
-        c += m;
-      }
-      n.x[t] = acc;
+      const float2 acc = mc_adjoint_at(n.l, n.g, size_t(i.f) * HW, p, in_rect, moved);
+      n.x[size_t(i.f) * HW + p] = acc;
       s2 = fmaf(acc.x, acc.x, fmaf(acc.y, acc.y, s2));
     }
     part = n.part + 4 * kNeMaxGrid;
     ne_put(part, s2, false);
     if (!ne_barrier(n.ne, (gen += gridDim.x))) return;
-    sc = 1.0f / float(sqrt(ne_total(part, &any)));
+    sc = 1.0f / ne_total(part, &any);
     cnt += 1;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -761,19 +758,24 @@ __global__ void __launch_bounds__(kNT, 4) k_normest(NeArgs n) {
 // host side
 // ---------------------------------------------------------------------------
 void tables_free(McTables* t) {
-  void* ptrs[] = {t->inv, t->cnt, t->off, t->bsum, t->key, t->srcmap, t->wts, t->tvpart, t->csrc, t->cw};
+  void* ptrs[] = {t->inv, t->cnt, t->off, t->bsum, t->key, t->srcmap, t->at, t->wts, t->tvpart};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   *t = McTables{};
 }
 
+dim3 frame_grid(int HW, int F) { return dim3((HW + kNT - 1) / kNT, std::min(F, 65535)); }
+McPoints points_of(const McTables& t) { return {t.inv, t.at, t.wts}; }
+McLists lists_of(const McTables& t) { return {t.off, t.key, t.srcmap, t.srcmap + t.hw, t.wts}; }
+
 // buffers for F*H*W pixels and E rectangle entries (kept when large enough)
 int tables_alloc(McTables* t, int W, int H, int F, int E) {
   const size_t HW = size_t(H) * W, X = HW * F;
   const int nbp = int((HW + kNT - 1) / kNT);
-  if (t->inv && t->x == X && size_t(E) <= t->entries) return GBN_OK;
+  if (t->inv && t->x == X && t->hw == HW && size_t(E) <= t->entries) return GBN_OK;
   tables_free(t);
   t->x = X;
+  t->hw = HW;
   t->entries = size_t(E);
   t->nbp = nbp;
   t->nscan = int((X + kScanBlock - 1) / kScanBlock);
@@ -782,11 +784,10 @@ int tables_alloc(McTables* t, int W, int H, int F, int E) {
   if (e == cudaSuccess) e = cudaMalloc(&t->off, (X + 1) * sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&t->bsum, size_t(t->nscan) * sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&t->key, 4 * size_t(E) * F * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&t->srcmap, HW * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&t->srcmap, (HW + 1) * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&t->at, X * sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&t->wts, X * sizeof(float2));
   if (e == cudaSuccess) e = cudaMalloc(&t->tvpart, 2 * size_t(F) * nbp * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&t->csrc, 4 * size_t(E) * F * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&t->cw, 4 * size_t(E) * F * sizeof(float2));
   if (e != cudaSuccess) {
     cudaGetLastError();
     tables_free(t);
@@ -801,20 +802,20 @@ int tables_build(gbn_ctx* ctx, McTables* t, const float* xn, const int* xm, cons
   const size_t HW = size_t(H) * W, X = HW * F;
   const int E = r.l1 * r.l2;
   cudaError_t e = cudaMemsetAsync(t->inv, 0xFF, HW * sizeof(int), s);  // -1
+  if (e == cudaSuccess) e = cudaMemsetAsync(t->srcmap + HW, 0, sizeof(int), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(t->cnt, 0, X * sizeof(int), s);
   if (e != cudaSuccess) return cuda_status(e, "motion compensation tables");
-  k_mc_inv<<<grid1(ctx, size_t(E)), kNT, 0, s>>>(xm, r, W, H, t->inv, t->srcmap, status);
-  k_mc_count<<<grid1(ctx, size_t(E) * F), kNT, 0, s>>>(xn, xm, r, W, H, F, t->cnt, status);
+  k_mc_inv<<<grid1(ctx, size_t(E)), kNT, 0, s>>>(xm, r, W, H, t->inv, t->srcmap, t->srcmap + HW, status);
+  const dim3 ge((E + kNT - 1) / kNT, std::min(F, 65535)), gx(unsigned((HW + kNT - 1) / kNT), std::min(F, 65535));
+  k_mc_count<<<ge, kNT, 0, s>>>(xn, t->srcmap, r, W, H, F, t->cnt, status);
   k_scan_blocks<<<t->nscan, kNT, 0, s>>>(t->cnt, X, t->off, t->bsum);
   k_scan_totals<<<1, 1024, 0, s>>>(t->bsum, t->nscan, t->off, X);
   k_scan_add<<<t->nscan, kNT, 0, s>>>(t->off, X, t->bsum);
   if ((e = cudaMemsetAsync(t->cnt, 0, X * sizeof(int), s)) != cudaSuccess)
     return cuda_status(e, "motion compensation tables");
-  k_mc_fill<<<grid1(ctx, size_t(E) * F), kNT, 0, s>>>(xn, xm, r, W, H, F, t->off, t->cnt, t->key, t->wts);
-  k_mc_sort<<<grid1(ctx, X), kNT, 0, s>>>(t->off, t->key, X);
-  k_mc_rekey<<<grid1(ctx, 4 * size_t(E) * F), kNT, 0, s>>>(t->key, t->off + X, r, W);
-  k_mc_pack<<<grid1(ctx, X), kNT, 0, s>>>(t->off, t->key, t->srcmap, t->wts, t->csrc, t->cw, X, HW);
-  ctx->launches += 10;
+  k_mc_fill<<<ge, kNT, 0, s>>>(xn, t->srcmap, r, W, H, F, t->off, t->cnt, t->key, t->at, t->wts);
+  k_mc_lists<<<gx, kNT, 0, s>>>(t->off, t->key, t->inv, r, W, int(HW), F);
+  ctx->launches += 7;
   return GBN_OK;
 }
 
@@ -868,9 +869,9 @@ namespace {
 
 // out = M in
 void mc_apply(gbn_ctx* ctx, gbn_problem* P, const float2* in, float2* out, cudaStream_t s) {
-  const size_t X = size_t(P->W) * P->H * P->F;
   const McRect r = mc_rect(P->W, P->H, P->mc_bb);
-  k_mc_warp<<<grid1(ctx, X), kNT, 0, s>>>(in, out, P->mc_xn, P->mc_tab->inv, r, P->W, P->H, P->F, &P->st->status);
+  const int HW = P->W * P->H;
+  k_mc_warp<<<frame_grid(HW, P->F), kNT, 0, s>>>(in, out, points_of(*P->mc_tab), P->W, HW, P->F);
   ctx->launches += 1;
 }
 
@@ -879,25 +880,14 @@ int mc_normest(gbn_ctx* ctx, gbn_problem* P, cudaStream_t s) {
   const size_t X = size_t(P->W) * P->H * P->F;
   const McTables* t = P->mc_tab;
   const Lcg48 jX = lcg48_jump(uint64_t(X));
-  static const int per_sm = [] {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_normest, kNT, 0) != cudaSuccess) {
-      cudaGetLastError();
-      n = 1;
-    }
-    return n;
-  }();
   NeArgs n{};
   n.x = P->mc_gm;
   n.g = P->mc_g;
   n.part = P->mc_part;
   n.ne = reinterpret_cast<McNe*>(P->mc_part + 3 * 2 * kNeMaxGrid);
   n.st = P->st;
-  n.xn = P->mc_xn;
-  n.inv = t->inv;
-  n.off = t->off;
-  n.csrc = t->csrc;
-  n.cw = t->cw;
+  n.m = points_of(*t);
+  n.l = lists_of(*t);
   n.r = mc_rect(P->W, P->H, P->mc_bb);
   n.W = P->W;
   n.H = P->H;
@@ -906,14 +896,14 @@ int mc_normest(gbn_ctx* ctx, gbn_problem* P, cudaStream_t s) {
   n.rand = (unsigned long long)ctx->rand48;
   n.ja = (unsigned long long)jX.a;
   n.jc = (unsigned long long)jX.c;
-  // every CTA of the launch is resident
-  const size_t blocks = size_t((P->W * P->H + kNT - 1) / kNT) * P->F;
-  const int grid = int(std::min<size_t>(std::min(kNeMaxGrid, ctx->nsm * per_sm), blocks));
+  // every CTA of the launch is resident: one per SM
+  const size_t items = size_t(P->W) * P->H * ((P->F + kNeFrames - 1) / kNeFrames);
+  const int grid = int(std::min<size_t>(std::min(kNeMaxGrid, ctx->nsm), (items + kNeNT - 1) / kNeNT));
   cudaError_t e = cudaMemsetAsync(n.ne, 0, sizeof(McNe), s);
   if (e != cudaSuccess) return cuda_status(e, "power method");
   k_fill<<<grid1(ctx, X), kNT, 0, s>>>(n.x, X, make_float2(1.f, 0.f));
   void* args[] = {&n};
-  e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_normest), dim3(grid), dim3(kNT), args, 0, s);
+  e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_normest), dim3(grid), dim3(kNeNT), args, 0, s);
   ctx->launches += 2;
   McNe h{};
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h, n.ne, sizeof(h), cudaMemcpyDeviceToHost, s);
@@ -945,11 +935,10 @@ int motion_op(gbn_ctx* ctx, int dir, const float2* in, float2* out, const float*
   if (e != cudaSuccess) rc = cuda_status(e, "motion compensation");
   if (rc == GBN_OK) rc = tables_build(ctx, &t, xn, xm, r, W, H, F, status, s);
   if (rc == GBN_OK) {
-    const size_t X = size_t(W) * H * F;
     if (dir == GBN_TTV_FORWARD)
-      k_mc_warp<<<grid1(ctx, X), kNT, 0, s>>>(in, out, xn, t.inv, r, W, H, F, status);
+      k_mc_warp<<<frame_grid(W * H, F), kNT, 0, s>>>(in, out, points_of(t), W, W * H, F);
     else
-      k_mc_adjoint<<<int((X + kNT - 1) / kNT), kNT, 0, s>>>(in, out, t.off, t.csrc, t.cw, r, W, H, F, 0);
+      k_mc_adjoint<<<frame_grid(W * H, F), kNT, 0, s>>>(in, out, lists_of(t), r, W, W * H, F, 0);
     ctx->launches += 1;
   }
   int h = 0;
@@ -981,7 +970,7 @@ int nesta_run_mc(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, floa
   const int g2 = row_grid(ctx, kw, true, steps, k2);
   const dim3 g3(W / kWB, 2, F);
   const dim3 gtv(t->nbp, (F + kTvFrames - 1) / kTvFrames);
-  const int gadj = int((size_t(W) * H * F + kNT - 1) / kNT);
+  const dim3 gadj = frame_grid(W * H, F);
   FusedArgs a = make_args(P, x_out);
   a.tv_src = P->mc_xw;  // marks the motion-compensated form: the forward pass skips its tTV sums
   a.grad_ext = P->mc_gm;
@@ -1045,10 +1034,8 @@ int nesta_run_mc(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, floa
       }
       for (unsigned it = 0; it < n_iter_launch; ++it) {
         launch_pdl(k_mc_tv, gtv, kNT, 0, s, (const float2*)P->xk0, (const float2*)P->xk1, int(it),
-                   (const float*)P->mc_xn, (const int*)t->inv, r, (const NestaDevState*)P->st, P->mc_g, t->tvpart, W,
-                   H, F, &P->st->status);
-        launch_pdl(k_mc_adjoint, dim3(gadj), kNT, 0, s, (const float2*)P->mc_g, P->mc_gm, (const int*)t->off,
-                   (const int*)t->csrc, (const float2*)t->cw, r, W, H, F, 1);
+                   points_of(*t), (const NestaDevState*)P->st, P->mc_g, t->tvpart, W, H, F);
+        launch_pdl(k_mc_adjoint, gadj, kNT, 0, s, (const float2*)P->mc_g, P->mc_gm, lists_of(*t), r, W, W * H, F, 1);
         GBN_LAUNCH(ctx, GBN_PROF_ITER, 1, kh->iter_cols(tab, bm, int(it), true, g3, s));
         ctx->launches += 2;
       }
@@ -1063,10 +1050,9 @@ int nesta_run_mc(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, floa
     for (unsigned it = 0; it < prm->maxIter; ++it) {
       cudaEventRecord(ctx->ev_mc_x, s);
       cudaStreamWaitEvent(aux, ctx->ev_mc_x, 0);
-      k_mc_tv<<<gtv, kNT, 0, aux>>>(P->xk0, P->xk1, int(it), P->mc_xn, t->inv, r, P->st, P->mc_g, t->tvpart, W, H, F,
-                                    &P->st->status);
+      k_mc_tv<<<gtv, kNT, 0, aux>>>(P->xk0, P->xk1, int(it), points_of(*t), P->st, P->mc_g, t->tvpart, W, H, F);
       cudaEventRecord(ctx->ev_mc_tv, aux);
-      k_mc_adjoint<<<gadj, kNT, 0, aux>>>(P->mc_g, P->mc_gm, t->off, t->csrc, t->cw, r, W, H, F, 0);
+      k_mc_adjoint<<<gadj, kNT, 0, aux>>>(P->mc_g, P->mc_gm, lists_of(*t), r, W, W * H, F, 0);
       cudaEventRecord(ctx->ev_mc_adj, aux);
       kh->fwd_cols(tab, bm, int(it), cpb, g1, s);
       cudaStreamWaitEvent(s, ctx->ev_mc_tv, 0);
