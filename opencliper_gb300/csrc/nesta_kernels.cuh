@@ -187,6 +187,15 @@ __global__ void __launch_bounds__(kColNT, fwd_min_blocks(H))
   issue_S(c0, 0);
 
   for (int i = t; i < H; i += kColNT) rmap[i] = a.rowmap[f * H + i];
+  // inter-pass twiddles of this thread's pass-1 items, identical for every coil
+  float2 twr[NI1][A];
+#pragma unroll
+  for (int ii = 0; ii < NI1; ++ii) {
+    const int i = t + ii * kColNT;
+    const int s = (i < N1) ? i / kWB : 0;
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) twr[ii][k1] = __ldg(a.twH + k1 * B + s);
+  }
   const int rowbase = a.rowoff[f];
   grid_dep_wait();  // x_k comes from the previous adjoint column pass
   grid_dep_release();
@@ -226,16 +235,6 @@ __global__ void __launch_bounds__(kColNT, fwd_min_blocks(H))
         }
       }
     }
-  }
-
-  // inter-pass twiddles of this thread's pass-1 items, identical for every coil
-  float2 twr[NI1][A];
-#pragma unroll
-  for (int ii = 0; ii < NI1; ++ii) {
-    const int i = t + ii * kColNT;
-    const int s = (i < N1) ? i / kWB : 0;
-#pragma unroll
-    for (int k1 = 0; k1 < A; ++k1) twr[ii][k1] = __ldg(a.twH + k1 * B + s);
   }
 
   for (int c = c0; c < c1; ++c) {
@@ -646,8 +645,9 @@ struct InvColsSmem {
   static_assert(cdiv(kWB * B, kColNT) * A * kColNT <= 2 * H * kWB, "accumulator exchange must fit the S buffers");
 };
 
+constexpr bool inv_prefetch(int H) { return cdiv(kWB * split_a(H), kColNT) == 1 && split_a(H) <= 16; }
 template <int H, bool UPDATE>
-__global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT)
+__global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT, inv_prefetch(H) ? 3 : 1)
     k_inv_cols(const FusedArgs* __restrict__ tab, const __grid_constant__ BatchMap bm, int it) {
   using L = InvColsSmem<H>;
   constexpr int A = L::A, B = L::B, KS = L::KS, RCAP = L::RCAP;
@@ -694,22 +694,6 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT)
   };
   if (cbeg < cend) issue_S(cbeg, 0);
   for (int i = t; i < H; i += kColNT) rmap[i] = a.rowmap[f * H + i];
-  grid_dep_wait();  // T and the scalar state come from the row pass
-  grid_dep_release();
-  if (UPDATE && it > st->last_iter) {  // uniform over the instance, so over each cluster
-    cp_async_commit();
-    cp_async_wait<0>();
-    return;
-  }
-  if (cbeg < cend) issue_T(cbeg, 0);
-  cp_async_commit();
-
-  float2 acc[NI2][A];
-#pragma unroll
-  for (int ii = 0; ii < NI2; ++ii)
-#pragma unroll
-    for (int k2 = 0; k2 < A; ++k2) acc[ii][k2] = make_float2(0.f, 0.f);
-  __syncthreads();
   // inter-pass twiddles of this thread's pass-1 items, identical for every coil
   float2 twr[NI1][B];
 #pragma unroll
@@ -719,6 +703,41 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT)
 #pragma unroll
     for (int k1p = 0; k1p < B; ++k1p) twr[ii][k1p] = __ldg(a.twH + H + k1p * A + s);
   }
+  grid_dep_wait();  // T and the scalar state come from the row pass
+  grid_dep_release();
+  if (UPDATE && it > st->last_iter) {  // uniform over the instance, so over each cluster
+    cp_async_commit();
+    cp_async_wait<0>();
+    return;
+  }
+  if (cbeg < cend) issue_T(cbeg, 0);
+  cp_async_commit();
+  // Frames that keep more rows than the shared buffers hold: the next coil's values
+  // travel to registers while this one is transformed, where a thread has one item and
+  // its state leaves room.  With the bound of three CTAs per SM: at two, without it, a
+  // solve is 6 % slower than with no prefetch, at three 2 % faster (pixel masks, 20
+  // iterations: 240 x 224 x 12, 8 coils 1475 -> 1441 us, 256 x 240 x 24, 16 coils 4022 ->
+  // 3963).
+  constexpr bool PREF = inv_prefetch(H);
+  float2 tn[PREF ? B : 1];
+  auto fetch_T = [&](int c) {
+    if constexpr (PREF) {
+      const int w = t % kWB, s = t / kWB;
+#pragma unroll
+      for (int n1 = 0; n1 < B; ++n1) {
+        const int j = t < N1 ? rmap[A * n1 + s] : -1;
+        tn[n1] = j >= 0 ? a.T[(size_t(rowbase + j) * C + c) * W + w0 + w] : make_float2(0.f, 0.f);
+      }
+    }
+  };
+
+  float2 acc[NI2][A];
+#pragma unroll
+  for (int ii = 0; ii < NI2; ++ii)
+#pragma unroll
+    for (int k2 = 0; k2 < A; ++k2) acc[ii][k2] = make_float2(0.f, 0.f);
+  __syncthreads();
+  if (PREF && !staged && cbeg < cend) fetch_T(cbeg);
 
   for (int c = cbeg; c < cend; ++c) {
     const int buf = (c - cbeg) & 1;
@@ -736,16 +755,22 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT)
       const int i = t + ii * kColNT;
       if (i < N1) {
         const int w = i % kWB, s = i / kWB;
-        int jv[B];
-#pragma unroll
-        for (int n1 = 0; n1 < B; ++n1) jv[n1] = rmap[A * n1 + s];
         float2 v[B];
+        if (PREF && !staged) {
 #pragma unroll
-        for (int n1 = 0; n1 < B; ++n1) {
-          float2 e = make_float2(0.f, 0.f);
-          if (jv[n1] >= 0)
-            e = staged ? Tc[jv[n1] * kWB + w] : a.T[(size_t(rowbase + jv[n1]) * C + c) * W + w0 + w];
-          v[n1] = conjf2(e);
+          for (int n1 = 0; n1 < B; ++n1) v[n1] = conjf2(tn[PREF ? n1 : 0]);
+          if (c + 1 < cend) fetch_T(c + 1);
+        } else {
+          int jv[B];
+#pragma unroll
+          for (int n1 = 0; n1 < B; ++n1) jv[n1] = rmap[A * n1 + s];
+#pragma unroll
+          for (int n1 = 0; n1 < B; ++n1) {
+            float2 e = make_float2(0.f, 0.f);
+            if (jv[n1] >= 0)
+              e = staged ? Tc[jv[n1] * kWB + w] : a.T[(size_t(rowbase + jv[n1]) * C + c) * W + w0 + w];
+            v[n1] = conjf2(e);
+          }
         }
         dft<B>(v);
 #pragma unroll
