@@ -29,9 +29,9 @@ struct SizeKernels {
                    cudaStream_t s);
   void (*adj_cols)(const float2* T, const float2* S, float2* x, int W, int C, int F, float scale, const float2* tw,
                    int cs, cudaStream_t s);
-  // row-local inner iteration (k_iter_cols<L, motion>), grid (W/8, 2, total
-  // frames) in clusters of 2; nullptr for lengths that run only the three-pass
-  // iteration
+  // row-local inner iteration: k_iter_pair<L, motion> where pair_cols, else
+  // k_iter_cols<L, motion> on grid (W/8, 2, total frames) in clusters of 2; nullptr
+  // for lengths that run only the three-pass iteration
   void (*iter_cols)(const FusedArgs* tab, const BatchMap& bm, int it, bool motion, dim3 grid, cudaStream_t s);
   // the sums and scalar step of iteration it - 1 alone (column-pair form)
   void (*iter_finish)(const FusedArgs* tab, const BatchMap& bm, int it, dim3 grid, cudaStream_t s);

@@ -2,7 +2,7 @@
 SimpleMRIRecon, SimpleMRIReconSOS) where their work splits unevenly, against the
 FP64 operators: coil counts around the CTAs of a cluster (1, 2, 3, 5, 9), lengths
 with one and several items per thread and with a first factor past 32 (504 = 63 x 8),
-partly sampled rows, and a series that goes in chunks of frames.  The
+partly sampled rows, and a series of several coil groups.  The
 per-operator bar of test_ops_gpu.py (1e-5; an FFT of these lengths rounds at
 ~1e-7)."""
 from __future__ import annotations
