@@ -97,15 +97,13 @@ struct Launchers {
     }
   }
   static void fft_rows(const float2* in, float2* out, int nrows, int inv, float scale, const float2* tw,
-                       const uint8_t* mask, int C, int H, int grid, cudaStream_t s) {
-    if (mask)
-      k_fft_rows_dense<L, true><<<grid, kRowNT, 0, s>>>(in, out, nrows, inv, scale, tw, mask, C, H);
-    else
-      k_fft_rows_dense<L, false><<<grid, kRowNT, 0, s>>>(in, out, nrows, inv, scale, tw, mask, C, H);
+                       const uint8_t* mask, int C, int H, int grid, bool first, cudaStream_t s) {
+    launch_chain(first, mask ? k_fft_rows_dense<L, true> : k_fft_rows_dense<L, false>, dim3(grid), kRowNT, 0, s, in, out,
+                 nrows, inv, scale, tw, mask, C, H);
   }
   static void fft_cols(const float2* in, float2* out, int W, int nimg, int inv, float scale, const float2* tw,
                        cudaStream_t s) {
-    k_fft_cols_dense<L><<<dim3(W / kWB, nimg), kColNT, 0, s>>>(in, out, W, inv, scale, tw);
+    launch_pdl(k_fft_cols_dense<L>, dim3(W / kWB, nimg), kColNT, 0, s, in, out, W, inv, scale, tw);
   }
   static void enc_cols(const float2* x, const float2* S, float2* out, int W, int C, int F, const float2* tw,
                        cudaStream_t s) {

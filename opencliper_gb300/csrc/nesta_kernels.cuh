@@ -946,6 +946,7 @@ __global__ void __launch_bounds__(kRowNT) k_fft_rows_dense(const float2* in, flo
   const int t = threadIdx.x;
   for (int i = t; i < W; i += kRowNT) tw[i] = twW[i];
   __syncthreads();
+  grid_dep_wait();  // E: its columns come before
   const float sg = inv ? -1.f : 1.f;
   for (int base = blockIdx.x * RPC; base < nrows; base += gridDim.x * RPC) {
     for (int i = t; i < RPC * B; i += kRowNT) {
@@ -1010,6 +1011,7 @@ __global__ void __launch_bounds__(kColNT, cols_dense_blocks(H))
   const float2* const src = in + off;
   for (int i = t; i < H; i += kColNT) tw[i] = twH[i];
   __syncthreads();
+  grid_dep_wait();
   const float sg = inv ? -1.f : 1.f;
   for (int i = t; i < N1; i += kColNT) {
     const int w = i % kWB, s = i / kWB;
@@ -1053,6 +1055,7 @@ __global__ void __launch_bounds__(kColNT) k_enc_cols(const float2* in, const flo
   const int w0 = blockIdx.x * kWB;
   const int c0 = blockIdx.y * kEncCoils, c1 = min(C, c0 + kEncCoils);
   const size_t N = size_t(H) * W;
+  grid_dep_release();  // the row pass waits for this grid before it reads `out`
   for (int i = t; i < H; i += kColNT) tw[i] = twH[i];
   float2 xv[NI1][A], sv[NI1][A];
   auto fetch = [&](float2 (*v)[A], const float2* src) {

@@ -265,11 +265,11 @@ int op_abs(gbn_ctx* ctx, const float2* in, float2* out, size_t n, int squared) {
 }
 
 static int rows_pass(gbn_ctx* ctx, const float2* in, float2* out, int W, int H, long long nrows, int inv, float scale,
-                     const uint8_t* mask, int C) {
+                     const uint8_t* mask, int C, bool first = true) {
   if (nrows > 0x7fffffff) return set_error(GBN_ERR_UNSUPPORTED, "too many rows for one transform");
   const SizeKernels* kw = find_size(W);
   const int g = int((nrows + kw->rows_per_cta - 1) / kw->rows_per_cta);
-  kw->fft_rows(in, out, int(nrows), inv, scale, ctx_twiddles(ctx, W), mask, C, H, g, ctx->stream);
+  kw->fft_rows(in, out, int(nrows), inv, scale, ctx_twiddles(ctx, W), mask, C, H, g, first, ctx->stream);
   ctx->launches += 1;
   return GBN_OK;
 }
@@ -303,7 +303,7 @@ int op_encode(gbn_ctx* ctx, const float2* x, const float2* S, const uint8_t* mas
   const float scale = float(1.0 / std::sqrt(double(unsigned(W * H))));
   kh->enc_cols(x, S, k, W, C, F, ctx_twiddles(ctx, H), ctx->stream);
   ctx->launches += 1;
-  const int rc = rows_pass(ctx, k, k, W, H, (long long)F * C * H, 0, scale, mask, C);
+  const int rc = rows_pass(ctx, k, k, W, H, (long long)F * C * H, 0, scale, mask, C, false);
   if (rc != GBN_OK) return rc;
   return cuda_status(cudaGetLastError(), "encode");
 }
