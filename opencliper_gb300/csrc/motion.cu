@@ -869,7 +869,6 @@ namespace {
 
 // out = M in
 void mc_apply(gbn_ctx* ctx, gbn_problem* P, const float2* in, float2* out, cudaStream_t s) {
-  const McRect r = mc_rect(P->W, P->H, P->mc_bb);
   const int HW = P->W * P->H;
   k_mc_warp<<<frame_grid(HW, P->F), kNT, 0, s>>>(in, out, points_of(*P->mc_tab), P->W, HW, P->F);
   ctx->launches += 1;
