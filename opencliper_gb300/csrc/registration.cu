@@ -43,6 +43,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "reg_sums.h"
 
 namespace gbn {
 
@@ -315,7 +316,7 @@ struct RegArgs {
   float* sterm;  // [F][2][7][box pixels] weighted squared smoothness terms
   float* H;    // [nmax + 1]
   float* part_h;  // per-CTA partial sums of the metric (k_reg_metric)
-  float* part_d;  // per-CTA partial sums of Dif^2 (k_reg_update)
+  float* part_d;  // per-CTA partial sums of Dif^2 (k_reg_update; k_reg_solve: two sets, reg_sums.h)
   RegState* st;
 };
 
@@ -887,8 +888,10 @@ __global__ void __launch_bounds__(kRegNT, 2) k_reg_solve(RegSolve s) {
       const int nh = (s.L * s.L + kRegNT - 1) / kRegNT;
       float h = 0.f, dd = 0.f;
       for (int q = t; q < nh; q += kRegNT) h = h + __ldcg(a.part_h + q);
-      if (it > 1)
-        for (int q = t; q < s.gu; q += kRegNT) dd = dd + __ldcg(a.part_d + q);
+      if (it > 1) {
+        const float* const part = a.part_d + reg_dif_at(it - 1, s.gu);
+        for (int q = t; q < s.gu; q += kRegNT) dd = dd + __ldcg(part + q);
+      }
       reg_solve_scalars(s, it - 1, h, dd, sw, &ss);
       if (ss.done) {
         fin = it - 1;
@@ -898,6 +901,7 @@ __global__ void __launch_bounds__(kRegNT, 2) k_reg_solve(RegSolve s) {
     const float Wn = ss.Wn;
     if (it > 0) {
       float* const Tnew = s.Tb[it & 1];
+      float* const part = a.part_d + reg_dif_at(it, s.gu);
       // k_reg_update's blocks, from the CTAs that have no tile
       for (int b = int(gridDim.x - 1 - blockIdx.x); b < s.gu; b += gridDim.x) {
         const int q = b * kRegNT + t;
@@ -920,7 +924,7 @@ __global__ void __launch_bounds__(kRegNT, 2) k_reg_solve(RegSolve s) {
           dd = dif * dif;
         }
         const float v = reg_block_sum(dd, sw);
-        if (t == 0) a.part_d[b] = v;
+        if (t == 0) part[b] = v;
         __syncthreads();
       }
     }
@@ -1125,7 +1129,7 @@ int registration_run(gbn_ctx* ctx, const float2* images, int N, int F, const gbn
     dH = c.take<float>(nT);
     H = c.take<float>(size_t(prm->nmax) + 1);
     part_h = c.take<float>(L2 / kRegNT + 1);
-    part_d = c.take<float>(nT / kRegNT + 1);
+    part_d = c.take<float>(solve ? reg_dif_floats(gu) : gu);
     if (solve) {
       sv.Tb[1] = c.take<float>(nT);
       sv.hv = c.take<float>(L2);
