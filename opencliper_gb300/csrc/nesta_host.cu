@@ -737,32 +737,32 @@ int problem_fit_rows(gbn_problem* P, int headroom, int* kept) {
     if ((e = cudaMemcpyAsync(&g, P->rowoff + P->F, sizeof(int), cudaMemcpyDeviceToHost, s)) == cudaSuccess &&
         (e = cudaStreamSynchronize(s)) == cudaSuccess) {
       const size_t want = std::min<size_t>(size_t(P->F) * P->H, size_t(g) + size_t(headroom));
-      if (want != saved) {
-        float2* nt = nullptr;
-        if ((e = cudaMalloc(&nt, std::max<size_t>(want, 1) * P->C * P->W * sizeof(float2))) == cudaSuccess) {
+      // the tiles follow: never more than the row-local iteration takes
+      const SizeKernels* kh = find_size(P->H);
+      const size_t tt = kh && kh->pair_cols
+                            ? std::min<size_t>(want, size_t(P->F) * std::min(P->H, iter_cols_rcap(P->H)))
+                            : 0;
+      // both buffers before either is given back: a failure leaves the problem as it was
+      const size_t row = size_t(P->C) * P->W;
+      float2* nt = nullptr;
+      float4* ntt = nullptr;
+      if (want != saved) e = cudaMalloc(&nt, std::max<size_t>(want, 1) * row * sizeof(float2));
+      if (e == cudaSuccess && tt != P->Tt_rows) e = cudaMalloc(&ntt, std::max<size_t>(tt, 1) * row * sizeof(float2));
+      if (e == cudaSuccess) {
+        if (nt) {
           cudaFree(P->T);
           P->T = nt;
-          P->T_rows = want;
-          // the tiles follow: never more than the row-local iteration takes
-          const size_t tt = std::min<size_t>(want, size_t(P->F) * std::min(P->H, iter_cols_rcap(P->H)));
-          if (P->Tt && tt != P->Tt_rows) {
-            cudaFree(P->Tt);
-            P->Tt = nullptr;
-            P->Tt_rows = 0;
-            if ((e = cudaMalloc(&P->Tt, std::max<size_t>(tt, 1) * P->C * P->W * sizeof(float2))) != cudaSuccess) {
-              cudaGetLastError();
-              return set_error(GBN_ERR_NOMEM, "row buffer allocation failed");
-            }
-            P->Tt_rows = tt;
-          }
-          if (kept) *kept = g;
-          return GBN_OK;
         }
-      } else {
-        P->T_rows = saved;
+        if (ntt) {
+          cudaFree(P->Tt);
+          P->Tt = ntt;
+          P->Tt_rows = tt;
+        }
+        P->T_rows = want;
         if (kept) *kept = g;
         return GBN_OK;
       }
+      if (nt) cudaFree(nt);
     }
   }
   P->T_rows = saved;
