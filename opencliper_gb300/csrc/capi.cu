@@ -143,6 +143,9 @@ int prof_collect(gbn_ctx* ctx) {
 
 int ctx_scratch(gbn_ctx* ctx, size_t bytes, void** out) {
   ctx->simple_plan = gbn_ctx::SimplePlan{};
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess) cudaGetLastError();
+  ctx->scratch_in_graph = ctx->scratch_in_graph || cap != cudaStreamCaptureStatusNone;
   if (bytes > ctx->scratch_bytes) {
     if (ctx->scratch) {
       cudaStreamSynchronize(ctx->stream);

@@ -38,6 +38,7 @@ struct gbn_ctx {
     const void* ws = nullptr;
     int W = 0, H = 0, F = 0, C = 0;
   } simple_plan;
+  bool scratch_in_graph = false;      // a captured call uses the scratch: replays write it unseen
   int k1_coils_per_block = 4;         // tuning: coils per CTA in the forward column pass
   int k2_ctas_per_sm = 4;             // tuning: persistent CTAs per SM in the row pass
   int mixed_adjoint_tc = 0;           // tuning: mixed form runs the adjoint column pass on the tensor cores

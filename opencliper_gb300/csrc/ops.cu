@@ -343,6 +343,10 @@ __global__ void k_stage_twiddles(const float2* __restrict__ tw, float2* __restri
 // SimpleMRIRecon: x = sum_c conj(S_c) ifft2(y_c).  Its column twiddles lie beside
 // the intermediates in the scratch, put there by the first call of a shape or
 // after another user of the scratch; further calls launch the two passes alone.
+// Once a call that uses the scratch has been captured into a graph, what the
+// scratch holds is no longer known here (a captured call has not run, a replay
+// overwrites it): from then on, and in the captured call itself, the context's
+// own table serves.
 int simple_recon(gbn_ctx* ctx, const float2* y, const float2* S, float2* x, int W, int H, int F, int C) {
   if (!find_size(H) || !find_size(W)) return set_error(GBN_ERR_UNSUPPORTED, "unsupported FFT length");
   gbn_ctx::SimplePlan& p = ctx->simple_plan;
@@ -352,12 +356,14 @@ int simple_recon(gbn_ctx* ctx, const float2* y, const float2* S, float2* x, int 
   const int rc = ctx_scratch(ctx, tb + simple_recon_bytes(W, H, F, C), &scr);  // forgets the plan
   if (rc != GBN_OK) return rc;
   float2* const tw = static_cast<float2*>(scr);
-  if (had.ws != scr || had.W != W || had.H != H || had.F != F || had.C != C) {
+  const bool keep = !ctx->scratch_in_graph;
+  if (keep && (had.ws != scr || had.W != W || had.H != H || had.F != F || had.C != C)) {
     k_stage_twiddles<<<1, 256, 0, ctx->stream>>>(ctx_twiddles(ctx, H), tw, 2 * H);
     ctx->launches += 1;
   }
-  const int rc2 = adjoint_in(ctx, tw + 2 * size_t(H), y, S, x, W, H, F, C, 1.0f / float(W * H), tw);
-  if (rc2 == GBN_OK) p = gbn_ctx::SimplePlan{scr, W, H, F, C};
+  const int rc2 = adjoint_in(ctx, tw + 2 * size_t(H), y, S, x, W, H, F, C, 1.0f / float(W * H),
+                             keep ? tw : ctx_twiddles(ctx, H));
+  if (rc2 == GBN_OK && keep) p = gbn_ctx::SimplePlan{scr, W, H, F, C};
   return rc2;
 }
 // the same in working memory of simple_recon_bytes that the caller has
