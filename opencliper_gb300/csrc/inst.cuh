@@ -113,11 +113,11 @@ struct Launchers {
   static void adj_cols_of(const float2* T, const float2* S, float2* x, int W, int C, int F, float scale,
                           const float2* tw, int cs, cudaStream_t s) {
     static bool ok = false;
-    constexpr int bytes = AdjColsSmem<L>::BYTES;
+    constexpr int bytes = AdjColsShape<L, RSS>::BYTES;
     allow_smem(k_adj_cols<L, RSS>, bytes, ok);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(W / kWB, cs, F);
-    cfg.blockDim = dim3(kColNT);
+    cfg.blockDim = dim3(AdjColsShape<L, RSS>::NT);
     cfg.dynamicSmemBytes = bytes;
     cfg.stream = s;
     cudaLaunchAttribute at[2];
@@ -141,7 +141,8 @@ struct Launchers {
   static SizeKernels entry() {
     static_assert(fft_size_ok(L), "unsupported transform length");
     return SizeKernels{L, &fwd_cols, &rows, &inv_cols, &fft_rows, &fft_cols, &enc_cols, &adj_cols,
-                       iter_cols_ok(L) ? &iter_cols : nullptr, &iter_finish, iter_pair_ok(L) ? pair_cols(L) : 0, RowCfg<L>::RPC, &rows_occupancy};
+                       iter_cols_ok(L) ? &iter_cols : nullptr, &iter_finish, iter_pair_ok(L) ? pair_cols(L) : 0,
+                       {AdjColsShape<L, false>::MINB, AdjColsShape<L, true>::MINB}, RowCfg<L>::RPC, &rows_occupancy};
   }
 };
 

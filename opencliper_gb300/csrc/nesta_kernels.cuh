@@ -1107,137 +1107,174 @@ __global__ void __launch_bounds__(kColNT) k_enc_cols(const float2* in, const flo
 // the sum of |scale IDFT_H(T_c)|^2.  grid (W/kWB, CS, frames) in clusters of CS
 // CTAs along y, which share a tile's coils (coil c on CTA c % CS) and add up
 // through distributed shared memory, in CTA order; each finishes part of the
-// tile's rows.  The next coil's values are loaded while this one is transformed.
-template <int H>
-struct AdjColsSmem {
-  static constexpr int A = Split<H>::A, B = Split<H>::B, KS = col_ks(A);
-  static constexpr int NI2 = cdiv(kWB * B, kColNT);
-  static constexpr int EXN = B * KS > NI2 * A * kColNT ? B * KS : NI2 * A * kColNT;  // exchange, then accumulators
-  static constexpr int BYTES = EXN * 8;
-};
-// (at 168 registers and three CTAs per SM, twiddles in shared memory, 60 against 51
-// us at 256 x 256 x 20 x 12)
+// tile's rows.
+//
+// Bound by memory.  The next coil's tiles of T and S are copied to shared memory
+// while this one is transformed.  (T alone ahead, in registers, and S read where it is
+// used left the loads' latency in the chain of every coil, 19 of 22 stall cycles an
+// instruction, and spilled past first factors of 16.  E^H, us, that form -> now: 256 x 256
+// x 20 x 12 coils 97 -> 84, 384 x 160 x 30 x 19 454 -> 167, 384 x 384 x 10 x 16 470 -> 127,
+// 512 x 512 x 4 x 8 189 -> 53, 96 x 504 x 6 x 9 125 -> 33; SOS at 512 83 -> 55.)  The first
+// pass works in place, so that a coil's exchange needs no memory of its own and two
+// coils' tiles leave several CTAs per SM.
 template <int H, bool RSS>
-__global__ void __launch_bounds__(kColNT) k_adj_cols(const float2* T, const float2* __restrict__ S,
-                                                     float2* __restrict__ x, int W, int C, float scale,
-                                                     const float2* __restrict__ twH) {
-  using L = AdjColsSmem<H>;
-  constexpr int A = L::A, B = L::B, KS = L::KS;
+struct AdjColsShape {
+  static constexpr int A = Split<H>::A, B = Split<H>::B;
+  // a thread per second-pass item: it holds A accumulators
+  static constexpr int NT = B <= 16 ? kColNT : cdiv(kWB * B, 32) * 32;
+  static constexpr int NI1 = cdiv(kWB * A, NT);
+  static_assert(kWB * B <= NT, "one second-pass item per thread");
+  static constexpr int AP = A | 1;                   // rows of a block of A, padded: blocks start in different banks
+  static constexpr int TN = B * AP * kWB;            // float2 of a coil's T tile
+  static constexpr bool TWS = B > 16 || (B == 16 && A > 24);  // twiddles in shared memory: they would take 2*NI1*B registers
+  static constexpr int FIX = 2 * TN + (TWS ? H : 0);
+  // two S tiles, or one (copied during the first pass) where two leave one CTA per SM
+  static constexpr int SB = RSS ? 0 : 2 * ((FIX + 2 * H * kWB) * 8 + 1024) <= 228 * 1024 ? 2 : 1;
+  static constexpr int BYTES = (FIX + SB * H * kWB) * 8;
+  static_assert(A * NT <= 2 * TN, "the accumulators' exchange fits the T tiles");
+  // CTAs per SM the registers are for: no more than shared memory holds
+  static constexpr int BY_SMEM = 228 * 1024 / (BYTES + 1024);
+  static constexpr int STATE = (RSS ? A : 2 * A) + 2 * (A > B ? A : B) + (TWS ? 0 : 2 * NI1 * B);  // a thread's registers, roughly
+  static constexpr int BY_REGS =
+      (A <= 12 ? 512 : A <= 16 ? (TWS ? 512 : 384) : (RSS && STATE <= 128) || NT > kColNT ? 384 : 256) / NT;
+  static constexpr int MINB = BY_SMEM < BY_REGS ? BY_SMEM : BY_REGS;
+  static_assert(MINB >= 1, "a CTA fits");
+};
+template <int H, bool RSS>
+__global__ void __launch_bounds__(AdjColsShape<H, RSS>::NT, AdjColsShape<H, RSS>::MINB)
+    k_adj_cols(const float2* T, const float2* __restrict__ S, float2* __restrict__ x, int W, int C, float scale,
+               const float2* __restrict__ twH) {
+  using L = AdjColsShape<H, RSS>;
+  constexpr int A = L::A, B = L::B, AP = L::AP, NI1 = L::NI1, NT = L::NT;
   constexpr int N1 = kWB * A, N2 = kWB * B;
-  constexpr int NI1 = cdiv(N1, kColNT), NI2 = L::NI2;
   extern __shared__ float4 smem4[];
-  float2* const ex = reinterpret_cast<float2*>(smem4);
+  float2* const Tb = reinterpret_cast<float2*>(smem4);  // [2][B][AP][kWB]
+  float2* const tws = Tb + 2 * L::TN;                   // [B][A]
+  float2* const Sb = Tb + L::FIX;                       // [SB][H][kWB]
   const int t = threadIdx.x, w0 = blockIdx.x * kWB, f = blockIdx.z;
   const int CS = gridDim.y, rank = blockIdx.y;  // the cluster covers the grid's y
   const size_t N = size_t(H) * W;
-  float2 twr[NI1][B];
+  const bool s16 = (reinterpret_cast<uintptr_t>(S) & 15) == 0;  // the caller's maps; T is 16-byte aligned
+  constexpr int GR = kWB / 2, RSTEP = NT / GR;                  // 16-byte granules of a row, rows per round
+  const int row0 = t / GR, part = 2 * (t % GR);
+  auto issue_S = [&](int c, int buf) {
+    const float2* const src = S + size_t(c) * N + w0 + part;
+    float2* const dst = Sb + buf * (H * kWB) + part;
+    if (s16) {
 #pragma unroll
-  for (int ii = 0; ii < NI1; ++ii) {
-    const int i = t + ii * kColNT, s = i < N1 ? i / kWB : 0;
-#pragma unroll
-    for (int k1p = 0; k1p < B; ++k1p) twr[ii][k1p] = __ldg(twH + H + k1p * A + s);
-  }
-  grid_dep_wait();  // T comes from the row pass
-  float2 pf[NI1][B];
-  auto fetch = [&](int c) {
-    const float2* const src = T + (size_t(f) * C + c) * N + w0;
-#pragma unroll
-    for (int ii = 0; ii < NI1; ++ii) {
-      const int i = t + ii * kColNT;
-      if (N1 % kColNT == 0 || i < N1) {
-        const int w = i % kWB, s = i / kWB;
-#pragma unroll
-        for (int n1 = 0; n1 < B; ++n1) pf[ii][n1] = src[size_t(A * n1 + s) * W + w];
+      for (int r = row0; r < H; r += RSTEP) cp_async16(dst + r * kWB, src + size_t(r) * W);
+    } else {
+      for (int r = row0; r < H; r += RSTEP) {
+        cp_async8(dst + r * kWB, src + size_t(r) * W);
+        cp_async8(dst + r * kWB + 1, src + size_t(r) * W + 1);
       }
     }
   };
-  float2 acc[NI2][A];
+  auto issue_T = [&](int c, int buf) {
+    const float2* const src = T + (size_t(f) * C + c) * N + w0 + part;
+    float2* const dst = Tb + buf * L::TN + part;
 #pragma unroll
-  for (int ii = 0; ii < NI2; ++ii)
-#pragma unroll
-    for (int k2 = 0; k2 < A; ++k2) acc[ii][k2] = make_float2(0.f, 0.f);
-  if (rank < C) fetch(rank);
-  for (int c = rank; c < C; c += CS) {
+    for (int r = row0; r < H; r += RSTEP) cp_async16(dst + (r / A * AP + r % A) * kWB, src + size_t(r) * W);
+  };
+  if constexpr (L::SB == 2) {
+    if (rank < C) issue_S(rank, 0);
+  }
+  float2 twr[L::TWS ? 1 : NI1][L::TWS ? 1 : B];
+  if constexpr (L::TWS) {
+    for (int i = t; i < H; i += NT) tws[i] = __ldg(twH + H + i);
+  } else {
 #pragma unroll
     for (int ii = 0; ii < NI1; ++ii) {
-      const int i = t + ii * kColNT;
-      if (N1 % kColNT == 0 || i < N1) {
-        const int w = i % kWB, s = i / kWB;
+      const int i = t + ii * NT, s = i < N1 ? i / kWB : 0;
+#pragma unroll
+      for (int k1p = 0; k1p < B; ++k1p) twr[ii][k1p] = __ldg(twH + H + k1p * A + s);
+    }
+  }
+  grid_dep_wait();  // T comes from the row pass
+  if (rank < C) issue_T(rank, 0);
+  cp_async_commit();
+  float2 acc[A];
+#pragma unroll
+  for (int k2 = 0; k2 < A; ++k2) acc[k2] = make_float2(0.f, 0.f);
+  int buf = 0;
+  for (int c = rank; c < C; c += CS, buf ^= 1) {
+    cp_async_wait<0>();
+    __syncthreads();  // coil c's tiles are there; the one before is done with
+    if constexpr (L::SB == 1) {
+      issue_S(c, 0);
+      cp_async_commit();
+    }
+    if (c + CS < C) {
+      if constexpr (L::SB == 2) issue_S(c + CS, buf ^ 1);
+      issue_T(c + CS, buf ^ 1);
+    }
+    cp_async_commit();
+    float2* const Tc = Tb + buf * L::TN;
+#pragma unroll
+    for (int ii = 0; ii < NI1; ++ii) {
+      const int i = t + ii * NT;
+      if (N1 % NT == 0 || i < N1) {
+        float2* const slot = Tc + i;  // row A*n1 + s of column w at n1*AP*kWB + s*kWB + w
         float2 v[B];
 #pragma unroll
-        for (int n1 = 0; n1 < B; ++n1) v[n1] = conjf2(pf[ii][n1]);
+        for (int n1 = 0; n1 < B; ++n1) v[n1] = conjf2(slot[n1 * AP * kWB]);
         dft<B>(v);
 #pragma unroll
-        for (int k1p = 0; k1p < B; ++k1p)
-          ex[k1p * KS + s * kWB + w] = (k1p == 0) ? v[k1p] : cmul(v[k1p], twr[ii][k1p]);
-      }
-    }
-    if (c + CS < C) fetch(c + CS);
-    __syncthreads();
-#pragma unroll
-    for (int ii = 0; ii < NI2; ++ii) {
-      const int i = t + ii * kColNT;
-      if (N2 % kColNT == 0 || i < N2) {
-        const int w = i % kWB, k1p = i / kWB;
-        float2 sv[RSS ? 1 : A];
-        if constexpr (!RSS) {
-          const float2* const sc = S + size_t(c) * N + w0 + w;
-#pragma unroll
-          for (int k2 = 0; k2 < A; ++k2) sv[k2] = __ldg(sc + size_t(k1p + B * k2) * W);
-        }
-        float2 v[A];
-#pragma unroll
-        for (int s = 0; s < A; ++s) v[s] = ex[k1p * KS + s * kWB + w];
-        dft<A>(v);
-#pragma unroll
-        for (int k2 = 0; k2 < A; ++k2) {
-          if constexpr (RSS) {
-            const float2 e = cscale(v[k2], scale);
-            acc[ii][k2].x = __fadd_rn(acc[ii][k2].x, __fadd_rn(__fmul_rn(e.x, e.x), __fmul_rn(e.y, e.y)));
-          } else {  // conj(v) * conj(S) == conj(v * S)
-            const float2 p = cmul(v[k2], sv[k2]);
-            acc[ii][k2].x += p.x;
-            acc[ii][k2].y -= p.y;
-          }
+        for (int k1p = 0; k1p < B; ++k1p) {
+          if constexpr (L::TWS)
+            slot[k1p * AP * kWB] = (k1p == 0) ? v[k1p] : cmul(v[k1p], tws[k1p * A + i / kWB]);
+          else
+            slot[k1p * AP * kWB] = (k1p == 0) ? v[k1p] : cmul(v[k1p], twr[ii][k1p]);
         }
       }
     }
+    if constexpr (L::SB == 1) cp_async_wait<1>();
     __syncthreads();
+    if (N2 % NT == 0 || t < N2) {
+      const int w = t % kWB, k1p = t / kWB;
+      float2 v[A];
+#pragma unroll
+      for (int s = 0; s < A; ++s) v[s] = Tc[(k1p * AP + s) * kWB + w];
+      dft<A>(v);
+#pragma unroll
+      for (int k2 = 0; k2 < A; ++k2) {
+        if constexpr (RSS) {
+          const float2 e = cscale(v[k2], scale);
+          acc[k2].x = __fadd_rn(acc[k2].x, __fadd_rn(__fmul_rn(e.x, e.x), __fmul_rn(e.y, e.y)));
+        } else {  // conj(v) * conj(S) == conj(v * S)
+          const float2 p = cmul(v[k2], Sb[(L::SB == 2 ? buf : 0) * (H * kWB) + (k1p + B * k2) * kWB + w]);
+          acc[k2].x += p.x;
+          acc[k2].y -= p.y;
+        }
+      }
+    }
   }
   int kb = 0, ke = A;  // the rows k2 this CTA finishes
   if (CS > 1) {
     namespace cgr = cooperative_groups;
     cgr::cluster_group cluster = cgr::this_cluster();
+    __syncthreads();  // the tiles are done with
 #pragma unroll
-    for (int ii = 0; ii < NI2; ++ii)
-#pragma unroll
-      for (int k2 = 0; k2 < A; ++k2) ex[(ii * A + k2) * kColNT + t] = acc[ii][k2];
+    for (int k2 = 0; k2 < A; ++k2) Tb[k2 * NT + t] = acc[k2];
     cluster.sync();
     kb = rank * A / CS;
     ke = (rank + 1) * A / CS;
 #pragma unroll
-    for (int ii = 0; ii < NI2; ++ii)
-#pragma unroll
-      for (int k2 = 0; k2 < A; ++k2)
-        if (k2 >= kb && k2 < ke) {
-          float2 sum = make_float2(0.f, 0.f);
-          for (int g = 0; g < CS; ++g)
-            sum = cadd(sum, cluster.map_shared_rank(ex, g)[(ii * A + k2) * kColNT + t]);
-          acc[ii][k2] = sum;
-        }
+    for (int k2 = 0; k2 < A; ++k2)
+      if (k2 >= kb && k2 < ke) {
+        float2 sum = make_float2(0.f, 0.f);
+        for (int g = 0; g < CS; ++g) sum = cadd(sum, cluster.map_shared_rank(Tb, g)[k2 * NT + t]);
+        acc[k2] = sum;
+      }
     cluster.sync();  // the others have read this CTA's accumulators
   }
+  if (N2 % NT == 0 || t < N2) {
+    const int w = t % kWB, k1p = t / kWB;
 #pragma unroll
-  for (int ii = 0; ii < NI2; ++ii) {
-    const int i = t + ii * kColNT;
-    if (N2 % kColNT == 0 || i < N2) {
-      const int w = i % kWB, k1p = i / kWB;
-#pragma unroll
-      for (int k2 = 0; k2 < A; ++k2)
-        if (k2 >= kb && k2 < ke)
-          x[size_t(f) * N + size_t(k1p + B * k2) * W + w0 + w] =
-              RSS ? make_float2(sqrtf(acc[ii][k2].x), 0.f) : cscale(acc[ii][k2], scale);
-    }
+    for (int k2 = 0; k2 < A; ++k2)
+      if (k2 >= kb && k2 < ke)
+        x[size_t(f) * N + size_t(k1p + B * k2) * W + w0 + w] =
+            RSS ? make_float2(sqrtf(acc[k2].x), 0.f) : cscale(acc[k2], scale);
   }
 }
 

@@ -315,10 +315,14 @@ static int adjoint_in(gbn_ctx* ctx, float2* scratch, const float2* k, const floa
                       int C, float scale, const float2* twH) {
   const int rc = rows_pass(ctx, k, scratch, W, H, (long long)F * C * H, 1, 1.0f, nullptr, C);
   if (rc != GBN_OK) return rc;
-  // CTAs that share a tile's coils: until there are two per SM (six: 192 x 160 x 20 x
-  // 12 coils 44 against 39 us)
+  // CTAs that share a tile's coils: as many as run at once.  A second wave costs more
+  // than shorter chains of coils give (E^H in us with 1, 2, 4, 8 CTAs a tile: 512 x 512 x
+  // 4 x 8 coils, 256 tiles on 304 places, 54, 100, 116, 155; 72 x 432 x 32 x 4, 288 on 304,
+  // 26, 51, 64, 64; 48 x 64 x 40 x 32, 240 on 608, 34, 30, 32, 38; recon of 256 x 256 x 1 x
+  // 8, 32 on 456, 19, 16, 12, 10).
+  const long long tiles = (long long)(W / kWB) * F, places = (long long)ctx->nsm * find_size(H)->adj_per_sm[S ? 0 : 1];
   int cs = 1;
-  while (cs < 8 && 2 * cs <= C && (long long)(W / kWB) * F * cs < 2LL * ctx->nsm) cs *= 2;
+  while (cs < 8 && 2 * cs <= C && 2 * cs * tiles <= places) cs *= 2;
   find_size(H)->adj_cols(scratch, S, x, W, C, F, scale, twH, cs, ctx->stream);
   ctx->launches += 1;
   return cuda_status(cudaGetLastError(), "adjoint");

@@ -37,6 +37,7 @@ struct SizeKernels {
   // the sums and scalar step of iteration it - 1 alone (column-pair form)
   void (*iter_finish)(const FusedArgs* tab, const BatchMap& bm, int it, dim3 grid, cudaStream_t s);
   int pair_cols;     // columns per tile of the column-pair form of iter_cols; 0: iter_cols works on natural buffers
+  int adj_per_sm[2];  // CTAs of adj_cols that share an SM: with S, and without
   int rows_per_cta;  // rows processed per CTA step by the row kernels
   int (*rows_occupancy)(bool resid);  // resident row-kernel CTAs per SM
 };
