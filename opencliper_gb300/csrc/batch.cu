@@ -284,10 +284,19 @@ int batch_create(gbn_ctx* ctx, int n, gbn_problem* const* problems, const gbn_ne
     // measured (the tensor-core row-local iteration, and the three-pass
     // iteration with the tensor-core forward pass, at 256 and 384)
     bool analysed = false;
+    // the row-local iteration's tiles of every member; without the memory the group runs
+    // the three-pass iteration
+    auto take_row_local = [&](bool all) {
+      for (int i : g.idx) {
+        bool fresh = false;
+        if (all && kh->pair_cols) all = problem_tiles(b->probs[i], true, &fresh) == GBN_OK;
+      }
+      g.row_local = all;
+    };
     if (kh->iter_cols && ctx->row_local && (precision == GBN_PRECISION_FP32 || ctx->mixed_fwd_tc < 0)) {
       bool all = false;
       if ((rc = rows_all_local(&all)) != GBN_OK) break;
-      g.row_local = all;
+      take_row_local(all);
       analysed = true;
     }
     if (precision == GBN_PRECISION_MIXED && !g.row_local) {
@@ -375,7 +384,10 @@ int batch_create(gbn_ctx* ctx, int n, gbn_problem* const* problems, const gbn_ne
         ctx->row_local) {
       bool all = false;
       if ((rc = rows_all_local(&all)) != GBN_OK) break;
-      g.row_local = all;
+      take_row_local(all);
+      for (int k = 0; k < ng && g.row_local; ++k)  // the entries once more, with the tiles
+        ctx->launches +=
+            launch_store_args(g.tab + k, make_args(b->probs[g.idx[k]], b->out[g.idx[k]]), ctx->stream);
     }
   }
   if (rc == GBN_OK && (e = cudaGetLastError()) != cudaSuccess) rc = cuda_status(e, "batch tables");

@@ -128,11 +128,13 @@ struct gbn_problem {
   float2* mc_gm = nullptr;            // M^T of it
   double* mc_part = nullptr;          // power-method norm partials
   gbn::McTables* mc_tab = nullptr;    // gather tables of the meshes (motion.cu)
-  // column-pair row-local iteration (rowpair.cuh)
+  // column-pair row-local iteration (rowpair.cuh): allocated by the first run that
+  // takes it (problem_tiles), but for ptab and rowslot
+  void* tiles[2] = {nullptr, nullptr};  // blocks of the following
   float4* St = nullptr;               // S in tiles
   float4* Tt = nullptr;               // kept rows' IDFT_W(y) in tiles
   size_t Tt_rows = 0;                 // kept rows Tt holds
-  float2* xk2 = nullptr;              // third x_k and w_k buffers
+  float2* xk2 = nullptr;              // third x_k and w_k buffers (not with motion compensation)
   float2* wacc2 = nullptr;
   float4* xt = nullptr;               // x_ref in tiles
   uint4* ptab = nullptr;              // [F][PA]

@@ -970,11 +970,15 @@ int nesta_run_mc(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, floa
   const dim3 g3(W / kWB, 2, F);
   const dim3 gtv(t->nbp, (F + kTvFrames - 1) / kTvFrames);
   const dim3 gadj = frame_grid(W * H, F);
-  FusedArgs a = make_args(P, x_out);
-  a.tv_src = P->mc_xw;  // marks the motion-compensated form: the forward pass skips its tTV sums
-  a.grad_ext = P->mc_gm;
-  a.part_tv = t->tvpart;
-  a.ntv = F * t->nbp;
+  auto entry = [&]() {
+    FusedArgs a = make_args(P, x_out);
+    a.tv_src = P->mc_xw;  // marks the motion-compensated form: the forward pass skips its tTV sums
+    a.grad_ext = P->mc_gm;
+    a.part_tv = t->tvpart;
+    a.ntv = F * t->nbp;
+    return a;
+  };
+  const FusedArgs a = entry();
   const FusedArgs* tab = P->d_args;
   const BatchMap bm = single_map(F, P->ctl);
   int rc;
@@ -1015,6 +1019,11 @@ int nesta_run_mc(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, floa
   if (check_rows) {
     if ((ef = cudaEventSynchronize(ctx->ev_partial)) != cudaSuccess) return cuda_status(ef, "row structure read-back");
     row_local = *ctx->host_partial == 0;
+  }
+  if (row_local && kh->pair_cols) {
+    bool fresh = false;
+    row_local = problem_tiles(P, false, &fresh) == GBN_OK;
+    if (row_local && fresh) ctx->launches += launch_store_args(P->d_args, entry(), s);
   }
   if (row_local) {
     // per inner iteration, on one stream with programmatic dependent launch:

@@ -664,17 +664,34 @@ void launch_normest_chunk(int fmax, int nblk, cudaStream_t s, int N, int F, cons
 
 }  // namespace
 
+// a buffer to carve from a block
+struct Part {
+  void** p;
+  size_t bytes;
+};
+// One allocation for all of them, each 256-byte aligned; on failure none is touched.
+static cudaError_t alloc_parts(void** block, const Part* parts, int n) {
+  auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+  size_t total = 0;
+  for (int k = 0; k < n; ++k) total += up(parts[k].bytes);
+  const cudaError_t e = cudaMalloc(block, total);
+  if (e != cudaSuccess) {
+    *block = nullptr;
+    return e;
+  }
+  unsigned char* b = static_cast<unsigned char*>(*block);
+  for (int k = 0; k < n; b += up(parts[k].bytes), ++k) *parts[k].p = b;
+  return cudaSuccess;
+}
+
 int problem_alloc(gbn_problem* P) {
   const size_t FH = size_t(P->F) * P->H;
   const size_t X = size_t(P->F) * P->H * P->W;
   const size_t K = X * P->C;
   const SizeKernels* kh = find_size(P->H);
   const bool pair = kh && kh->pair_cols;
-  // one allocation for everything but the row buffers, which fit_rows resizes
-  struct Part {
-    void** p;
-    size_t bytes;
-  };
+  // one allocation for everything but the row buffer, which fit_rows resizes, and the
+  // tiles, which only row-local runs of column-pair lengths need
   const Part parts[] = {{(void**)&P->flags, FH * sizeof(int)},
                         {(void**)&P->full_fh, FH * sizeof(int)},
                         {(void**)&P->rowmap, FH * sizeof(int)},
@@ -690,32 +707,54 @@ int problem_alloc(gbn_problem* P) {
                         {(void**)&P->d_args, sizeof(FusedArgs)},
                         {(void**)&P->ctl, sizeof(ClassCtl)},
                         // column pairs only
-                        {(void**)&P->St, size_t(P->C) * P->H * P->W * sizeof(float2)},
-                        {(void**)&P->xt, X * sizeof(float2)},
-                        {(void**)&P->xk2, X * sizeof(float2)},
-                        {(void**)&P->wacc2, X * sizeof(float2)},
                         {(void**)&P->ptab, size_t(P->F) * pair_a(P->H) * sizeof(uint4)},
                         {(void**)&P->rowslot, FH * sizeof(int)}};
-  const size_t nparts = sizeof(parts) / sizeof(parts[0]) - (pair ? 0 : 6);
-  auto up = [](size_t v) { return (v + 255) / 256 * 256; };
-  size_t total = 0;
-  for (size_t k = 0; k < nparts; ++k) total += up(parts[k].bytes);
-  cudaError_t e = cudaMalloc(&P->block, total);
+  const int nparts = int(sizeof(parts) / sizeof(parts[0])) - (pair ? 0 : 2);
+  cudaError_t e = alloc_parts(&P->block, parts, nparts);
   if (e == cudaSuccess) {
-    unsigned char* b = static_cast<unsigned char*>(P->block);
-    for (size_t k = 0; k < nparts; b += up(parts[k].bytes), ++k) *parts[k].p = b;
     e = cudaMalloc(&P->T, K * sizeof(float2));
     P->T_rows = FH;
-  }
-  if (e == cudaSuccess && pair) {
-    P->Tt_rows = size_t(P->F) * std::min(P->H, iter_cols_rcap(P->H));
-    e = cudaMalloc(&P->Tt, P->Tt_rows * P->C * P->W * sizeof(float2));
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return set_error(GBN_ERR_NOMEM, std::string("problem workspace allocation failed: ") + cudaGetErrorString(e));
   }
   return GBN_OK;
+}
+
+int problem_tiles(gbn_problem* P, bool plain, bool* fresh) {
+  const size_t X = size_t(P->F) * P->H * P->W;
+  Part parts[5];
+  int n = 0;
+  size_t trows = P->Tt_rows;
+  if (!P->St) {
+    trows = std::min<size_t>(P->T_rows, size_t(P->F) * std::min(P->H, iter_cols_rcap(P->H)));
+    parts[n++] = {(void**)&P->Tt, std::max<size_t>(trows, 1) * P->C * P->W * sizeof(float2)};
+    parts[n++] = {(void**)&P->St, size_t(P->C) * P->H * P->W * sizeof(float2)};
+    parts[n++] = {(void**)&P->xt, X * sizeof(float2)};
+  }
+  if (plain && !P->xk2) {
+    parts[n++] = {(void**)&P->xk2, X * sizeof(float2)};
+    parts[n++] = {(void**)&P->wacc2, X * sizeof(float2)};
+  }
+  *fresh = n > 0;
+  if (n == 0) return GBN_OK;
+  if (alloc_parts(&P->tiles[P->tiles[0] ? 1 : 0], parts, n) != cudaSuccess) {
+    cudaGetLastError();
+    return GBN_ERR_NOMEM;
+  }
+  P->Tt_rows = trows;
+  return GBN_OK;
+}
+
+static void tiles_free(gbn_problem* P) {
+  for (void*& b : P->tiles) {
+    if (b) cudaFree(b);
+    b = nullptr;
+  }
+  P->St = P->Tt = P->xt = nullptr;
+  P->xk2 = P->wacc2 = nullptr;
+  P->Tt_rows = 0;
 }
 
 void launch_row_analysis(gbn_problem* P, ClassCtl* ctl, cudaStream_t s);
@@ -737,32 +776,18 @@ int problem_fit_rows(gbn_problem* P, int headroom, int* kept) {
     if ((e = cudaMemcpyAsync(&g, P->rowoff + P->F, sizeof(int), cudaMemcpyDeviceToHost, s)) == cudaSuccess &&
         (e = cudaStreamSynchronize(s)) == cudaSuccess) {
       const size_t want = std::min<size_t>(size_t(P->F) * P->H, size_t(g) + size_t(headroom));
-      // the tiles follow: never more than the row-local iteration takes
-      const SizeKernels* kh = find_size(P->H);
-      const size_t tt = kh && kh->pair_cols
-                            ? std::min<size_t>(want, size_t(P->F) * std::min(P->H, iter_cols_rcap(P->H)))
-                            : 0;
-      // both buffers before either is given back: a failure leaves the problem as it was
-      const size_t row = size_t(P->C) * P->W;
+      // the new buffer before the old one is given back: a failure leaves the problem as it was
       float2* nt = nullptr;
-      float4* ntt = nullptr;
-      if (want != saved) e = cudaMalloc(&nt, std::max<size_t>(want, 1) * row * sizeof(float2));
-      if (e == cudaSuccess && tt != P->Tt_rows) e = cudaMalloc(&ntt, std::max<size_t>(tt, 1) * row * sizeof(float2));
-      if (e == cudaSuccess) {
+      if (want == saved || (e = cudaMalloc(&nt, std::max<size_t>(want, 1) * P->C * P->W * sizeof(float2))) == cudaSuccess) {
         if (nt) {
           cudaFree(P->T);
           P->T = nt;
-        }
-        if (ntt) {
-          cudaFree(P->Tt);
-          P->Tt = ntt;
-          P->Tt_rows = tt;
+          tiles_free(P);  // sized for the rows before; the next run that takes them allocates them
         }
         P->T_rows = want;
         if (kept) *kept = g;
         return GBN_OK;
       }
-      if (nt) cudaFree(nt);
     }
   }
   P->T_rows = saved;
@@ -774,8 +799,9 @@ int problem_fit_rows(gbn_problem* P, int headroom, int* kept) {
 void motion_free(gbn_problem* P);
 
 void problem_free(gbn_problem* P) {
-  void* ptrs[] = {P->block,   P->T,    P->Tt, P->fmean,  P->part_tv, P->part_r,
-                  P->part_ne, P->ne_b, P->fk, P->colmax, P->smax,    P->fa};
+  tiles_free(P);
+  void* ptrs[] = {P->block,   P->T,    P->fmean,  P->part_tv, P->part_r, P->part_ne,
+                  P->ne_b, P->fk, P->colmax, P->smax,    P->fa};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   motion_free(P);
@@ -1070,6 +1096,11 @@ int nesta_run(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm, float2*
   if (ctx->row_local && kh->iter_cols) {
     if ((ef = cudaEventSynchronize(ctx->ev_partial)) != cudaSuccess) return cuda_status(ef, "row structure read-back");
     row_local = *ctx->host_partial == 0;
+  }
+  if (row_local && kh->pair_cols) {  // the setup is still running while the tiles are allocated
+    bool fresh = false;
+    row_local = problem_tiles(P, true, &fresh) == GBN_OK;
+    if (row_local && fresh) ctx->launches += launch_store_args(P->d_args, make_args(P, x_out), s);
   }
   // stopping test on: the launches that recompute the last update if the rule
   // stops the loop (row-local iteration only; the column pairs run one iteration

@@ -30,6 +30,12 @@ struct RandStart {
 // Checks the parameters of a run of P and grows its workspace for them.
 int run_prepare(gbn_ctx* ctx, gbn_problem* P, const gbn_nesta_params* prm);
 
+// The tiles of the column-pair row-local iteration; plain: and its third buffers, which
+// the motion-compensated form does without.  *fresh: some were allocated now, so that
+// tables stored before lack them.  GBN_ERR_NOMEM, with nothing kept of the attempt, when
+// they cannot be had: the three-pass iteration, which does without them, then runs.
+int problem_tiles(gbn_problem* P, bool plain, bool* fresh);
+
 // Instance-table entry of P writing its image (x_ref, the output XData) to xref.
 FusedArgs make_args(gbn_problem* P, float2* xref);
 BatchMap single_map(int F, ClassCtl* ctl);

@@ -36,3 +36,8 @@ def _host_program(tmp_path, name):
 def test_fit_rows_keeps_the_problem_when_memory_runs_out(tmp_path):
     r = subprocess.run([_host_program(tmp_path, "fit_rows")], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+def test_row_local_tiles_are_allocated_where_they_are_used(tmp_path):
+    r = subprocess.run([_host_program(tmp_path, "tile_memory")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
