@@ -645,9 +645,17 @@ struct InvColsSmem {
   static_assert(cdiv(kWB * B, kColNT) * A * kColNT <= 2 * H * kWB, "accumulator exchange must fit the S buffers");
 };
 
-constexpr bool inv_prefetch(int H) { return cdiv(kWB * split_a(H), kColNT) == 1 && split_a(H) <= 16; }
+// The form whose next coil's unstaged rows travel in registers and whose twiddles come
+// before the wait, bounded for three CTAs per SM: both factors up to 16.  Past that it
+// spills (second factors 20 to 28: 280, 360, 392) or leaves two CTAs per SM (first
+// factors 18 to 27: 168, 200, 216, 288), and the launch bound stays open: a minimum of
+// one CTA lets the compiler take half as many registers again.  Pixel masks, W = 128, 12
+// frames, 8 coils, 20 iterations, us, plain form / this one: H = 72 721 / 701, 120 832 /
+// 800, 128 794 / 759, 160 888 / 865, 192 918 / 874, 256 1004 / 1003; 168 933 / 1135, 288
+// 1328 / 1545, 360 1819 / 1990, 392 1900 / 2169.
+constexpr bool inv_prefetch(int H) { return split_a(H) <= 16 && split_b(H) <= 16; }
 template <int H, bool UPDATE>
-__global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT, inv_prefetch(H) ? 3 : 1)
+__global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT, inv_prefetch(H) ? 3 : 0)
     k_inv_cols(const FusedArgs* __restrict__ tab, const __grid_constant__ BatchMap bm, int it) {
   using L = InvColsSmem<H>;
   constexpr int A = L::A, B = L::B, KS = L::KS, RCAP = L::RCAP;
@@ -696,13 +704,17 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT, inv_prefetch
   for (int i = t; i < H; i += kColNT) rmap[i] = a.rowmap[f * H + i];
   // inter-pass twiddles of this thread's pass-1 items, identical for every coil
   float2 twr[NI1][B];
+  auto load_twiddles = [&]() {
 #pragma unroll
-  for (int ii = 0; ii < NI1; ++ii) {
-    const int i = t + ii * kColNT;
-    const int s = (i < N1) ? i / kWB : 0;
+    for (int ii = 0; ii < NI1; ++ii) {
+      const int i = t + ii * kColNT;
+      const int s = (i < N1) ? i / kWB : 0;
 #pragma unroll
-    for (int k1p = 0; k1p < B; ++k1p) twr[ii][k1p] = __ldg(a.twH + H + k1p * A + s);
-  }
+      for (int k1p = 0; k1p < B; ++k1p) twr[ii][k1p] = __ldg(a.twH + H + k1p * A + s);
+    }
+  };
+  constexpr bool PREF = inv_prefetch(H);
+  if constexpr (PREF) load_twiddles();
   grid_dep_wait();  // T and the scalar state come from the row pass
   grid_dep_release();
   if (UPDATE && it > st->last_iter) {  // uniform over the instance, so over each cluster
@@ -713,12 +725,8 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT, inv_prefetch
   if (cbeg < cend) issue_T(cbeg, 0);
   cp_async_commit();
   // Frames that keep more rows than the shared buffers hold: the next coil's values
-  // travel to registers while this one is transformed, where a thread has one item and
-  // its state leaves room.  With the bound of three CTAs per SM: at two, without it, a
-  // solve is 6 % slower than with no prefetch, at three 2 % faster (pixel masks, 20
-  // iterations: 240 x 224 x 12, 8 coils 1475 -> 1441 us, 256 x 240 x 24, 16 coils 4022 ->
-  // 3963).
-  constexpr bool PREF = inv_prefetch(H);
+  // travel to registers while this one is transformed (inv_prefetch; at two CTAs per SM,
+  // without the bound, a solve is 6 % slower than with no prefetch).
   float2 tn[PREF ? B : 1];
   auto fetch_T = [&](int c) {
     if constexpr (PREF) {
@@ -737,6 +745,7 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT, inv_prefetch
 #pragma unroll
     for (int k2 = 0; k2 < A; ++k2) acc[ii][k2] = make_float2(0.f, 0.f);
   __syncthreads();
+  if constexpr (!PREF) load_twiddles();
   if (PREF && !staged && cbeg < cend) fetch_T(cbeg);
 
   for (int c = cbeg; c < cend; ++c) {
