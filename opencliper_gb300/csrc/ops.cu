@@ -10,28 +10,33 @@
 
 namespace gbn {
 
-// Element-wise processes: bound by memory.  A thread takes two adjacent complex
-// values (an image has an even number: W is a multiple of 8) in one 16-byte access
-// where every buffer is 16-byte aligned, else in two of 8; frames and coils are grid
-// dimensions (strided over, past the grid's limit), so that no thread divides (with
-// 8-byte accesses and two 64-bit divisions a value, the eight processes of a gradient
-// at 224 x 200 x 16, 10 coils took 117 us; 88 now).
+// Element-wise processes: bound by memory.  In those that write as many values as they
+// read a thread takes two adjacent complex values (an image has an even number: W is a
+// multiple of 8) in one 16-byte access where every buffer is 16-byte aligned, else in two
+// of 8; frames and coils are grid dimensions (strided over, past the grid's limit), so
+// that no thread divides (with 8-byte accesses and two 64-bit divisions a value, the eight
+// processes of a gradient at 224 x 200 x 16, 10 coils took 117 us; 86 now).
+// The normalisation and the sums over coils keep a value per thread: their time is a
+// thread's own chain (a root and divisions; a load per coil), which a pair makes longer
+// and halves the threads for (us, pairs / values: normalisation of 384 x 384 x 20 11.4 /
+// 9.9; coil sum of 128 x 128 x 1, 32 coils 11.3 / 5.1).
 namespace {
 inline int grid_for(gbn_ctx* ctx, size_t n, int nt = 256) {
   return int(std::max<size_t>(1, std::min<size_t>((n + nt - 1) / nt, size_t(ctx->nsm) * 16)));
 }
-// CTAs along the pixel pairs of an image, for y x z images
-inline dim3 image_grid(gbn_ctx* ctx, int N, int y, int z) {
+// CTAs along the pixels of an image, `per` of them a thread, for y x z images
+inline dim3 image_grid(gbn_ctx* ctx, int N, int y, int z, int per = 2) {
   y = std::min(y, 65535);
   z = std::min(z, 65535);
   const long long want = std::max<long long>(1, (long long)ctx->nsm * 64 / ((long long)y * z));
-  return dim3(unsigned(std::min<long long>((N / 2 + 255) / 256, want)), unsigned(y), unsigned(z));
+  return dim3(unsigned(std::min<long long>((N / per + 255) / 256, want)), unsigned(y), unsigned(z));
 }
 inline bool aligned16(const void* a, const void* b = nullptr, const void* c = nullptr) {
   return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
 }
 #define GRID_STRIDE(i, n) \
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < (n); i += size_t(gridDim.x) * blockDim.x)
+#define GRID_PIXELS(i, N) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (N); i += gridDim.x * blockDim.x)
 #define GRID_PAIRS(i, N) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (N) / 2; i += gridDim.x * blockDim.x)
 
 template <bool V>
@@ -67,19 +72,13 @@ __global__ void __launch_bounds__(256) k_ttv(const float2* __restrict__ in, floa
   }
 }
 
-// vectorNormalization.cl:42-56: out = in / fmax(mu, length(in)); pairs, an odd last value apart
-__device__ __forceinline__ float2 normalized(float2 v, float mu) {
-  const float m = fmaxf(mu, sqrtf(fmaf(v.x, v.x, v.y * v.y)));
-  return make_float2(v.x / m, v.y / m);
-}
-template <bool V>
+// vectorNormalization.cl:42-56: out = in / fmax(mu, length(in))
 __global__ void __launch_bounds__(256) k_normalize(const float2* in, float2* out, size_t n, float mu) {
-  GRID_STRIDE(i, n / 2) {
-    const float4 v = ld_pair<V>(in, i);
-    const float2 a = normalized(make_float2(v.x, v.y), mu), b = normalized(make_float2(v.z, v.w), mu);
-    st_pair<V>(out, i, make_float4(a.x, a.y, b.x, b.y));
+  GRID_STRIDE(i, n) {
+    const float2 v = in[i];
+    const float m = fmaxf(mu, sqrtf(fmaf(v.x, v.x, v.y * v.y)));
+    out[i] = make_float2(v.x / m, v.y / m);
   }
-  if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) out[n - 1] = normalized(in[n - 1], mu);
 }
 
 // complexElementProd.cl:42-76: out[f][c][p] = in[f][(c)][p] * (conj?)S[c][p]; grid y: coils, z: frames
@@ -104,22 +103,36 @@ __global__ void __launch_bounds__(256) k_sensmul(const float2* in, int in_has_co
     }
 }
 
+// Pixel i's values of the C coils of a frame (src: coil 0), in order, the loads of
+// eight coils (four, one at the end) on their way before the first is used.
+template <int U, typename Add>
+__device__ __forceinline__ void add_coils(const float2* __restrict__ src, int N, int c, Add&& add) {
+  float2 v[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) v[u] = src[size_t(c + u) * N];
+#pragma unroll
+  for (int u = 0; u < U; ++u) add(v[u]);
+}
+template <typename Add>
+__device__ __forceinline__ void over_coils(const float2* __restrict__ src, int N, int C, Add&& add) {
+  int c = 0;
+  for (; c + 8 <= C; c += 8) add_coils<8>(src, N, c, add);
+  if (c + 4 <= C) {
+    add_coils<4>(src, N, c, add);
+    c += 4;
+  }
+  for (; c < C; ++c) add_coils<1>(src, N, c, add);
+}
+
 // xImageSum.cl:42-61: out[f][p] = sum over coils in order; grid y: frames
-template <bool V>
 __global__ void __launch_bounds__(256) k_coilsum(const float2* __restrict__ in, float2* __restrict__ out, int N, int F,
                                                  int C) {
-  for (int f = blockIdx.y; f < F; f += gridDim.y) {
-    const float2* const src = in + size_t(f) * C * N;
-    GRID_PAIRS(i, N) {
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-      for (int c = 0; c < C; ++c) {
-        const float4 v = ld_pair<V>(src + size_t(c) * N, i);
-        acc = make_float4(acc.x + v.x, acc.y + v.y, acc.z + v.z, acc.w + v.w);
-      }
-      st_pair<V>(out + size_t(f) * N, i, acc);
+  for (int f = blockIdx.y; f < F; f += gridDim.y)
+    GRID_PIXELS(i, N) {
+      float2 acc = make_float2(0.f, 0.f);
+      over_coils(in + size_t(f) * C * N + i, N, C, [&](float2 v) { acc = cadd(acc, v); });
+      out[size_t(f) * N + i] = acc;
     }
-  }
 }
 
 // applyMask.cl:5-40; grid y: coils, z: frames.  Only the masked samples are written.
@@ -172,11 +185,7 @@ int op_ttv(gbn_ctx* ctx, int dir, const float2* in, float2* out, int W, int H, i
 }
 
 int op_normalize(gbn_ctx* ctx, const float2* in, float2* out, size_t n, float mu) {
-  const int g = grid_for(ctx, (n + 1) / 2);
-  if (aligned16(in, out))
-    k_normalize<true><<<g, 256, 0, ctx->stream>>>(in, out, n, mu);
-  else
-    k_normalize<false><<<g, 256, 0, ctx->stream>>>(in, out, n, mu);
+  k_normalize<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(in, out, n, mu);
   return cuda_status(cudaGetLastError(), "normalize");
 }
 
@@ -194,12 +203,7 @@ int op_sensmul(gbn_ctx* ctx, int conj, const float2* in, int in_has_coils, const
 }
 
 int op_coilsum(gbn_ctx* ctx, const float2* in, float2* out, int W, int H, int F, int C) {
-  const int N = W * H;
-  const dim3 g = image_grid(ctx, N, F, 1);
-  if (aligned16(in, out))
-    k_coilsum<true><<<g, 256, 0, ctx->stream>>>(in, out, N, F, C);
-  else
-    k_coilsum<false><<<g, 256, 0, ctx->stream>>>(in, out, N, F, C);
+  k_coilsum<<<image_grid(ctx, W * H, F, 1, 1), 256, 0, ctx->stream>>>(in, out, W * H, F, C);
   return cuda_status(cudaGetLastError(), "coilsum");
 }
 
@@ -231,30 +235,18 @@ int op_rowmask(gbn_ctx* ctx, const uint32_t* rm, uint8_t* pm, int W, int H, int 
 
 // rss.cl:43-74 (RSoS): out[f][p] = (sqrt(sum_c |k[f][c][p]|^2), 0), the sum in
 // coil order in FP32; grid y: frames
-template <bool V>
 __global__ void __launch_bounds__(256) k_rss(const float2* __restrict__ k, float2* __restrict__ out, int N, int F, int C) {
-  for (int f = blockIdx.y; f < F; f += gridDim.y) {
-    const float2* const src = k + size_t(f) * C * N;
-    GRID_PAIRS(i, N) {
-      float a = 0.f, b = 0.f;
-#pragma unroll 4
-      for (int c = 0; c < C; ++c) {
-        const float4 v = ld_pair<V>(src + size_t(c) * N, i);
-        a = __fadd_rn(a, __fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y)));
-        b = __fadd_rn(b, __fadd_rn(__fmul_rn(v.z, v.z), __fmul_rn(v.w, v.w)));
-      }
-      st_pair<V>(out + size_t(f) * N, i, make_float4(sqrtf(a), 0.f, sqrtf(b), 0.f));
+  for (int f = blockIdx.y; f < F; f += gridDim.y)
+    GRID_PIXELS(i, N) {
+      float acc = 0.f;
+      over_coils(k + size_t(f) * C * N + i, N, C,
+                 [&](float2 v) { acc = __fadd_rn(acc, __fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y))); });
+      out[size_t(f) * N + i] = make_float2(sqrtf(acc), 0.f);
     }
-  }
 }
 
 int op_rss(gbn_ctx* ctx, const float2* k, float2* out, int W, int H, int F, int C) {
-  const int N = W * H;
-  const dim3 g = image_grid(ctx, N, F, 1);
-  if (aligned16(k, out))
-    k_rss<true><<<g, 256, 0, ctx->stream>>>(k, out, N, F, C);
-  else
-    k_rss<false><<<g, 256, 0, ctx->stream>>>(k, out, N, F, C);
+  k_rss<<<image_grid(ctx, W * H, F, 1, 1), 256, 0, ctx->stream>>>(k, out, W * H, F, C);
   ctx->launches += 1;
   return cuda_status(cudaGetLastError(), "rss");
 }
