@@ -1001,11 +1001,21 @@ __global__ void __launch_bounds__(kRowNT) k_fft_rows_dense(const float2* in, flo
   }
 }
 
-// columns along H of every image, grid (W/kWB, images).  Five CTAs per SM: with more
-// registers the compiler's fewer CTAs, and with fewer registers the loads in two
-// batches, are slower (384 x 384 x 120 images, 283 MB: 69 us without the bound, 50
-// with five CTAs, 53 with six, 70 with seven); first factors past 24 need more.
-constexpr int cols_dense_blocks(int H) { return split_a(H) <= 24 && split_b(H) <= 24 ? 5 : 1; }
+// columns along H of every image, grid (W/kWB, images).  Bound by memory; the bound on
+// CTAs per SM decides how many registers the loads of an item get.  us there and back,
+// 256 images of W = 256 unless said otherwise, other bounds -> this one:
+//   first factors 17 to 24, and 512: five CTAs (384 x 384 x 120 images, columns alone, 69
+//     without a bound, 53 with six, 70 with seven -> 50; 504 221 open -> 188; 512 198
+//     with a minimum of one -> 187)
+//   25 to 30, and 392: four (400 168 open -> 150, 448 188 -> 166, 480 202 -> 178)
+//   up to 16 (second factor 16), and second factor 8: open (192 x 160 x 240
+//     images 41.2 with five -> 38.6, 128 x 128 x 600 55.8 -> 51.9, 200 86.0 with a minimum
+//     of one -> 77.5, 216 91.6 -> 83.3, 168 70.2 with five -> 65.4)
+constexpr int cols_dense_blocks(int H) {
+  return split_b(H) == 8 || (split_a(H) <= 16 && split_b(H) == 16)       ? 0
+         : (split_a(H) <= 24 && split_b(H) <= 24) || split_a(H) > 30 ? 5
+                                                                     : 4;
+}
 template <int H>
 __global__ void __launch_bounds__(kColNT, cols_dense_blocks(H))
     k_fft_cols_dense(const float2* in, float2* out, int W, int inv, float scale, const float2* twH) {
