@@ -589,7 +589,20 @@ __device__ __forceinline__ bool ne_barrier(McNe* ne, unsigned target) {
   return ok;
 }
 
-// The CTA's partial: FP32 within a thread's few values and a warp, FP64 over the warps.
+// A thread's sum of squares, whose number of terms grows with the series (11 items at
+// 256 x 256 x 20, 140 at 512 x 512 x 64): with Kahan's compensation, so that its error
+// stays that of one FP32 addition.  Four FP32 operations an item; an FP64 addition would
+// cost 4 K cycles a phase.
+struct NeSum {
+  float s = 0.f, c = 0.f;
+  __device__ __forceinline__ void add(float v) {
+    const float y = __fsub_rn(v, c), t = __fadd_rn(s, y);
+    c = __fsub_rn(__fsub_rn(t, s), y);
+    s = t;
+  }
+};
+
+// The CTA's partial: FP32 within a thread and a warp, FP64 over the warps.
 __device__ __forceinline__ void ne_put(double* part, float s2, bool any) {
   __shared__ float sred[kNeNT / 32];
 #pragma unroll
@@ -685,7 +698,7 @@ __global__ void __launch_bounds__(kNeNT, 1) k_normest(NeArgs n) {
   unsigned gen = 0;
   bool any;
   while (fabsf(e - e0) > kNeTol * e && cnt < kNeMax) {
-    float s2 = 0.f;
+    NeSum s2;
     bool nz = false;
     for (NeItems i = it1; i.left > 0; i.next(HW)) {
       constexpr int NW = kNeFrames + 2;
@@ -704,44 +717,44 @@ __global__ void __launch_bounds__(kNeNT, 1) k_normest(NeArgs n) {
       for (int u = 0; u < kNeFrames; ++u) {
         if (u < nf) {
           const float2 d = csub(w[u + 1], w[u]);
-          s2 = fmaf(d.x, d.x, fmaf(d.y, d.y, s2));
+          s2.add(fmaf(d.x, d.x, d.y * d.y));
           nz |= fabsf(d.x) + fabsf(d.y) != 0.f;
           n.g[size_t(f0 + u) * HW + i.p] = csub(csub(w[u + 2], w[u + 1]), d);
         }
       }
     }
     double* part = n.part;
-    ne_put(part, s2, nz);
+    ne_put(part, s2.s, nz);
     if (!ne_barrier(n.ne, (gen += gridDim.x))) return;
     e0 = e;
     float root = ne_total(part, &any);
     if (!any) {  // uniform over the grid
-      s2 = 0.f;
+      s2 = NeSum{};
       for (NeItems i = it2; i.left > 0; i.next(HW)) {
         const size_t o = size_t(i.f) * HW;
         const float a = ne_draw(rand, o + i.p);
-        s2 = fmaf(a, a, s2);
+        s2.add(a * a);
         n.g[o + i.p] =
             make_float2(__fsub_rn(ne_draw(rand, (unsigned long long)wrap_frame(i.f + 1, F) * HW + i.p), a), 0.f);
       }
       part += 2 * kNeMaxGrid;
-      ne_put(part, s2, false);
+      ne_put(part, s2.s, false);
       if (!ne_barrier(n.ne, (gen += gridDim.x))) return;
       root = ne_total(part, &any);
       rand = (n.ja * rand + n.jc) & ((1ULL << 48) - 1);
       nrestart += 1;
     }
     e = root;
-    s2 = 0.f;
+    s2 = NeSum{};
     for (NeItems i = it2; i.left > 0; i.next(HW)) {
       const int p = i.p, row = p / W, col = p - row * W;
       const bool in_rect = row >= r.r1b && row < r.r1b + r.l1 && col >= r.r2b && col < r.r2b + r.l2;
       const float2 acc = mc_adjoint_at(n.l, n.g, size_t(i.f) * HW, p, in_rect, moved);
       n.x[size_t(i.f) * HW + p] = acc;
-      s2 = fmaf(acc.x, acc.x, fmaf(acc.y, acc.y, s2));
+      s2.add(fmaf(acc.x, acc.x, acc.y * acc.y));
     }
     part = n.part + 4 * kNeMaxGrid;
-    ne_put(part, s2, false);
+    ne_put(part, s2.s, false);
     if (!ne_barrier(n.ne, (gen += gridDim.x))) return;
     sc = 1.0f / ne_total(part, &any);
     cnt += 1;
