@@ -13,7 +13,7 @@
 //
 // FP32 groups whose members' kept rows are each fully sampled or unsampled
 // (checked when the batch is created) run the one-kernel row-local iteration
-// (rowlocal.cuh); a later replay whose data break that sets the members'
+// (rowlocal.cuh), if the memory for its tiles can be had then; a later replay whose data break that sets the members'
 // status (7) and leaves their images unsolved.
 //
 // Power-method restart draws follow the reference's process-wide drand48

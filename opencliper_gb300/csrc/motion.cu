@@ -541,8 +541,8 @@ int grid1(gbn_ctx* ctx, size_t n) { return int(std::min<size_t>((n + kNT - 1) / 
 // which rounds exactly as a separate scaling pass would.  Bound by the latency of the
 // gathers out of L2 and of the barriers: at 256 x 256 x 20, 30 steps, 25 K and 33 K
 // cycles in the phases and 18 K at each barrier with its sums and the SMs' unevenness,
-// 1.4 ms (1.9 before with six launches a step; four frames a thread in phase 1 +70 us,
-// 512 threads +200, 1024 and the next item's loads ahead of this one's: nothing).
+// 1.13 ms under ncu (1.9 before with six launches a step; four frames a thread in phase 1
+// +70 us, 512 threads +200, 1024 and the next item's loads ahead of this one's: nothing).
 constexpr int kNeFrames = 2;     // frames per thread of phase 1
 constexpr int kNeNT = 768;        // threads of a CTA, one CTA per SM
 constexpr int kNeMaxGrid = 256;

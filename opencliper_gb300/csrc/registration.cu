@@ -23,7 +23,11 @@
 // non-zero, with the reference's pairing of spline factors (optimizer.cl:
 // 746-830) and at the transposed pixel (optimizer.cl:138-187).
 //
-// Here one iteration is four kernels:
+// With the reference's default splines (cubic, spacing 4), no smoothness terms in the
+// metric and at most 64 frames, the whole descent is one cooperative launch
+// (k_reg_solve).  Other orders and spacings, a non-zero sumLambda() and longer series
+// run four kernels an iteration, enqueued eight iterations at a time, the host reading
+// the stop flag once per chunk:
 //   k_reg_grad    one thread per (d, frame, control point, column offset): the
 //                 support sums in the reference's order (auxiliarCost,
 //                 cost6DReduction, cost6D)
@@ -34,9 +38,8 @@
 //   k_reg_metric  one thread per bounding-box pixel: the frames' mean, V, dy,
 //                 per-CTA partial sums of the metric; its last CTA sums the
 //                 partials (H, |Dif|) and runs evolution() and stopCondition()
-// iterations are enqueued eight at a time; the host reads the stop flag once
-// per chunk.  This file is compiled without FMA contraction, so products and
-// sums round separately as in the reference's kernels.
+// This file is compiled without FMA contraction, so products and sums round
+// separately as in the reference's kernels.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -642,9 +645,9 @@ __device__ void reg_finish(RegArgs& a, int it, int nh, int nd, float et, float e
 //      the element blocks whose sums of Dif^2 the stopping rule reads.
 // Every sum runs in the order of the kernels above (k_reg_grad ... k_reg_metric),
 // so the results are theirs bit for bit.  Bound by the latency of the two phases
-// and barriers: about 24 K cycles an iteration at 256 x 256 x 20, radius 40, of which
-// the barriers 8 K; a registration of 100 iterations 4.47 -> 1.6 ms (400 launches of
-// ~10 us each on grids of 25 to 1,400 small CTAs before).
+// and barriers: 11.4 us (22 K cycles) an iteration at 256 x 256 x 20, radius 40, 8 K of
+// them the barriers; a registration of 100 iterations 4.47 -> 1.57 ms with its host work
+// (400 launches of ~10 us each on grids of 25 to 1,400 small CTAs before).
 // Data that other CTAs write is read with __ldcg: L1 is not coherent within a launch.
 // ---------------------------------------------------------------------------
 constexpr int kSolveDp = 4, kSolveSup = 17, kSolveE1 = 4;

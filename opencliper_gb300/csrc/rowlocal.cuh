@@ -238,8 +238,10 @@ constexpr int iter_cols_min_blocks(int H) {
   return split_a(H) <= 16 ? 3 : (iter_cols_bytes(H) + 1024 <= 114 * 1024 ? 2 : 1);
 }
 
-// Lengths that run the row-local iteration, in this form or as column pairs;
-// the others (200, 216, 504) run the three-pass iteration.
+// Lengths that run the row-local iteration, in this form or as column pairs.  The
+// others run the three-pass iteration: 200 = 25 x 8 and 216 = 27 x 8 exceed this form's
+// first factor for a second factor of 8 (the column pairs, which run 400 = 25 x 16 and
+// 432 = 27 x 16, follow its rule), and 504 = 21 x 24 has no second factor of 8 or 16.
 constexpr bool iter_cols_ok(int H) {
   return split_a(H) != 0 &&
          (split_a(H) <= 16 || (split_b(H) == 8 && split_a(H) <= 24) || (split_b(H) == 16 && split_a(H) <= 32));

@@ -18,7 +18,7 @@
 // kept rows' IDFT_W(y) is copied one coil ahead.
 //
 // Every operand is read in tiles that a setup kernel lays out once per solve
-// (k_pair_tables, k_pair_pack): planar pairs, [row][pair] of one column group
+// (k_outer_begin_pair; the kept rows' tables are k_rowscan's): planar pairs, [row][pair] of one column group
 // contiguous, so that a warp's 16-byte loads are 512 contiguous bytes.  Read in
 // the natural order, a tile's rows are 32-byte pieces W apart, and the sixteen
 // cache lines a load touches made this kernel no faster than k_iter_cols
@@ -55,8 +55,9 @@ namespace gbn {
 constexpr int kPairNT = 128;
 constexpr int kPairWarps = 4;
 // Largest PA whose accumulators stay in registers: past it they and the
-// transform spill at 168 registers (H = 192: 46.6 us with tensor memory, 50.3
-// with registers; H = 64, PA = 8: 11.3 and 9.8).
+// transform spill much at 168 registers (H = 192: 46.6 us with tensor memory, 50.3
+// with registers; H = 64, PA = 8: 11.3 and 9.8).  Most lengths still spill 16 to 100
+// bytes a thread (256: 72).
 constexpr int kPairAccReg = 8;
 // S is used by F1 and again, at the same rows of the same lane, by I2.  With
 // four pairs per warp (PB = 8) it stays in registers in between; with two the

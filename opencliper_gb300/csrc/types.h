@@ -102,7 +102,8 @@ struct FusedArgs {
   CUtensorMap tm_se;
   CUtensorMap tm_y;
   // column-pair row-local iteration (rowpair.cuh): operands in tiles of planar
-  // pairs, laid out per solve; nullptr for lengths without that iteration
+  // pairs, laid out per solve; nullptr for lengths without that iteration and until
+  // a run takes it
   const float4* St;       // S, [C][column group][row][pair]
   const float4* Tt;       // kept rows' IDFT_W(y), per frame [column group][C][slot][pair]
   float4* px[3];          // x_k and w_k in tiles, in turn: the iteration runs one ahead of the stopping test
