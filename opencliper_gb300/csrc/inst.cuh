@@ -2,26 +2,17 @@
 #pragma once
 
 #include "nesta_kernels.cuh"
+#include "pdl.cuh"
 #include "registry.h"
 #include "rowlocal.cuh"
 #include "rowpair.cuh"
 
 namespace gbn {
 
-// opt a kernel into more than 48 KB of dynamic shared memory (once)
-template <typename K>
-inline void allow_smem(K kernel, int bytes, bool& done) {
-  if (!done) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    done = true;
-  }
-}
-
-
 template <int L>
 struct Launchers {
   static void fwd_cols(const FusedArgs* tab, const BatchMap& bm, int it, int cpb, dim3 grid, cudaStream_t s) {
-    static bool ok = false;
+    static OptedIn ok;
     allow_smem(k_fwd_cols<L>, FwdColsSmem<L>::BYTES, ok);
     launch_chain(it == 0, k_fwd_cols<L>, grid, kColNT, FwdColsSmem<L>::BYTES, s, tab, bm, it, cpb);
   }
@@ -30,7 +21,7 @@ struct Launchers {
     static int occ1 = 0, occ0 = 0;
     int& o = resid ? occ1 : occ0;
     if (o == 0) {
-      static bool ok1 = false, ok0 = false;
+      static OptedIn ok1, ok0;
       int nb = 0;
       if (resid) {
         allow_smem(k_rows<L, true>, RowsSmem<L, true>::BYTES, ok1);
@@ -44,7 +35,7 @@ struct Launchers {
     return o;
   }
   static void rows(const FusedArgs* tab, const BatchMap& bm, int it, bool resid, int grid, cudaStream_t s) {
-    static bool ok1 = false, ok0 = false;
+    static OptedIn ok1, ok0;
     if (resid) {
       allow_smem(k_rows<L, true>, RowsSmem<L, true>::BYTES, ok1);
       launch_pdl(k_rows<L, true>, dim3(grid), kRowNT, RowsSmem<L, true>::BYTES, s, tab, bm, it);
@@ -54,7 +45,7 @@ struct Launchers {
     }
   }
   static void inv_cols(const FusedArgs* tab, const BatchMap& bm, int it, bool update, dim3 grid, cudaStream_t s) {
-    static bool ok1 = false, ok0 = false;
+    static OptedIn ok1, ok0;
     if (update) {
       allow_smem(k_inv_cols<L, true>, InvColsSmem<L>::BYTES, ok1);
       launch_pdl(k_inv_cols<L, true>, grid, kColNT, InvColsSmem<L>::BYTES, s, tab, bm, it);
@@ -66,7 +57,7 @@ struct Launchers {
   static void iter_cols(const FusedArgs* tab, const BatchMap& bm, int it, bool motion, dim3 grid, cudaStream_t s) {
     if constexpr (iter_pair_ok(L)) {
       using P = PairShape<L>;
-      static bool ok0 = false, ok1 = false;
+      static OptedIn ok0, ok1;
       const int ncg = int(grid.x) * kWB / P::COLS, frames = int(grid.z);
       if (motion) {
         allow_smem(k_iter_pair<L, true>, P::BYTES, ok1);
@@ -77,7 +68,7 @@ struct Launchers {
                      it, 0);
       }
     } else if constexpr (iter_cols_ok(L)) {
-      static bool ok0 = false, ok1 = false;
+      static OptedIn ok0, ok1;
       if (motion) {
         allow_smem(k_iter_cols<L, true>, IterColsSmem<L>::BYTES, ok1);
         launch_pdl(k_iter_cols<L, true>, grid, IterColsSmem<L>::NT, IterColsSmem<L>::BYTES, s, tab, bm, it);
@@ -90,7 +81,7 @@ struct Launchers {
   static void iter_finish(const FusedArgs* tab, const BatchMap& bm, int it, dim3 grid, cudaStream_t s) {
     if constexpr (iter_pair_ok(L)) {
       using P = PairShape<L>;
-      static bool ok = false;
+      static OptedIn ok;
       allow_smem(k_iter_pair<L, false>, P::BYTES, ok);
       const int ncg = int(grid.x) * kWB / P::COLS;
       launch_pdl(k_iter_pair<L, false>, dim3(ncg, cdiv(bm.n, ncg)), kPairNT, P::BYTES, s, tab, bm, it, int(grid.z));
@@ -112,7 +103,7 @@ struct Launchers {
   template <bool RSS>
   static void adj_cols_of(const float2* T, const float2* S, float2* x, int W, int C, int F, float scale,
                           const float2* tw, int cs, cudaStream_t s) {
-    static bool ok = false;
+    static OptedIn ok;
     constexpr int bytes = AdjColsShape<L, RSS>::BYTES;
     allow_smem(k_adj_cols<L, RSS>, bytes, ok);
     cudaLaunchConfig_t cfg = {};

@@ -689,13 +689,13 @@ int inv_cols_tc_smem(int nmax) {
 }
 
 void launch_inv_cols_tc(const FusedArgs* tab, const BatchMap& bm, int it, int nmax, dim3 grid, cudaStream_t s) {
-  static bool ok = false;
+  static OptedIn ok;
   allow_smem(k_inv_cols_tc, inv_cols_tc_smem(256), ok);
   launch_pdl(k_inv_cols_tc, grid, 128, inv_cols_tc_smem(nmax), s, tab, bm, it);
 }
 
 void launch_fwd_cols_tc(const FusedArgs* tab, const BatchMap& bm, int it, int npad_max, dim3 grid, cudaStream_t s) {
-  static bool ok = false;
+  static OptedIn ok;
   allow_smem(k_fwd_cols_tc, fwd_cols_tc_smem(256), ok);
   launch_chain(it == 0, k_fwd_cols_tc, grid, 128, fwd_cols_tc_smem(npad_max), s, tab, bm, it);
 }

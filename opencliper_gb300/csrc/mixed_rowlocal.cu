@@ -563,13 +563,10 @@ dim3 iter_tc_grid(int W, int frames) { return dim3(W / kRtCols, 1, frames); }
 
 void launch_iter_tc(const FusedArgs* tab, const BatchMap& bm, int it, int npad_max, int cnmax, dim3 grid,
                     cudaStream_t s) {
-  static bool ok = false;
-  if (!ok) {
-    cudaFuncSetAttribute(k_iter_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, rt_smem(256, 16));
-    // the whole unified memory as shared memory: two CTAs of ~100 KB per SM
-    cudaFuncSetAttribute(k_iter_tc, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    ok = true;
-  }
+  static OptedIn ok, carve;
+  allow_smem(k_iter_tc, rt_smem(256, 16), ok);
+  // the whole unified memory as shared memory: two CTAs of ~100 KB per SM
+  opt_in(k_iter_tc, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared, carve);
   launch_chain(it == 0, k_iter_tc, grid, kRtNT, rt_smem(npad_max, cnmax), s, tab, bm, it, npad_max, cnmax);
 }
 

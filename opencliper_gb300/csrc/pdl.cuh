@@ -9,6 +9,8 @@
 // reads only what the launch three back wrote.
 #pragma once
 
+#include <atomic>
+
 #include <cuda_runtime.h>
 
 namespace gbn {
@@ -40,6 +42,27 @@ inline void launch_chain(bool first, void (*kernel)(KArgs...), dim3 grid, int th
 template <typename... KArgs, typename... Args>
 inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, int smem, cudaStream_t s, Args... args) {
   launch_chain(false, kernel, grid, threads, smem, s, args...);
+}
+
+// The devices a kernel's attribute has been set on: it holds on the device that is
+// current when it is set, and a process may have contexts on several.
+struct OptedIn {
+  std::atomic<unsigned long long> devices{0};  // bit per device; those past 63 set it on every launch
+};
+template <typename K>
+inline void opt_in(K kernel, cudaFuncAttribute attr, int value, OptedIn& done) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+  if (!(done.devices.load(std::memory_order_acquire) & bit)) {
+    cudaFuncSetAttribute(kernel, attr, value);
+    done.devices.fetch_or(bit, std::memory_order_release);
+  }
+}
+// more than 48 KB of dynamic shared memory
+template <typename K>
+inline void allow_smem(K kernel, int bytes, OptedIn& done) {
+  opt_in(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes, done);
 }
 
 }  // namespace gbn

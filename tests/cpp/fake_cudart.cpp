@@ -8,6 +8,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <set>
+#include <utility>
 
 namespace fake {
 static std::map<void*, size_t> g_live;
@@ -21,6 +23,9 @@ size_t live_bytes() {
   return n;
 }
 int bad_frees = 0;
+int device = 0, refused = 0;
+static std::set<std::pair<int, const void*>> g_opted_in;
+size_t opted_in() { return g_opted_in.size(); }
 }  // namespace fake
 
 extern "C" {
@@ -54,6 +59,22 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
 }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
   *p = std::calloc(1, n);
+  return cudaSuccess;
+}
+cudaError_t cudaGetDevice(int* d) {
+  *d = fake::device;
+  return cudaSuccess;
+}
+cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute, int) {
+  fake::g_opted_in.insert({fake::device, f});
+  return cudaSuccess;
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
+  if (c->dynamicSmemBytes > 48 * 1024 && !fake::g_opted_in.count({fake::device, f})) ++fake::refused;
+  return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) {
+  *n = 1;
   return cudaSuccess;
 }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
