@@ -92,9 +92,12 @@ struct Launchers {
     launch_chain(first, mask ? k_fft_rows_dense<L, true> : k_fft_rows_dense<L, false>, dim3(grid), kRowNT, 0, s, in, out,
                  nrows, inv, scale, tw, mask, C, H);
   }
-  static void fft_cols(const float2* in, float2* out, int W, int nimg, int inv, float scale, const float2* tw,
+  static void fft_cols(const float2* in, float2* out, int W, int nimg, int inv, float scale, const float2* tw, int nsm,
                        cudaStream_t s) {
-    launch_pdl(k_fft_cols_dense<L>, dim3(W / kWB, nimg), kColNT, 0, s, in, out, W, inv, scale, tw);
+    constexpr bool two = cols_dense_two_forms(L);
+    const bool few = two && cols_dense_few((long long)(W / kWB) * nimg, nsm);
+    launch_pdl(few ? k_fft_cols_dense<L, two> : k_fft_cols_dense<L, false>, dim3(W / kWB, nimg), kColNT, 0, s, in, out,
+               W, inv, scale, tw);
   }
   static void enc_cols(const float2* x, const float2* S, float2* out, int W, int C, int F, const float2* tw,
                        cudaStream_t s) {

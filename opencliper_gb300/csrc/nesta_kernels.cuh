@@ -1016,8 +1016,16 @@ constexpr int cols_dense_blocks(int H) {
          : (split_a(H) <= 24 && split_b(H) <= 24) || split_a(H) > 30 ? 5
                                                                      : 4;
 }
-template <int H>
-__global__ void __launch_bounds__(kColNT, cols_dense_blocks(H))
+// Few CTAs, at most three per SM, gain nothing from room for five: there those lengths
+// take a thread's whole item in registers (a minimum of one CTA).  us there and back,
+// five CTAs / one: H = 512, images of W = 64, 128 CTAs 24.6 / 16.7, 256 28.8 / 20.9, 384
+// 29.0 / 24.8, 640 34.5 / 37.2, 1280 62.9 / 64.7; 384 128 CTAs 20.5 / 15.0, 384 24.7 /
+// 20.8; 360 256 CTAs 22.7 / 20.6, 640 28.9 / 32.4; 504 64 CTAs 24.0 / 20.3, 640 37.1 /
+// 41.2; with the bound of four no difference up to 384.
+constexpr bool cols_dense_two_forms(int H) { return cols_dense_blocks(H) == 5; }
+inline bool cols_dense_few(long long ctas, int nsm) { return ctas <= 3LL * nsm; }
+template <int H, bool FEW>
+__global__ void __launch_bounds__(kColNT, FEW ? 1 : cols_dense_blocks(H))
     k_fft_cols_dense(const float2* in, float2* out, int W, int inv, float scale, const float2* twH) {
   constexpr int A = Split<H>::A, B = Split<H>::B;
   constexpr int KS = col_ks(B);

@@ -280,7 +280,7 @@ int op_fft2(gbn_ctx* ctx, int direction, const float2* in, float2* out, int W, i
   // against 230 us there and back)
   const int rc = rows_pass(ctx, in, out, W, H, (long long)batch * H, inv, 1.0f, nullptr, 1);
   if (rc != GBN_OK) return rc;
-  kh->fft_cols(out, out, W, batch, inv, scale, ctx_twiddles(ctx, H), ctx->stream);
+  kh->fft_cols(out, out, W, batch, inv, scale, ctx_twiddles(ctx, H), ctx->nsm, ctx->stream);
   ctx->launches += 1;
   return cuda_status(cudaGetLastError(), "fft2");
 }

@@ -24,7 +24,7 @@ struct SizeKernels {
   void (*fft_rows)(const float2* in, float2* out, int nrows, int inv, float scale, const float2* tw,
                    const uint8_t* mask, int C, int H, int grid, bool first, cudaStream_t s);
   // fft_cols, adj_cols: after fft_rows, which releases them; fft_rows not first: after enc_cols
-  void (*fft_cols)(const float2* in, float2* out, int W, int nimg, int inv, float scale, const float2* tw,
+  void (*fft_cols)(const float2* in, float2* out, int W, int nimg, int inv, float scale, const float2* tw, int nsm,
                    cudaStream_t s);
   void (*enc_cols)(const float2* x, const float2* S, float2* out, int W, int C, int F, const float2* tw,
                    cudaStream_t s);
