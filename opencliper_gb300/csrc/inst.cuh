@@ -44,15 +44,19 @@ struct Launchers {
       launch_chain(true, k_rows<L, false>, dim3(grid), kRowNT, RowsSmem<L, false>::BYTES, s, tab, bm, it);
     }
   }
+  template <bool UPDATE, bool PREF>
+  static void inv_cols_of(const FusedArgs* tab, const BatchMap& bm, int it, dim3 grid, cudaStream_t s) {
+    static OptedIn ok;
+    allow_smem(k_inv_cols<L, UPDATE, PREF>, InvColsSmem<L>::BYTES, ok);
+    launch_pdl(k_inv_cols<L, UPDATE, PREF>, grid, kColNT, InvColsSmem<L>::BYTES, s, tab, bm, it);
+  }
   static void inv_cols(const FusedArgs* tab, const BatchMap& bm, int it, bool update, dim3 grid, cudaStream_t s) {
-    static OptedIn ok1, ok0;
-    if (update) {
-      allow_smem(k_inv_cols<L, true>, InvColsSmem<L>::BYTES, ok1);
-      launch_pdl(k_inv_cols<L, true>, grid, kColNT, InvColsSmem<L>::BYTES, s, tab, bm, it);
-    } else {
-      allow_smem(k_inv_cols<L, false>, InvColsSmem<L>::BYTES, ok0);
-      launch_pdl(k_inv_cols<L, false>, grid, kColNT, InvColsSmem<L>::BYTES, s, tab, bm, it);
-    }
+    constexpr bool pref = inv_prefetch(L), other = pref != inv_two_forms<L>();
+    const bool plain = inv_two_forms<L>() && inv_fewer_waves((long long)grid.x * grid.y * grid.z, device_sms());
+    if (update)
+      plain ? inv_cols_of<true, other>(tab, bm, it, grid, s) : inv_cols_of<true, pref>(tab, bm, it, grid, s);
+    else
+      plain ? inv_cols_of<false, other>(tab, bm, it, grid, s) : inv_cols_of<false, pref>(tab, bm, it, grid, s);
   }
   static void iter_cols(const FusedArgs* tab, const BatchMap& bm, int it, bool motion, dim3 grid, cudaStream_t s) {
     if constexpr (iter_pair_ok(L)) {

@@ -654,8 +654,21 @@ struct InvColsSmem {
 // 800, 128 794 / 759, 160 888 / 865, 192 918 / 874, 256 1004 / 1003; 168 933 / 1135, 288
 // 1328 / 1545, 360 1819 / 1990, 392 1900 / 2169.
 constexpr bool inv_prefetch(int H) { return split_a(H) <= 16 && split_b(H) <= 16; }
-template <int H, bool UPDATE>
-__global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT, inv_prefetch(H) ? 3 : 0)
+// Where shared memory holds four CTAs per SM (up to 192) the plain form, at 128 registers,
+// runs four and this one three: the plain form is taken for grids that four per SM finish
+// in fewer waves.  Pixel masks, 8 coils, 10 iterations, us, plain / this form, by CTAs on
+// 152 SMs: H = 96 432 CTAs 453 / 438, 480 468 / 518, 600 489 / 540, 800 600 / 574, 1200 669
+// / 722, 5120 2057 / 2166; 128 432 470 / 451, 600 512 / 562, 800 629 / 598, 1200 720 / 766,
+// 2560 1318 / 1313, 5120 2315 / 2415; 192 432 540 / 515, 600 572 / 646, 1200 857 / 931.
+template <int H>
+constexpr bool inv_two_forms() {
+  return inv_prefetch(H) && 4 * (InvColsSmem<H>::BYTES + 1024) <= 228 * 1024;
+}
+constexpr bool inv_fewer_waves(long long ctas, int nsm) {
+  return (ctas + 4LL * nsm - 1) / (4LL * nsm) < (ctas + 3LL * nsm - 1) / (3LL * nsm);
+}
+template <int H, bool UPDATE, bool PREF = inv_prefetch(H)>
+__global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT, PREF ? 3 : 0)
     k_inv_cols(const FusedArgs* __restrict__ tab, const __grid_constant__ BatchMap bm, int it) {
   using L = InvColsSmem<H>;
   constexpr int A = L::A, B = L::B, KS = L::KS, RCAP = L::RCAP;
@@ -713,7 +726,6 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kColNT, inv_prefetch
       for (int k1p = 0; k1p < B; ++k1p) twr[ii][k1p] = __ldg(a.twH + H + k1p * A + s);
     }
   };
-  constexpr bool PREF = inv_prefetch(H);
   if constexpr (PREF) load_twiddles();
   grid_dep_wait();  // T and the scalar state come from the row pass
   grid_dep_release();

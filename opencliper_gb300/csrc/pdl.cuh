@@ -59,6 +59,16 @@ inline void opt_in(K kernel, cudaFuncAttribute attr, int value, OptedIn& done) {
     done.devices.fetch_or(bit, std::memory_order_release);
   }
 }
+// the current device's SMs
+inline int device_sms() {
+  static std::atomic<int> known[64];
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  if (dev < 64 && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 1;
+  if (dev < 64) known[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
 // more than 48 KB of dynamic shared memory
 template <typename K>
 inline void allow_smem(K kernel, int bytes, OptedIn& done) {
